@@ -77,25 +77,90 @@ template <bool F> __device__ __forceinline__ double d_max_nn(double a, double b)
     return fmax(a, b);
 }
 
-/* 1/y from the hardware's approximate FP64 reciprocal refined by two
- * Newton-Raphson steps r <- r + r (1 - y r) (quadratic convergence: about
- * 2^-84 relative before the last rounding, i.e. within an ulp of the
- * correctly rounded quotient). For normal, non-zero y only: the inputs
- * here are depths, speeds and their differences away from zero. */
-__device__ __forceinline__ double gf_rcp(double y)
+/* The hardware's approximate FP64 reciprocal and reciprocal root (subnormal
+ * arguments count as zero). A host build of these headers (tests) brings its
+ * own. */
+#ifndef GF_HOST_MATH
+__device__ __forceinline__ double gf_rcp_seed(double y)
 {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
-    double e = fma(-y, r, 1.0);
-    r = fma(r, e, r);
-    e = fma(-y, r, 1.0);
-    return fma(r, e, r);
+    return r;
 }
+__device__ __forceinline__ double gf_rsqrt_seed(double a)
+{
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    return y;
+}
+#endif
+
+/* 1/y from the hardware's approximate FP64 reciprocal r refined once with
+ * the third-order step r + r (e + e^2), e = 1 - y r (the geometric series of
+ * 1 / (1 - e) cut after e^2): the remainder e^3 is far below the last
+ * rounding, so the result is within an ulp of the correctly rounded
+ * quotient. One FP64 instruction fewer than two Newton-Raphson steps. For
+ * normal, non-zero y only: the inputs here are depths, speeds and their
+ * differences away from zero. */
+__device__ __forceinline__ double gf_rcp(double y)
+{
+    const double r = gf_rcp_seed(y);
+    const double e = fma(-y, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+/* positive and normal (neither zero, subnormal, infinite, NaN nor negative) */
+__device__ __forceinline__ bool gf_pos_normal(double x)
+{
+    return static_cast<unsigned>(__double2hiint(x)) - 0x00100000u < 0x7ff00000u - 0x00100000u;
+}
+
+/* The root and its reciprocal of a positive normal a from the hardware's
+ * approximate FP64 reciprocal root y and one third-order step: with
+ * e = 1 - a y^2, a^(-1/2) = y (1 - e)^(-1/2) = y (1 + e/2 + 3 e^2/8 + ...);
+ * the remainder of order e^3 is far below the last rounding. */
+__device__ __forceinline__ double gf_rsqrt_n(double a)
+{
+    const double y = gf_rsqrt_seed(a);
+    const double e = fma(-(a * y), y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+__device__ __forceinline__ double gf_sqrt_n(double a)
+{
+    const double y = gf_rsqrt_seed(a);
+    const double t = a * y;
+    const double e = fma(-t, y, 1.0);
+    return fma(t * e, fma(0.375, e, 0.5), t);
+}
+
+/* Single-precision value of x, cut to its leading bits on the integer pipe
+ * (a conversion instruction runs at the FP64 pipe's rate): below the normal
+ * range zero, above it infinity. And a normal float as a double. */
+__device__ __forceinline__ float gf_f32(double x)
+{
+    const unsigned hi = static_cast<unsigned>(__double2hiint(x)), lo = static_cast<unsigned>(__double2loint(x));
+    const unsigned a = hi & 0x7fffffffu;
+    unsigned r = __funnelshift_l(lo, a - 0x38000000u, 3);
+    r = a < 0x38100000u ? 0u : a >= 0x47f00000u ? 0x7f800000u : r;
+    return __uint_as_float(r | (hi & 0x80000000u));
+}
+__device__ __forceinline__ double gf_f64_pos(float x)
+{
+    const unsigned u = __float_as_uint(x);
+    return __hiloint2double(static_cast<int>((u >> 3) + 0x38000000u), static_cast<int>(u << 29));
+}
+
+/* Products and sums of the contracted build that are written as the operation
+ * they become: the compiler fuses none of them, so every kernel instantiated
+ * from one source gives the same bits. */
+__device__ __forceinline__ double gf_mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double gf_add(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double gf_sub(double a, double b) { return __dadd_rn(a, -b); }
 
 /* x / y: the IEEE quotient, or x * gf_rcp(y) in the production build */
 template <bool F> __device__ __forceinline__ double d_div(double x, double y)
 {
-    if (F) return x * gf_rcp(y);
+    if (F) return gf_mul(x, gf_rcp(y));
     return x / y;
 }
 

@@ -5,7 +5,7 @@
  * Tile shapes per patch size m (threads per CTA, slices per band):
  *   m = 32: 256 threads, 7 slices  (245 / 231 faces per band stage)
  *   m = 16: 128 threads, 6 slices  (114 / 102)
- *   m =  8:  64 threads, 5 slices  ( 55 /  45)
+ *   m =  8: 128 threads, 10 slices (110 /  90)
  * chosen so the flattened face loops of a band fill the CTA.
  */
 #include <cuda_runtime.h>
@@ -91,11 +91,11 @@ using UpdateFn = cudaError_t (*)(const gf_patch_work*, int, const gf_phys*, doub
                                  const int*, int, double*, unsigned long long*, int*, int, cudaStream_t);
 using OccFn = int (*)();
 
-template <int M, int NT, int RB>
+template <int M, int NT, int RB, int MINB>
 static int occupancy_of()
 {
     using L = Smem<M, RB, false>;
-    auto kern = patch_update_kernel<M, NT, RB, 1, false>;
+    auto kern = patch_update_kernel<M, NT, RB, MINB, false>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) !=
         cudaSuccess)
         return 0;
@@ -104,8 +104,8 @@ static int occupancy_of()
     return n;
 }
 
-template <int M, int NT, int RB>
-static int tile_slots() { return occupancy_of<M, NT, RB>() * sm_count(); }
+template <int M, int NT, int RB, int MINB>
+static int tile_slots() { return occupancy_of<M, NT, RB, MINB>() * sm_count(); }
 
 struct Tile {
     int nt, rb, k; /* k > 1: the patch split over a cluster of k CTAs */
@@ -114,18 +114,18 @@ struct Tile {
     OccFn slots; /* patches resident at once in one launch */
 };
 
-#define GF_TILE(M, NT, RB) \
-    {NT, RB, 1, &launch_update<M, NT, RB, 1>, &occupancy_of<M, NT, RB>, &tile_slots<M, NT, RB>}
+#define GF_TILE(M, NT, RB, MINB)                                                              \
+    {NT, RB, 1, &launch_update<M, NT, RB, MINB>, &occupancy_of<M, NT, RB, MINB>,              \
+     &tile_slots<M, NT, RB, MINB>}
 #define GF_WTILE(M, NT, RB, K)                                                                \
     {NT, RB, K, &launch_window<M, NT, RB, K>, &window_occupancy<M, NT, RB, K>,                \
      &window_slots<M, NT, RB, K>}
-static const Tile kTiles8[] = {GF_TILE(8, 64, 5), GF_TILE(8, 128, 10), GF_TILE(8, 128, 5),
+static const Tile kTiles8[] = {GF_TILE(8, 64, 5, 6), GF_TILE(8, 128, 10, 4), GF_TILE(8, 128, 5, 3),
                                GF_WTILE(8, 64, 5, 2), GF_WTILE(8, 64, 5, 4)};
-static const Tile kTiles16[] = {GF_TILE(16, 128, 6), GF_TILE(16, 256, 13), GF_TILE(16, 256, 9),
-                                GF_WTILE(16, 128, 6, 2), GF_WTILE(16, 128, 6, 4),
-                                GF_WTILE(16, 256, 9, 4)};
-static const Tile kTiles32[] = {GF_TILE(32, 256, 7), GF_TILE(32, 256, 5), GF_TILE(32, 384, 7),
-                                GF_TILE(32, 384, 9), GF_TILE(32, 512, 8), GF_TILE(32, 512, 9),
+static const Tile kTiles16[] = {GF_TILE(16, 128, 6, 3), GF_TILE(16, 256, 13, 1), GF_TILE(16, 256, 9, 2),
+                                GF_WTILE(16, 128, 6, 2), GF_WTILE(16, 128, 6, 4), GF_WTILE(16, 256, 9, 4)};
+static const Tile kTiles32[] = {GF_TILE(32, 256, 7, 1), GF_TILE(32, 256, 5, 1), GF_TILE(32, 384, 7, 1),
+                                GF_TILE(32, 384, 9, 1), GF_TILE(32, 512, 8, 1), GF_TILE(32, 512, 9, 1),
                                 GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8)};
 #undef GF_TILE
 #undef GF_WTILE
@@ -140,8 +140,11 @@ static const Tile* tiles_of(int m, int* n)
     }
 }
 
-/* selected variant per goal (0 throughput, 1 latency) and patch size */
-static int g_tile[2][3] = {{0, 0, 0}, {0, 0, 0}};
+/* selected variant per goal (0 throughput, 1 latency) and patch size. 8^2
+ * patches start with a whole patch per band and a thread per face: the
+ * classes of a band's faces then fill warps better, and the list pass is one
+ * round (24 patches 41 us, 4096 patches 361 us; 64 x 5: 58 and 399 us). */
+static int g_tile[2][3] = {{1, 0, 0}, {1, 0, 0}};
 static inline int mcls(int m) { return m == 8 ? 0 : m == 16 ? 1 : 2; }
 
 int tile_count(int m)

@@ -22,10 +22,10 @@
  * ceiling), so the layout of the work aims at few FP64 instructions and
  * uniform warps:
  *   - per-cell quotients computed once (hu/h, hv/h, sqrt(g h), and in the
- *     contracted build 1/h and 1/sqrt(g h));
- *   - the faces of each band are listed by class (both cells wet, grouped
- *     by the wave structure riemanntype will find; one wet; both dry) so a
- *     warp runs one code path; dry faces only store zeros;
+ *     contracted build 1/sqrt(g h));
+ *   - the faces of each band are listed by class (both cells wet, with the
+ *     short solve or the full one; one wet; both dry) so a warp runs one
+ *     code path; dry faces only store zeros;
  *   - the per-face outputs of a band go to shared memory and each interior
  *     cell gathers its six contributing faces in slice order, so every cell
  *     is written by one thread per band, in a fixed order: deterministic and
@@ -98,6 +98,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
+/* Barrier of the CTAs of a cluster, in two halves. */
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.aligned;" ::: "memory"); }
+
 /* sign(s) * x for the limiter's factor: x with its sign bit flipped when s
  * is negative (-0 included), on the integer pipe instead of a product */
 __device__ __forceinline__ double with_sign_of(double x, double s)
@@ -124,16 +128,18 @@ struct Geo {
 
 /* Shared-memory layout (doubles unless noted). NACC flux accumulators of 3
  * components per interior cell: 2 (DX, DY) in the contracted build, 4 (fm,
- * fp, gm, gp) in the exact build. The contracted build also keeps 1/h and
- * 1/sqrt(g h) planes. */
+ * fp, gm, gp) in the exact build. The contracted build also keeps a
+ * 1/sqrt(g h) plane. */
 template <int M, int RB, bool EXACT = false>
 struct Smem {
     using G = Geo<M>;
     static constexpr int NACC = EXACT ? 4 : 2;
     static constexpr int NBAND = (G::NSLICE + RB - 1) / RB;
     /* Odd strides (in doubles) spread a warp's accesses to face records and
-     * accumulator rows over the shared-memory banks. */
-    static constexpr int W_STRIDE = 13; /* s[3] + fw[3][3], 1 pad            */
+     * accumulator rows over the shared-memory banks. Face record: s[3] +
+     * fw[3][3] (1 pad) in the exact build; the contracted build leaves out the
+     * middle f-wave's two zero components: s[3], fw0[3], fw1[1], fw2[3], 1 pad */
+    static constexpr int W_STRIDE = EXACT ? 13 : 11;
     /* limited-face records: exact build faddm faddp A B C D (3 comps each, 1
      * pad); contracted build amdq apdq cq (local order) */
     static constexpr int O_STRIDE = EXACT ? 19 : 9;
@@ -149,27 +155,38 @@ struct Smem {
     static constexpr int OFF_U = OFF_B + G::S;
     static constexpr int OFF_V = OFF_U + G::S;
     static constexpr int OFF_C = OFF_V + G::S;
-    static constexpr int OFF_RH = OFF_C + G::S;                     /* contracted only */
-    static constexpr int OFF_RC = OFF_RH + (EXACT ? 0 : G::S);      /* contracted only */
+    static constexpr int OFF_RC = OFF_C + G::S;                     /* contracted only */
     static constexpr int OFF_ACC = OFF_RC + (EXACT ? 0 : G::S);     /* NACC x [3][M*M] */
     static constexpr int OFF_W = OFF_ACC + NACC * 3 * PLANE;
     static constexpr int OFF_O = OFF_W + RB * G::FA * W_STRIDE;
     static constexpr int OFF_C2 = OFF_O + RB * G::FB * O_STRIDE;   /* contracted only */
-    static constexpr int OFF_RED = OFF_C2 + (EXACT ? 0 : RB * G::FB * C_STRIDE); /* 2*32 doubles */
-    static constexpr int OFF_BAR = OFF_RED + 64;                    /* 1 x u64     */
+    /* per item: dt/dx, dt/dy, 1/(16 g), 1/sqrt(g), the sonic tolerances, the
+     * friction factors, the CFL maximum (SC_*) */
+    static constexpr int OFF_SC = OFF_C2 + (EXACT ? 0 : RB * G::FB * C_STRIDE);
+    static constexpr int OFF_BAR = OFF_SC + 16;                     /* 1 x u64     */
     /* integer region: class counts per band and face lists (u16) */
     static constexpr int OFF_INT = OFF_BAR + 2;
     static constexpr int NCLS = 5;                                  /* face classes, see build_lists */
-    static constexpr int CNT_INTS = NBAND * 2 * NCLS * 2;           /* [band][A|B][class][count|pos] */
+    /* exact: [band][A|B][class][count|pos]; contracted: [sweep][band][A classes
+     * smooth, edge, full, dry | B classes wet, dry], then a chunk cursor per
+     * phase of each sweep */
+    static constexpr int CNT_SWEEP = NBAND * 6, CNT_CUR = 2 * CNT_SWEEP, CUR_SWEEP = 2 * (NBAND + 1);
+    static constexpr int CNT_INTS = EXACT ? NBAND * 2 * NCLS * 2 : CNT_CUR + 2 * CUR_SWEEP;
     static constexpr int LIST_A = G::NSLICE * G::FA;
     static constexpr int LIST_B = G::NSLICE * G::FB;
-    static constexpr size_t INT_BYTES = ((CNT_INTS * 4 + (LIST_A + LIST_B) * 2) + 15) / 16 * 16;
+    /* contracted: also a list of edge and full-solve faces, and all three for
+     * either sweep (the y sweep's are made during the x sweep) */
+    static constexpr int LIST_SWEEP = 2 * LIST_A + LIST_B;
+    static constexpr int LISTS = EXACT ? LIST_A + LIST_B : 2 * LIST_SWEEP;
+    static constexpr size_t INT_BYTES = ((CNT_INTS * 4 + LISTS * 2) + 15) / 16 * 16;
     static constexpr size_t OFF_WET_BYTES = (size_t)OFF_INT * 8 + INT_BYTES;
-    /* class of each normal-solve face of the sweep (u8), kept between the
-     * count and place passes */
+    /* exact: class of each normal-solve face of the sweep (u8), kept between
+     * the count and place passes */
     static constexpr size_t OFF_FCLS_BYTES = OFF_WET_BYTES + ((G::S + 15) / 16) * 16;
-    static constexpr size_t BYTES = OFF_FCLS_BYTES + ((LIST_A + 15) / 16) * 16;
+    static constexpr size_t BYTES = OFF_FCLS_BYTES + (EXACT ? ((LIST_A + 15) / 16) * 16 : 0);
 };
+
+enum { SC_DTDX, SC_DTDY, SC_C16G, SC_RSG, SC_CRIT, SC_CRIT2, SC_KF, SC_CFL = SC_KF + GF_MAX_MANNING, SC_PART };
 
 /* Load the cell view for a face sweep in direction DIR (0 = x, 1 = y). */
 template <int DIR, bool EXACT, class L>
@@ -187,13 +204,7 @@ __device__ __forceinline__ gf_cell load_cell(const double* sm, const unsigned ch
         c.hun = sm[L::OFF_HV + k]; c.hut = sm[L::OFF_HU + k];
         c.un = sm[L::OFF_V + k];   c.ut = sm[L::OFF_U + k];
     }
-    if (!EXACT) {
-        c.rh = sm[L::OFF_RH + k];
-        c.rc = sm[L::OFF_RC + k];
-    } else {
-        c.rh = 0.0;
-        c.rc = 0.0;
-    }
+    c.rc = EXACT ? 0.0 : sm[L::OFF_RC + k];
     return c;
 }
 
@@ -228,23 +239,93 @@ struct SweepWin {
     }
 };
 
-/* Build, for every band of one sweep direction, the normal-solve faces
- * (list A) and the limited faces (list B) ordered by class, so that a warp
- * runs one code path. Classes: 0..2 both cells wet, by the wave structure
- * riemanntype will find (0 two shocks, the costly branch, first so that one
- * class boundary at most splits its warps; 1 two rarefactions; 2 a shock
- * and a rarefaction; list B puts all wet pairs in class 0); 3 one cell wet;
- * 4 both dry. The wave structure is estimated without a square root (F_max <= 0 as
- * delu <= 0 and delu^2 hmin hmax >= (hmax - hmin)^2 g (hmin + hmax) / 2); a
- * borderline face in the neighbouring class only costs divergence, since
- * every face's solve is the same computation wherever it is listed. Two
- * passes (count, then place) over all faces. */
-template <int M, int NT, int RB, int DIR, bool EXACT>
-__device__ __forceinline__ void build_lists(const double* sm, const unsigned char* wet, int* cnt, uint16_t* la,
-                                            uint16_t* lb, double g, const SweepWin<M, RB, DIR>& w)
+/* The full solve into a face record (contracted build). Not inlined: faces
+ * that need it are few, its registers stay its own, and the kernels share one
+ * body of it and so its bits. */
+static __device__ __noinline__ void full_solve(const gf_cell& cl, const gf_cell& cr, double g, double drytol,
+                                               const double* sc, double* w)
+{
+    double s[3], fw[3][3];
+    gf_rpn2_face<true>(cl, cr, g, drytol, sc[SC_C16G], sc[SC_RSG], sc[SC_CRIT], sc[SC_CRIT2], s, fw);
+    w[0] = s[0]; w[1] = s[1]; w[2] = s[2];
+    w[3] = fw[0][0]; w[4] = fw[0][1]; w[5] = fw[0][2];
+    w[6] = fw[1][1];
+    w[7] = fw[2][0]; w[8] = fw[2][1]; w[9] = fw[2][2];
+}
+
+/* A sweep's face lists in shared memory: class counts, cursors, lists. */
+struct SweepLists {
+    int* cnt;
+    int* cur;
+    uint16_t *la, *lb, *lm;
+};
+
+/* Contracted build: the faces 32 c .. 32 c + 31 of one band of a sweep into
+ * the band's lists by class (gf_face_class), so that a warp of the solves runs
+ * one code path. Normal solves: edge faces (lm from the front, their flag in
+ * bit 15), faces for the full solve (lm from the back), smooth faces (la from
+ * the front), both cells dry (la from the back); limited faces: some water (lb
+ * from the front), none (from the back). Lists filled from both ends need no
+ * counts beforehand, and a warp's faces of one class take their places with
+ * one atomic. */
+template <int M, int RB, int DIR>
+__device__ __forceinline__ void list_chunk(const double* sm, const unsigned char* wet, const SweepLists& ls, double g,
+                                           double crit, double crit2, const SweepWin<M, RB, DIR>& w, int band, int c)
+{
+    using L = Smem<M, RB, false>;
+    constexpr int N = Geo<M>::N;
+    const double* U = sm + (DIR == 0 ? L::OFF_U : L::OFF_V);
+    const int lane = threadIdx.x & 31;
+    const int ns = min(w.rb, w.nsl - band * w.rb), na = ns * w.fa;
+    if (32 * c >= na) return; /* the whole warp */
+    const bool act = 32 * c + lane < na;
+    const int i = act ? 32 * c + lane : 0;
+    const int ts = i / w.fa, n = w.na_lo + (i - ts * w.fa), t = w.ts_lo + band * w.rb + ts;
+    const int kl = DIR == 0 ? (t + 1) * N + n : n * N + (t + 1), kr = kl + (DIR == 0 ? 1 : N);
+    const bool wl = wet[kl] != 0, wr = wet[kr] != 0;
+    int cls = 3; /* 0 smooth, 1 edge, 2 full, 3 dry */
+    bool flag = false;
+    if (wl | wr) {
+        const int k = gf_face_class(gf_f32(sm[L::OFF_H + kl]), gf_f32(sm[L::OFF_H + kr]), gf_f32(U[kl]), gf_f32(U[kr]),
+                                    gf_f32(sm[L::OFF_C + kl]), gf_f32(sm[L::OFF_C + kr]), gf_f32(sm[L::OFF_B + kl]),
+                                    gf_f32(sm[L::OFF_B + kr]), wl, wr, gf_f32(g), gf_f32(crit), gf_f32(crit2));
+        cls = k == 0 ? 0 : k == 3 ? 2 : 1;
+        flag = k == 2;
+    }
+    /* one place in the list of class k (k < 0: none) for every lane */
+    auto place = [&](int k) -> int {
+        const unsigned m = __match_any_sync(0xffffffffu, k);
+        const int lead = __ffs(m) - 1;
+        int base = 0;
+        if (lane == lead && k >= 0) base = atomicAdd(&ls.cnt[band * 6 + k], __popc(m));
+        return __shfl_sync(0xffffffffu, base, lead) + __popc(m & ((1u << lane) - 1u));
+    };
+    const int pa = place(act ? cls : -1);
+    if (act) {
+        uint16_t* to = ((cls == 1 || cls == 2) ? ls.lm : ls.la) + band * w.rb * w.fa;
+        to[cls >= 2 ? na - 1 - pa : pa] = (uint16_t)(i | (flag ? 0x8000 : 0));
+    }
+    const bool limited = act && n >= w.nb_lo && n < w.nb_lo + w.fb, dry = cls == 3;
+    const int pb = place(limited ? (dry ? 5 : 4) : -1);
+    if (limited)
+        ls.lb[band * w.rb * w.fb + (dry ? ns * w.fb - 1 - pb : pb)] = (uint16_t)(ts * w.fb + (n - w.nb_lo));
+}
+
+/* Exact build: for every band of one sweep direction, the normal-solve faces
+ * (list A) and the limited faces (list B) ordered by class. Classes: 0..2
+ * both cells wet, by the wave structure riemanntype will find (0 two shocks,
+ * the costly branch, first so that one class boundary at most splits its
+ * warps; 1 two rarefactions; 2 a shock and a rarefaction; list B puts all wet
+ * pairs in class 0); 3 one cell wet; 4 both dry. The wave structure is
+ * estimated without a square root (F_max <= 0 as delu <= 0 and
+ * delu^2 hmin hmax >= (hmax - hmin)^2 g (hmin + hmax) / 2); it only orders the
+ * list. Two passes (count, then place) over all faces. */
+template <int M, int NT, int RB, int DIR>
+__device__ __forceinline__ void build_lists_exact(const double* sm, const unsigned char* wet, int* cnt, uint16_t* la,
+                                                  uint16_t* lb, double g, const SweepWin<M, RB, DIR>& w)
 {
     using G = Geo<M>;
-    using L = Smem<M, RB, EXACT>;
+    using L = Smem<M, RB, true>;
     constexpr int N = G::N;
     constexpr int NC = L::NCLS;
     unsigned char* fcls = const_cast<unsigned char*>(reinterpret_cast<const unsigned char*>(sm)) + L::OFF_FCLS_BYTES;
@@ -263,34 +344,16 @@ __device__ __forceinline__ void build_lists(const double* sm, const unsigned cha
         const int kl = cidx(n - 1, t), kr = cidx(n, t);
         const int nw = wet[kl] + wet[kr];
         int cls = nw == 0 ? 4 : nw == 1 ? 3 : 0;
-        if (nw == 2 && EXACT) {
+        if (nw == 2) {
             const double hL = sm[L::OFF_H + kl], hR = sm[L::OFF_H + kr];
             const double uL = sm[(DIR == 0 ? L::OFF_U : L::OFF_V) + kl];
             const double uR = sm[(DIR == 0 ? L::OFF_U : L::OFF_V) + kr];
             const double cL = sm[L::OFF_C + kl], cR = sm[L::OFF_C + kr];
-            constexpr bool F = false;
             const double delu = uR - uL;
-            const double hmin = d_min<F>(hL, hR), hmax = d_max<F>(hL, hR);
+            const double hmin = fmin(hL, hR), hmax = fmax(hL, hR);
             const double dh = hmax - hmin;
-            if (d_gtz<F>(delu + 2.0 * (d_min<F>(cL, cR) - d_max<F>(cL, cR)))) cls = 1;
-            else if (d_lez<F>(delu) && d_ge<F>(delu * delu * (hmin * hmax), dh * dh * (0.5 * g) * (hmin + hmax)))
-                cls = 0;
-            else cls = 2;
-        } else if (nw == 2) {
-            /* The class only orders the list (a face in the neighbouring
-             * class costs divergence, not bits), so the contracted build
-             * estimates it in single precision off the FP64 pipe. */
-            const float hL = __double2float_rn(sm[L::OFF_H + kl]), hR = __double2float_rn(sm[L::OFF_H + kr]);
-            const float uL = __double2float_rn(sm[(DIR == 0 ? L::OFF_U : L::OFF_V) + kl]);
-            const float uR = __double2float_rn(sm[(DIR == 0 ? L::OFF_U : L::OFF_V) + kr]);
-            const float cL = __double2float_rn(sm[L::OFF_C + kl]), cR = __double2float_rn(sm[L::OFF_C + kr]);
-            const float delu = uR - uL;
-            const float hmin = fminf(hL, hR), hmax = fmaxf(hL, hR);
-            const float dh = hmax - hmin;
-            if (delu + 2.0f * (fminf(cL, cR) - fmaxf(cL, cR)) > 0.0f) cls = 1;
-            else if (delu <= 0.0f &&
-                     delu * delu * (hmin * hmax) >= dh * dh * (0.5f * (float)g) * (hmin + hmax))
-                cls = 0;
+            if (delu + 2.0 * (fmin(cL, cR) - fmax(cL, cR)) > 0.0) cls = 1;
+            else if (delu <= 0.0 && delu * delu * (hmin * hmax) >= dh * dh * (0.5 * g) * (hmin + hmax)) cls = 0;
             else cls = 2;
         }
         fcls[f] = (unsigned char)cls;
@@ -329,12 +392,13 @@ __device__ __forceinline__ void build_lists(const double* sm, const unsigned cha
 }
 
 /* One sweep direction over all slices, banded. Accumulates into the flux
- * accumulators; returns this thread's max |s| over normal faces. */
-template <int M, int NT, int RB, int DIR, bool EXACT>
-__device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, int* cnt,
-                                        uint16_t* la, uint16_t* lb, const gf_phys& P, double dtdn,
-                                        double c16g, double rsg, double crit, double crit2,
-                                        int rlo, int rhi)
+ * accumulators (contracted build: the x sweep starts them); returns this
+ * thread's max |s| over normal faces. side: further work of 32 items a chunk
+ * that its phases take along (contracted build; the face lists still to be
+ * made). */
+template <int M, int NT, int RB, int DIR, bool EXACT, class Side>
+__device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, const SweepLists& ls, const gf_phys& P,
+                                        int rlo, int rhi, const Side& side)
 {
     using G = Geo<M>;
     using L = Smem<M, RB, EXACT>;
@@ -343,7 +407,13 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
     double* W = sm + L::OFF_W;
     double* O = sm + L::OFF_O;
     const double g = P.grav, drytol = P.dry_tolerance;
+    const double* sc = sm + L::OFF_SC;
+    const double dtdn = sc[DIR == 0 ? SC_DTDX : SC_DTDY], c16g = sc[SC_C16G], rsg = sc[SC_RSG];
+    const double crit = sc[SC_CRIT], crit2 = sc[SC_CRIT2];
     const double half_dtdn = 0.5 * dtdn;
+    int* cnt = ls.cnt;
+    uint16_t *la = ls.la, *lb = ls.lb;
+    const uint16_t* lm = ls.lm; /* contracted build */
     /* local component l -> global component (h, hu, hv) */
     constexpr int G1 = (DIR == 0) ? 1 : 2; /* normal momentum     */
     constexpr int G2 = (DIR == 0) ? 2 : 1; /* transverse momentum */
@@ -362,7 +432,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
 
     const SweepWin<M, RB, DIR> win(rlo, rhi);
     const int fa = win.fa, fb = win.fb;
-    build_lists<M, NT, RB, DIR, EXACT>(sm, wet, cnt, la, lb, g, win);
+    if constexpr (EXACT) build_lists_exact<M, NT, RB, DIR>(sm, wet, cnt, la, lb, g, win);
     /* cells the gather writes: slice-direction t clamped to the window's rows
      * in the x sweep, cell-direction n clamped to them in the y sweep */
     const int gt_lo = DIR == 0 ? rlo : 1, gt_hi = DIR == 0 ? rhi : M;
@@ -388,15 +458,18 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
     double* TM = sm + L::OFF_ACC + (DIR == 0 ? 6 * MM : 0);
     double* TP = TM + 3 * MM;
 
-    auto gather = [&](int t0, int t1) {
-        /* slices t0..t1 feed cells n in [1, M], t in [t0-1, t1+1] (interior),
-         * within the window */
-        const int ta = max(gt_lo, t0 - 1), tb = min(gt_hi, t1 + 1);
+    /* cells [e0, e0 + step, ..) of those the slices t0..t1 feed: n in [1, M],
+     * t in [t0-1, t1+1] (interior), within the window */
+    auto gather_cells = [&](int t0, int t1) -> int {
+        return (min(gt_hi, t1 + 1) - max(gt_lo, t0 - 1) + 1) * (gn_hi - gn_lo + 1);
+    };
+    auto gather = [&](int t0, int t1, int e0, int e1, int step) {
+        const int ta = max(gt_lo, t0 - 1);
         const int nn = gn_hi - gn_lo + 1;
-        const int cnt_c = (tb - ta + 1) * nn;
-        for (int e = threadIdx.x; e < cnt_c; e += NT) {
-            const int t = ta + e / nn;
-            const int n = gn_lo + e % nn;
+        for (int e = e0; e < e1; e += step) {
+            const int ts = e / nn;
+            const int t = ta + ts;
+            const int n = gn_lo + (e - ts * nn);
             const int a = aidx(n, t);
             if (EXACT) {
                 if (t - 1 >= t0 && t - 1 <= t1) { /* slice below: up-going parts */
@@ -427,34 +500,38 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
                  * increasing order, so the sums do not depend on where the band
                  * boundaries fall: every tile shape gives the same bits. A
                  * slice's per-cell record holds its flux difference N and the
-                 * up-going (U) and down-going (Dn) transverse parts. */
+                 * up-going (U) and down-going (Dn) transverse parts. The slice
+                 * below comes first: in the x sweep it starts the sums. */
+                double T[3];
                 if (t - 1 >= t0 && t - 1 <= t1) { /* slice below: up-going parts */
                     const double* r = crec(t - 1 - t0, n);
-                    ACCT[a] += half_dtdn * r[3];
-                    ACCT[a + MM] += half_dtdn * r[4];
-                    ACCT[a + 2 * MM] += half_dtdn * r[5];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                        T[c] = DIR == 0 ? gf_mul(half_dtdn, r[3 + c]) : fma(half_dtdn, r[3 + c], ACCT[a + c * MM]);
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) T[c] = ACCT[a + c * MM];
                 }
                 if (t >= t0 && t <= t1) {
                     const double* r = crec(t - t0, n);
-                    ACCN[a] += r[0];
-                    ACCN[a + MM] += r[1];
-                    ACCN[a + 2 * MM] += r[2];
-                    ACCT[a] += half_dtdn * (r[6] - r[3]);
-                    ACCT[a + MM] += half_dtdn * (r[7] - r[4]);
-                    ACCT[a + 2 * MM] += half_dtdn * (r[8] - r[5]);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        ACCN[a + c * MM] = DIR == 0 ? r[c] : gf_add(ACCN[a + c * MM], r[c]);
+                        T[c] = fma(half_dtdn, gf_sub(r[6 + c], r[3 + c]), T[c]);
+                    }
                 }
                 if (t + 1 >= t0 && t + 1 <= t1) { /* slice above: down-going parts */
                     const double* r = crec(t + 1 - t0, n);
-                    ACCT[a] -= half_dtdn * r[6];
-                    ACCT[a + MM] -= half_dtdn * r[7];
-                    ACCT[a + 2 * MM] -= half_dtdn * r[8];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) T[c] = fma(-half_dtdn, r[6 + c], T[c]);
                 }
+#pragma unroll
+                for (int c = 0; c < 3; ++c) ACCT[a + c * MM] = T[c];
             }
         }
     };
 
-    /* a2 / b2 both cells wet (list A by wave structure), a1 / b1 one wet,
-     * a0 / b0 both dry */
+    /* exact build: a2 / b2 both cells wet, a1 / b1 one wet, a0 / b0 both dry */
     auto counts_a = [&](int band, int& a2, int& a1, int& a0) {
         a2 = C(band, 0, 0) + C(band, 0, 1) + C(band, 0, 2);
         a1 = C(band, 0, 3);
@@ -467,7 +544,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
     };
 
     /* ---- stage A: normal Riemann solves, faces 0..M+2, by class ---- */
-    auto stage_a = [&](int t0, int band) {
+    auto stage_a_exact = [&](int t0, int band) {
         const uint16_t* lA = la + band * win.rb * fa;
         int a2, a1, a0;
         counts_a(band, a2, a1, a0);
@@ -484,24 +561,62 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
             const gf_cell cl = load_cell<DIR, EXACT, L>(sm, wet, cidx(n - 1, t));
             const gf_cell cr = load_cell<DIR, EXACT, L>(sm, wet, cidx(n, t));
             double s[3], fw[3][3];
-            gf_rpn2_face<FAST>(cl, cr, g, drytol, c16g, rsg, crit, crit2, s, fw);
+            gf_rpn2_face<false>(cl, cr, g, drytol, c16g, rsg, crit, crit2, s, fw);
 #pragma unroll
             for (int mw = 0; mw < 3; ++mw) {
                 w[mw] = s[mw];
                 w[3 + 3 * mw + 0] = fw[mw][0];
                 w[3 + 3 * mw + 1] = fw[mw][1];
                 w[3 + 3 * mw + 2] = fw[mw][2];
-                smax = d_max_nn<FAST>(smax, fabs(s[mw]));
+                smax = fmax(smax, fabs(s[mw]));
             }
         }
+    };
+    /* contracted build: faces 32 c .. 32 c + 31 of the band's list, in the
+     * order full solve, edge, smooth, dry: the longest first. A chunk with an
+     * edge face solves its smooth faces as edge faces too, not both ways. */
+    auto chunk_a = [&](int t0, int band, int c) {
+        const int ns = cnt[band * 6], ne = cnt[band * 6 + 1], nh = cnt[band * 6 + 2], nd = cnt[band * 6 + 3];
+        const int nA = ns + ne + nh + nd, idx = 32 * c + (int)(threadIdx.x & 31);
+        if (idx >= nA) return;
+        const uint16_t* lA = la + band * win.rb * fa;
+        const uint16_t* lM = lm + band * win.rb * fa;
+        const int v = idx < nh ? lM[nA - 1 - idx] : idx < nh + ne ? lM[idx - nh] : idx < nA - nd ? lA[idx - nh - ne] : lA[idx];
+        const int f = v & 0x7fff;
+        double* w = W + f * L::W_STRIDE;
+        if (idx >= nA - nd) { /* both cells dry: no waves */
+#pragma unroll
+            for (int q = 0; q < L::W_STRIDE; ++q) w[q] = 0.0;
+            return;
+        }
+        const int ts = f / fa;
+        const int t = t0 + ts;
+        const int n = win.na_lo + (f - ts * fa);
+        const gf_cell cl = load_cell<DIR, EXACT, L>(sm, wet, cidx(n - 1, t));
+        const gf_cell cr = load_cell<DIR, EXACT, L>(sm, wet, cidx(n, t));
+        if (idx < nh) {
+            full_solve(cl, cr, g, drytol, sc, w);
+#pragma unroll
+            for (int mw = 0; mw < 3; ++mw) smax = d_max_nn<FAST>(smax, fabs(w[mw]));
+            return;
+        }
+        double s[3], fw[3][3];
+        if (32 * c < nh + ne) gf_rpn2_edge(cl, cr, (v & 0x8000) != 0, g, crit, crit2, s, fw);
+        else gf_rpn2_smooth(cl, cr, g, s, fw);
+#pragma unroll
+        for (int mw = 0; mw < 3; ++mw) {
+            w[mw] = s[mw];
+            smax = d_max_nn<FAST>(smax, fabs(s[mw]));
+        }
+        w[3] = fw[0][0]; w[4] = fw[0][1]; w[5] = fw[0][2];
+        w[6] = fw[1][1];
+        w[7] = fw[2][0]; w[8] = fw[2][1]; w[9] = fw[2][2];
     };
 
     /* Fluctuations from the unlimited f-waves (rpn2_geoclaw.f:359-376) and
      * the limited second-order term cqxx of one face (flux2: limiter.f /
-     * philim.f and the correction loop). The middle f-wave is (0, beta2, 0) in
-     * local order: the contracted build skips its two zero components (adding
-     * +0.0 to a sum that starts at +0.0 changes no bits). */
-    auto face_terms = [&](const double* wc, double amdq[3], double apdq[3], double cq[3]) {
+     * philim.f and the correction loop), exact build. */
+    auto face_terms_exact = [&](const double* wc, double amdq[3], double apdq[3], double cq[3]) {
         double s[3], fw[3][3];
 #pragma unroll
         for (int mw = 0; mw < 3; ++mw) {
@@ -513,31 +628,9 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
         cq[0] = cq[1] = cq[2] = 0.0;
 #pragma unroll
         for (int mw = 0; mw < 3; ++mw) {
-            if (FAST && mw == 1) {
-                if (d_ltz<FAST>(s[1])) {
-                    amdq[1] += fw[1][1];
-                } else if (d_gtz<FAST>(s[1])) {
-                    apdq[1] += fw[1][1];
-                } else {
-                    amdq[1] += 0.5 * fw[1][1];
-                    apdq[1] += 0.5 * fw[1][1];
-                }
-                continue;
-            }
-            if (FAST && mw == 0) { /* into zero sums: assigned (a zero's sign aside) */
-                if (d_ltz<FAST>(s[0])) {
-                    amdq[0] = fw[0][0]; amdq[1] = fw[0][1]; amdq[2] = fw[0][2];
-                } else if (d_gtz<FAST>(s[0])) {
-                    apdq[0] = fw[0][0]; apdq[1] = fw[0][1]; apdq[2] = fw[0][2];
-                } else {
-                    amdq[0] = 0.5 * fw[0][0]; amdq[1] = 0.5 * fw[0][1]; amdq[2] = 0.5 * fw[0][2];
-                    apdq[0] = amdq[0]; apdq[1] = amdq[1]; apdq[2] = amdq[2];
-                }
-                continue;
-            }
-            if (d_ltz<FAST>(s[mw])) {
+            if (s[mw] < 0.0) {
                 amdq[0] += fw[mw][0]; amdq[1] += fw[mw][1]; amdq[2] += fw[mw][2];
-            } else if (d_gtz<FAST>(s[mw])) {
+            } else if (s[mw] > 0.0) {
                 apdq[0] += fw[mw][0]; apdq[1] += fw[mw][1]; apdq[2] += fw[mw][2];
             } else {
                 amdq[0] += 0.5 * fw[mw][0]; amdq[1] += 0.5 * fw[mw][1]; amdq[2] += 0.5 * fw[mw][2];
@@ -550,23 +643,6 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
 #pragma unroll
         for (int mw = 0; mw < 3; ++mw) {
             const double* fa = fw[mw];
-            if (FAST && mw == 1) {
-                /* the middle wave has one non-zero component: its norm and
-                 * projections are single products */
-                double lim = 1.0;
-                const double a = fa[1];
-                if (P.mthlim[1] != 0) {
-                    const double wnorm2 = a * a;
-                    if (!d_eqz<FAST>(wnorm2)) {
-                        /* the upwind neighbour's projection only */
-                        const double up = d_gtz<FAST>(s[1]) ? (wl + 3 + 3)[1] : (wr + 3 + 3)[1];
-                        lim = gf_philim<FAST>(wnorm2, up * a, P.mthlim[1]);
-                    }
-                }
-                const double fac = with_sign_of(1.0 - fabs(s[1]) * dtdn, s[1]);
-                cq[1] += (fac * lim) * a;
-                continue;
-            }
             double lim = 1.0;
             if (P.mthlim[mw] != 0) {
                 /* dot products in the global (h, hu, hv) order */
@@ -576,27 +652,84 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
                 const double l0 = ql[0], l1 = (DIR == 0) ? ql[1] : ql[2], l2 = (DIR == 0) ? ql[2] : ql[1];
                 const double r0 = qr[0], r1 = (DIR == 0) ? qr[1] : qr[2], r2 = (DIR == 0) ? qr[2] : qr[1];
                 const double wnorm2 = a0 * a0 + a1 * a1 + a2 * a2;
-                if (!d_eqz<FAST>(wnorm2)) {
+                if (wnorm2 != 0.0) {
                     /* the upwind neighbour's projection only (the same
                      * products in the same order) */
-                    const bool up = d_gtz<FAST>(s[mw]);
+                    const bool up = s[mw] > 0.0;
                     const double p0 = up ? l0 : r0, p1 = up ? l1 : r1, p2 = up ? l2 : r2;
                     const double dot = p0 * a0 + p1 * a1 + p2 * a2;
-                    lim = gf_philim<FAST>(wnorm2, dot, P.mthlim[mw]);
+                    lim = gf_philim<false>(wnorm2, dot, P.mthlim[mw]);
                 }
             }
-            const double fac = FAST ? with_sign_of(1.0 - fabs(s[mw]) * dtdn, s[mw])
-                                    : copysign(1.0, s[mw]) * (1.0 - fabs(s[mw]) * dtdn);
-            if (FAST) {
-                const double fl = fac * lim;
-                cq[0] += fl * fa[0];
-                cq[1] += fl * fa[1];
-                cq[2] += fl * fa[2];
-            } else {
-                cq[0] += fac * (lim * fa[0]);
-                cq[1] += fac * (lim * fa[1]);
-                cq[2] += fac * (lim * fa[2]);
+            const double fac = copysign(1.0, s[mw]) * (1.0 - fabs(s[mw]) * dtdn);
+            cq[0] += fac * (lim * fa[0]);
+            cq[1] += fac * (lim * fa[1]);
+            cq[2] += fac * (lim * fa[2]);
+        }
+    };
+
+    /* The same in the contracted build, on its shorter face records (the
+     * middle f-wave is (0, beta2, 0) in local order). Only the upwind neighbour's
+     * projection is formed; the middle wave's ratio of projection and norm is
+     * the quotient of the two beta2. */
+    auto face_terms_fast = [&](const double* wc, double amdq[3], double apdq[3], double cq[3]) {
+        constexpr bool F = true;
+        const double s0 = wc[0], s1 = wc[1], s2 = wc[2];
+        const double f0[3] = {wc[3], wc[4], wc[5]}, f1 = wc[6], f2[3] = {wc[7], wc[8], wc[9]};
+        if (d_ltz<F>(s0) && d_gtz<F>(s2)) { /* one outer wave each way: no sums */
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                amdq[c] = f0[c];
+                apdq[c] = f2[c];
             }
+        } else {
+            const double w0m = d_ltz<F>(s0) ? 1.0 : d_gtz<F>(s0) ? 0.0 : 0.5;
+            const double w2m = d_ltz<F>(s2) ? 1.0 : d_gtz<F>(s2) ? 0.0 : 0.5;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                amdq[c] = fma(w0m, f0[c], gf_mul(w2m, f2[c]));
+                apdq[c] = fma(1.0 - w0m, f0[c], gf_mul(1.0 - w2m, f2[c]));
+            }
+        }
+        if (d_eqz<F>(s1)) {
+            amdq[1] = fma(0.5, f1, amdq[1]);
+            apdq[1] = fma(0.5, f1, apdq[1]);
+        } else {
+            const bool l = d_ltz<F>(s1);
+            const double v = gf_add(l ? amdq[1] : apdq[1], f1);
+            amdq[1] = l ? v : amdq[1];
+            apdq[1] = l ? apdq[1] : v;
+        }
+        cq[0] = cq[1] = cq[2] = 0.0;
+        if (P.order == 1) return;
+        auto outer = [&](double s, const double* fa, int at, int meth) -> double { /* waves 0 and 2 */
+            double lim = 1.0;
+            if (meth != 0) {
+                const double* pw = (d_gtz<F>(s) ? wc - L::W_STRIDE : wc + L::W_STRIDE) + at;
+                const double wnorm2 = fma(fa[2], fa[2], fma(fa[1], fa[1], gf_mul(fa[0], fa[0])));
+                if (gf_pos_normal(wnorm2))
+                    lim = gf_philim<F>(wnorm2, fma(pw[2], fa[2], fma(pw[1], fa[1], gf_mul(pw[0], fa[0]))), meth);
+            }
+            return gf_mul(with_sign_of(fma(-fabs(s), dtdn, 1.0), s), lim);
+        };
+        {
+            const double fl = outer(s0, f0, 3, P.mthlim[0]);
+            cq[0] = gf_mul(fl, f0[0]); cq[1] = gf_mul(fl, f0[1]); cq[2] = gf_mul(fl, f0[2]);
+        }
+        {
+            double lim = 1.0;
+            if (P.mthlim[1] != 0 && gf_pos_normal(fabs(f1))) {
+                const double up = (d_gtz<F>(s1) ? wc - L::W_STRIDE : wc + L::W_STRIDE)[6];
+                /* MC: opposite signs, or no upwind wave, give zero without the quotient */
+                lim = P.mthlim[1] == 4 && (d_eqz<F>(up) || opposite_signs(up, f1))
+                          ? 0.0
+                          : gf_philim_r<F>(d_div<F>(up, f1), P.mthlim[1]);
+            }
+            cq[1] = fma(gf_mul(with_sign_of(fma(-fabs(s1), dtdn, 1.0), s1), lim), f1, cq[1]);
+        }
+        {
+            const double fl = outer(s2, f2, 7, P.mthlim[2]);
+            cq[0] = fma(fl, f2[0], cq[0]); cq[1] = fma(fl, f2[1], cq[1]); cq[2] = fma(fl, f2[2], cq[2]);
         }
     };
 
@@ -619,7 +752,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
             const int kl = cidx(n - 1, t), kr = cidx(n, t);
             const double* wc = W + ((t - t0) * fa + (n - win.na_lo)) * L::W_STRIDE;
             double amdq[3], apdq[3], cq[3];
-            face_terms(wc, amdq, apdq, cq);
+            face_terms_exact(wc, amdq, apdq, cq);
             double faddm[3] = {amdq[0], amdq[1], amdq[2]};
             double faddp[3] = {-apdq[0], -apdq[1], -apdq[2]};
             if (P.order != 1) {
@@ -641,7 +774,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
                 double bm[3], bp[3];
                 if (wet[kl]) { /* rpt2 imp=1: left-going part into cell n-1 */
                     const gf_cell cl = load_cell<DIR, EXACT, L>(sm, wet, kl);
-                    gf_rpt2_face<FAST>(cl, sm[L::OFF_B + cidx(n - 1, t - 1)],
+                    gf_rpt2_face(cl, sm[L::OFF_B + cidx(n - 1, t - 1)],
                                        sm[L::OFF_B + cidx(n - 1, t + 1)], drytol, amdq, bm, bp);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
@@ -651,7 +784,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
                 }
                 if (wet[kr]) { /* rpt2 imp=2: right-going part into cell n */
                     const gf_cell cr = load_cell<DIR, EXACT, L>(sm, wet, kr);
-                    gf_rpt2_face<FAST>(cr, sm[L::OFF_B + cidx(n, t - 1)],
+                    gf_rpt2_face(cr, sm[L::OFF_B + cidx(n, t - 1)],
                                        sm[L::OFF_B + cidx(n, t + 1)], drytol, apdq, bm, bp);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
@@ -672,29 +805,28 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
 
     /* ---- contracted build, stage B1: per limited face, the fluctuations
      * amdq, apdq and the limited second-order term cq (local order) ---- */
-    auto stage_b1 = [&](int t0, int band) {
+    auto chunk_b1 = [&](int band, int c) {
         const uint16_t* lB = lb + band * win.rb * fb;
-        int b2, b1, b0;
-        counts_b(band, b2, b1, b0);
-        for (int idx = threadIdx.x; idx < b2 + b1 + b0; idx += NT) {
-            const int f = lB[idx];
-            double* o = O + f * L::O_STRIDE;
-            if (idx >= b2 + b1) {
+        const int nw = cnt[band * 6 + 4], nB = nw + cnt[band * 6 + 5];
+        const int idx = 32 * c + (int)(threadIdx.x & 31);
+        if (idx >= nB) return;
+        const int f = lB[idx];
+        double* o = O + f * L::O_STRIDE;
+        if (idx >= nw) {
 #pragma unroll
-                for (int q = 0; q < L::O_STRIDE; ++q) o[q] = 0.0;
-                continue;
-            }
-            const int t = t0 + f / fb;
-            const int n = win.nb_lo + f % fb;
-            const double* wc = W + ((t - t0) * fa + (n - win.na_lo)) * L::W_STRIDE;
-            double amdq[3], apdq[3], cq[3];
-            face_terms(wc, amdq, apdq, cq);
+            for (int q = 0; q < L::O_STRIDE; ++q) o[q] = 0.0;
+            return;
+        }
+        const int ts = f / fb;
+        const int n = win.nb_lo + (f - ts * fb);
+        const double* wc = W + (ts * fa + (n - win.na_lo)) * L::W_STRIDE;
+        double amdq[3], apdq[3], cq[3];
+        face_terms_fast(wc, amdq, apdq, cq);
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                o[c] = amdq[c];
-                o[3 + c] = apdq[c];
-                o[6 + c] = cq[c];
-            }
+        for (int k = 0; k < 3; ++k) {
+            o[k] = amdq[k];
+            o[3 + k] = apdq[k];
+            o[6 + k] = cq[k];
         }
     };
 
@@ -708,12 +840,12 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
      * P + Q (P for transverse = 1): bm is the down-going part Dn, bp the
      * up-going part U, equal to the sum of the reference's two splits up to
      * rounding. ---- */
-    auto stage_b2 = [&](int t0, int t1) {
+    auto chunk_b2 = [&](int t0, int t1, int c) {
         const int ncell = fb - 1;
-        const int cnt_c = (t1 - t0 + 1) * ncell;
-        for (int e = threadIdx.x; e < cnt_c; e += NT) {
+        const int e = 32 * c + (int)(threadIdx.x & 31);
+        if (e < (t1 - t0 + 1) * ncell) {
             const int ts = e / ncell;
-            const int n = win.nb_lo + e % ncell;
+            const int n = win.nb_lo + (e - ts * ncell);
             const int t = t0 + ts;
             const int k = cidx(n, t);
             double* r = crec(ts, n);
@@ -721,25 +853,24 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
                 /* faces n and n+1 both between dry cells: no waves */
 #pragma unroll
                 for (int q = 0; q < L::C_STRIDE; ++q) r[q] = 0.0;
-                continue;
+                return;
             }
             const double* orr = O + (ts * fb + (n + 1 - win.nb_lo)) * L::O_STRIDE; /* face n+1 */
             const double* orl = O + (ts * fb + (n - win.nb_lo)) * L::O_STRIDE;     /* face n   */
             double Pv[3], Qv[3], Nv[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                Pv[c] = orr[c] + orl[3 + c];
-                Qv[c] = orr[6 + c] - orl[6 + c];
-                Nv[c] = Pv[c] + 0.5 * Qv[c];
+            for (int q = 0; q < 3; ++q) {
+                Pv[q] = gf_add(orr[q], orl[3 + q]);
+                Qv[q] = gf_sub(orr[6 + q], orl[6 + q]);
+                Nv[q] = fma(0.5, Qv[q], Pv[q]);
             }
             double bm[3] = {0.0, 0.0, 0.0}, bp[3] = {0.0, 0.0, 0.0};
             if (P.transverse != 0 && wet[k]) {
                 double x[3];
 #pragma unroll
-                for (int c = 0; c < 3; ++c) x[c] = P.transverse == 2 ? Pv[c] + Qv[c] : Pv[c];
+                for (int q = 0; q < 3; ++q) x[q] = P.transverse == 2 ? gf_add(Pv[q], Qv[q]) : Pv[q];
                 const gf_cell cc = load_cell<DIR, EXACT, L>(sm, wet, k);
-                gf_rpt2_face<FAST>(cc, sm[L::OFF_B + cidx(n, t - 1)], sm[L::OFF_B + cidx(n, t + 1)], drytol, x,
-                                   bm, bp);
+                gf_rpt2_fast(cc, sm[L::OFF_B + cidx(n, t - 1)], sm[L::OFF_B + cidx(n, t + 1)], x, bm, bp);
             }
             /* global component order (h, hu, hv) */
             r[0] = Nv[0]; r[G1] = Nv[1]; r[G2] = Nv[2];
@@ -750,49 +881,77 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, in
 
     const int ts_end = win.ts_lo + win.nsl;
     int prev_t0 = -1, prev_t1 = -1;
-    if (EXACT) {
+    if constexpr (EXACT) {
+        auto gather_all = [&](int ta, int tb) { gather(ta, tb, threadIdx.x, gather_cells(ta, tb), NT); };
         for (int t0 = win.ts_lo, band = 0; t0 < ts_end; t0 += win.rb, ++band) {
             const int t1 = min(t0 + win.rb, ts_end) - 1; /* last slice of band */
-            stage_a(t0, band);
-            if (prev_t0 >= 0) gather(prev_t0, prev_t1);
+            stage_a_exact(t0, band);
+            if (prev_t0 >= 0) gather_all(prev_t0, prev_t1);
             __syncthreads();
             stage_b_exact(t0, band);
             __syncthreads();
             prev_t0 = t0;
             prev_t1 = t1;
         }
-        gather(prev_t0, prev_t1);
+        gather_all(prev_t0, prev_t1);
         __syncthreads();
-        return smax;
-    }
-    /* Contracted build, pipelined over bands with two barriers per band:
-     * [stage A of band b | B2 of band b-1], [B1 of band b | gather of band
-     * b-1]. Each stage reads what the phase before the last barrier wrote. */
-    for (int t0 = win.ts_lo, band = 0;; t0 += win.rb, ++band) {
-        const bool have = t0 < ts_end;
-        const int t1 = have ? min(t0 + win.rb, ts_end) - 1 : -1;
-        if (have) stage_a(t0, band);
-        if (prev_t0 >= 0) stage_b2(prev_t0, prev_t1);
-        __syncthreads();
-        if (have) stage_b1(t0, band);
-        if (prev_t0 >= 0) gather(prev_t0, prev_t1);
-        __syncthreads();
-        if (!have) break;
-        prev_t0 = t0;
-        prev_t1 = t1;
+    } else {
+        /* Contracted build, pipelined over bands with two barriers per band:
+         * [stage A of band b | B2 of band b-1], [B1 of band b | gather of band
+         * b-1]. Each stage reads what the phase before the last barrier wrote.
+         * A warp takes the next 32 items of a phase from its cursor, the
+         * costly stage first: warps (and the four schedulers, each with an
+         * FP64 pipe of its own) that got short items take more of them. The
+         * lists' chunks run beside the solves, off the FP64 pipe. */
+        int* cur = ls.cur;
+        auto next = [&](int phase) -> int {
+            int c = 0;
+            if ((threadIdx.x & 31) == 0) c = atomicAdd(&cur[phase], 1);
+            return __shfl_sync(0xffffffffu, c, 0);
+        };
+        for (int t0 = win.ts_lo, band = 0;; t0 += win.rb, ++band) {
+            const bool have = t0 < ts_end;
+            const int t1 = have ? min(t0 + win.rb, ts_end) - 1 : -1;
+            const int nsl = t1 - t0 + 1, psl = prev_t0 >= 0 ? prev_t1 - prev_t0 + 1 : 0;
+            const int ca = have ? (nsl * fa + 31) / 32 : 0, c2 = (psl * (fb - 1) + 31) / 32;
+            const int sa = side.count(2 * band);
+            for (int c; (c = next(2 * band)) < ca + sa + c2;) {
+                if (c < ca) chunk_a(t0, band, c);
+                else if (c < ca + sa) side.run(2 * band, c - ca);
+                else chunk_b2(prev_t0, prev_t1, c - ca - sa);
+            }
+            __syncthreads();
+            const int c1 = have ? (nsl * fb + 31) / 32 : 0;
+            const int ng = psl ? gather_cells(prev_t0, prev_t1) : 0, cg = (ng + 31) / 32;
+            const int sb = side.count(2 * band + 1);
+            for (int c; (c = next(2 * band + 1)) < c1 + sb + cg;) {
+                if (c < c1) {
+                    chunk_b1(band, c);
+                } else if (c < c1 + sb) {
+                    side.run(2 * band + 1, c - c1);
+                } else {
+                    const int e0 = 32 * (c - c1 - sb);
+                    gather(prev_t0, prev_t1, e0 + (int)(threadIdx.x & 31), min(ng, e0 + 32), 32);
+                }
+            }
+            __syncthreads();
+            if (!have) break;
+            prev_t0 = t0;
+            prev_t1 = t1;
+        }
     }
     return smax;
 }
 
 /* Manning friction source term on one interior cell (geoclaw_src2_fort.f90:41-71).
- * The contracted build forms h^(-7/3) = y^7 from y = h^(-1/3) and one
- * reciprocal of 1 + dt gamma instead of pow and three divisions: y by
- * Newton's iteration for the inverse cube root, y <- y + y (1 - h y^3) / 3,
- * two steps from the single-precision value (each step doubles the correct
- * bits, 23 -> 46 -> the FP64 rounding), so no FP64 division or cube root
- * is taken. */
+ * The contracted build forms h^(-7/3) and one reciprocal of 1 + dt gamma
+ * instead of pow and three divisions: from the single-precision y0 of
+ * h^(-1/3), one third-order step of the binomial series,
+ * y0^7 (1 - e)^(-7/3) = y0^7 (1 + 7 e/3 + 35 e^2/9 + ...), e = 1 - h y0^3
+ * (23 bits -> past the FP64 rounding): no FP64 division, cube root or
+ * conversion is taken. */
 template <bool FAST>
-__device__ __forceinline__ void src2_cell(const gf_phys& P, double dt, double bathy, double nvar,
+__device__ __forceinline__ void src2_cell(const gf_phys& P, double dt, const double* kf, double bathy, double nvar,
                                           double& h, double& hu, double& hv)
 {
     if (!P.friction_forcing) return;
@@ -800,27 +959,26 @@ __device__ __forceinline__ void src2_cell(const gf_phys& P, double dt, double ba
         hu = 0.0;
         hv = 0.0;
     } else if (h <= P.friction_depth) {
+        /* coefficient, or in the contracted build dt g coefficient^2 (kf: of
+         * the Manning table) */
         double coeff = 0.0;
         if (!P.variable_friction) {
             for (int nman = P.num_manning; nman >= 1; --nman)
-                if (bathy < P.manning_break[nman - 1]) coeff = P.manning_coefficient[nman - 1];
+                if (bathy < P.manning_break[nman - 1]) coeff = FAST ? kf[nman - 1] : P.manning_coefficient[nman - 1];
         } else {
-            coeff = nvar;
+            coeff = FAST ? gf_mul(gf_mul(dt, P.grav), gf_mul(nvar, nvar)) : nvar;
         }
         if (FAST) {
             /* 1e-30 <= h here: a normal single-precision number */
-            double y = (double)rcbrtf((float)h);
-#pragma unroll
-            for (int it = 0; it < 2; ++it) {
-                const double e = fma(-h, (y * y) * y, 1.0);
-                y = fma(y * (1.0 / 3.0), e, y);
-            }
-            const double y2 = y * y;
-            const double hm73 = ((y2 * y2) * y2) * y; /* h^(-7/3) */
-            const double gamma = d_sqrt<FAST>(hu * hu + hv * hv) * P.grav * (coeff * coeff) * hm73;
-            const double rdg = gf_rcp(1.0 + dt * gamma);
-            hu = hu * rdg;
-            hv = hv * rdg;
+            const double y0 = gf_f64_pos(rcbrtf(gf_f32(h)));
+            const double y3 = gf_mul(gf_mul(y0, y0), y0);
+            const double e = fma(-h, y3, 1.0);
+            const double y7 = gf_mul(gf_mul(y3, y3), y0);
+            const double hm73 = fma(gf_mul(y7, e), fma(35.0 / 9.0, e, 7.0 / 3.0), y7); /* h^(-7/3) */
+            const double mom = d_sqrt<FAST>(fma(hu, hu, gf_mul(hv, hv)));
+            const double rdg = gf_rcp(fma(gf_mul(mom, coeff), hm73, 1.0));
+            hu = gf_mul(hu, rdg);
+            hv = gf_mul(hv, rdg);
         } else {
             const double gamma =
                 sqrt(hu * hu + hv * hv) * P.grav * (coeff * coeff) / pow(h, 7.0 / 3.0);
@@ -850,10 +1008,10 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
     constexpr int S = G::S;
     constexpr bool FAST = !EXACT;
     int* cnt = reinterpret_cast<int*>(sm + L::OFF_INT);
-    uint16_t* la = reinterpret_cast<uint16_t*>(cnt + L::CNT_INTS);
-    uint16_t* lb = la + L::LIST_A;
+    uint16_t* lists = reinterpret_cast<uint16_t*>(cnt + L::CNT_INTS);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned char* wet = reinterpret_cast<unsigned char*>(sm) + L::OFF_WET_BYTES;
-    double* red = sm + L::OFF_RED;
+    double* sc = sm + L::OFF_SC;
 
     const double dt = group_dt ? group_dt[wk.group] : dt_uniform;
     /* a group with no step this round (dt <= 0) is skipped as a whole */
@@ -871,7 +1029,14 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
 
     /* after a wait of this launch (or an earlier one of the same step) gave
      * up, the step has failed: later items leave at once */
-    if (__syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<volatile int*>(err) != 0)) return false;
+    const bool failed = __syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<volatile int*>(err) != 0);
+    if (failed) {
+        if (part) {
+            cluster_arrive();
+            cluster_wait();
+        }
+        return false;
+    }
 
     /* ---- stage the patch (h, hu, hv planes and b) with bulk copies ---- */
     if (threadIdx.x == 0) {
@@ -881,14 +1046,37 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
     }
     const uint32_t ph = phase;
     phase ^= 1u;
-    if (!__syncthreads_and(mbar_wait(bar, ph, kWaitPolls))) {
+    const bool staged = __syncthreads_and(mbar_wait(bar, ph, kWaitPolls));
+    if (!staged) {
         if (threadIdx.x == 0) atomicExch(err, 1);
         mbar_wait(bar, ph, kWaitPolls); /* let any copy in flight land */
+    }
+    /* the CTAs of a split item update it in place: none writes before all have staged it */
+    if (part) cluster_arrive();
+    if (!staged) {
+        if (part) cluster_wait();
         return false;
     }
 
     /* ---- b4step2 on all cells + per-cell quotients ---- */
     int any_wet = 0, changed = 0;
+    if (warp == NT / 32 - 1) {
+        /* the item's constants, one lane each: formed by every thread they
+         * would cost as much FP64 time as a band's limiter */
+        const double q = (lane < 2 ? dt : 1.0) / (lane == 0 ? wk.dx : lane == 1 ? wk.dy : 16.0 * g);
+        if (lane < 3) sc[SC_DTDX + lane] = q;
+        if (lane == 3) sc[SC_RSG] = rsqrt(g);
+        if (lane == 4) {
+            const double crit = fmax(drytol * g, 1e-6);
+            sc[SC_CRIT] = crit;
+            sc[SC_CRIT2] = sqrt(crit);
+        }
+        if (lane >= 8 && lane < 8 + GF_MAX_MANNING) {
+            const double n = P.manning_coefficient[lane - 8];
+            sc[SC_KF + lane - 8] = (dt * g) * (n * n);
+        }
+        if (lane == 16) sc[SC_CFL] = 0.0;
+    }
     for (int k = threadIdx.x; k < S; k += NT) {
         double h = sm[L::OFF_H + k];
         if (d_lt<FAST>(h, drytol)) {
@@ -903,15 +1091,15 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         const bool w = d_gt<FAST>(h, drytol);
         wet[k] = w ? 1 : 0;
         any_wet |= w;
-        double u = 0.0, v = 0.0, c = 0.0, rh = 0.0, rc = 0.0;
+        double u = 0.0, v = 0.0, c = 0.0, rc = 0.0;
         if (w) {
             if (FAST) {
                 /* rc^2 = 1 / (g h), so 1 / h = g rc^2 within a few ulps:
                  * two products instead of a reciprocal */
                 const double gh = g * h;
-                rc = rsqrt(gh);
+                rc = gf_pos_normal(gh) ? gf_rsqrt_n(gh) : rsqrt(gh);
                 c = gh * rc;
-                rh = g * (rc * rc);
+                const double rh = g * (rc * rc);
                 u = sm[L::OFF_HU + k] * rh;
                 v = sm[L::OFF_HV + k] * rh;
             } else {
@@ -923,27 +1111,79 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         sm[L::OFF_U + k] = u;
         sm[L::OFF_V + k] = v;
         sm[L::OFF_C + k] = c;
-        if (FAST) {
-            sm[L::OFF_RH + k] = rh;
-            sm[L::OFF_RC + k] = rc;
-        }
+        if (FAST) sm[L::OFF_RC + k] = rc;
     }
-    for (int k = threadIdx.x; k < L::NACC * 3 * L::PLANE; k += NT) sm[L::OFF_ACC + k] = 0.0;
+    if (EXACT)
+        for (int k = threadIdx.x; k < L::NACC * 3 * L::PLANE; k += NT) sm[L::OFF_ACC + k] = 0.0;
+    else
+        for (int k = threadIdx.x; k < L::CNT_INTS; k += NT) cnt[k] = 0;
     any_wet = __syncthreads_or(any_wet);
     if (wk.fl) changed = __syncthreads_or(changed);
 
-    const double dtdx = dt / wk.dx, dtdy = dt / wk.dy;
+    const double dtdx = sc[SC_DTDX], dtdy = sc[SC_DTDY];
     double smax_x = 0.0, smax_y = 0.0;
     if (any_wet) {
-        const double c16g = 1.0 / (16.0 * g);
-        const double rsg = rsqrt(g);
-        const double crit = fmax(drytol * g, 1e-6);
-        const double crit2 = sqrt(crit);
-        smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, cnt, la, lb, P, dtdx, c16g, rsg, crit, crit2, rlo, rhi);
-        smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, cnt, la, lb, P, dtdy, c16g, rsg, crit, crit2, rlo, rhi);
+        if constexpr (EXACT) {
+            struct {
+                __device__ int count(int) const { return 0; }
+                __device__ void run(int, int) const {}
+            } none;
+            const SweepLists ls = {cnt, nullptr, lists, lists + L::LIST_A, nullptr};
+            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, ls, P, rlo, rhi, none);
+            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, ls, P, rlo, rhi, none);
+        } else {
+            /* The x sweep's first band is listed before it, every next band's
+             * faces during the band before, and the y sweep's spread over all
+             * phases of the x sweep. */
+            struct Side {
+                const double* sm;
+                const unsigned char* wet;
+                SweepLists x, y;
+                SweepWin<M, RB, 0> wx;
+                SweepWin<M, RB, 1> wy;
+                double g, crit, crit2;
+                int nbx, ncx, ncy, ny; /* x bands, chunks of a band of x and y, chunks of y */
+                __device__ __forceinline__ int xs(int p) const
+                {
+                    return (p >> 1) + 1 < nbx ? ((p & 1) ? ncx - ncx / 2 : ncx / 2) : 0;
+                }
+                __device__ __forceinline__ int y0(int p) const { return min(p, 2 * nbx) * ny / (2 * nbx); }
+                __device__ __forceinline__ int count(int p) const { return xs(p) + y0(p + 1) - y0(p); }
+                __device__ __forceinline__ void run(int p, int c) const
+                {
+                    const int nx = xs(p);
+                    if (c < nx) {
+                        list_chunk<M, RB, 0>(sm, wet, x, g, crit, crit2, wx, (p >> 1) + 1, (p & 1) ? ncx / 2 + c : c);
+                    } else {
+                        const int e = y0(p) + c - nx, band = e / ncy;
+                        list_chunk<M, RB, 1>(sm, wet, y, g, crit, crit2, wy, band, e - band * ncy);
+                    }
+                }
+            };
+            struct None {
+                __device__ __forceinline__ int count(int) const { return 0; }
+                __device__ __forceinline__ void run(int, int) const {}
+            };
+            auto lists_of = [&](int d) -> SweepLists {
+                uint16_t* p = lists + d * L::LIST_SWEEP;
+                return {cnt + d * L::CNT_SWEEP, cnt + L::CNT_CUR + d * L::CUR_SWEEP, p, p + L::LIST_A,
+                        p + L::LIST_A + L::LIST_B};
+            };
+            const SweepWin<M, RB, 0> wx(rlo, rhi);
+            const SweepWin<M, RB, 1> wy(rlo, rhi);
+            Side side = {sm, wet, lists_of(0), lists_of(1), wx, wy, g, sc[SC_CRIT], sc[SC_CRIT2],
+                         (wx.nsl + wx.rb - 1) / wx.rb, (wx.rb * wx.fa + 31) / 32, (wy.rb * wy.fa + 31) / 32, 0};
+            side.ny = (wy.nsl + wy.rb - 1) / wy.rb * side.ncy;
+            for (int c = warp; c < side.ncx; c += NT / 32)
+                list_chunk<M, RB, 0>(sm, wet, side.x, g, side.crit, side.crit2, wx, 0, c);
+            __syncthreads();
+            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, side.x, P, rlo, rhi, side);
+            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, side.y, P, rlo, rhi, None());
+        }
     }
 
     /* ---- flux-difference update, src2, write interior ---- */
+    if (part) cluster_wait();
     double* gq = wk.qout ? wk.qout : wk.q;
     const double* gaux = wk.aux;
     const int fidx = P.friction_index - 1;
@@ -962,18 +1202,18 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
             h = h - dtdx * (FM[a] - FP[a]) - dtdy * (GM[a] - GP[a]);
             hu = hu - dtdx * (FM[a + PL] - FP[a + PL]) - dtdy * (GM[a + PL] - GP[a + PL]);
             hv = hv - dtdx * (FM[a + 2 * PL] - FP[a + 2 * PL]) - dtdy * (GM[a + 2 * PL] - GP[a + 2 * PL]);
-        } else {
+        } else if (any_wet) {
             const double* DX = sm + L::OFF_ACC;
             const double* DY = sm + L::OFF_ACC + 3 * PL;
-            h = h - dtdx * DX[a] - dtdy * DY[a];
-            hu = hu - dtdx * DX[a + PL] - dtdy * DY[a + PL];
-            hv = hv - dtdx * DX[a + 2 * PL] - dtdy * DY[a + 2 * PL];
+            h = fma(-dtdy, DY[a], fma(-dtdx, DX[a], h));
+            hu = fma(-dtdy, DY[a + PL], fma(-dtdx, DX[a + PL], hu));
+            hv = fma(-dtdy, DY[a + 2 * PL], fma(-dtdx, DX[a + 2 * PL], hv));
         }
         if (P.src_term > 0) {
             const double nvar = (P.variable_friction && fidx >= 0 && fidx < maux)
                                     ? gaux[(size_t)fidx * S + k]
                                     : 0.0;
-            src2_cell<FAST>(P, dt, sm[L::OFF_B + k], nvar, h, hu, hv);
+            src2_cell<FAST>(P, dt, sc + SC_KF, sm[L::OFF_B + k], nvar, h, hu, hv);
         }
         gq[k] = h;
         gq[S + k] = hu;
@@ -985,42 +1225,26 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         wk.fl->wet = any_wet ? 1 : 0;
     }
 
-    /* ---- CFL: warp-shuffle max, then across warps ---- */
-    double cx = smax_x, cy = smax_y;
+    /* ---- CFL: the largest of dt/dx |s| and dt/dy |s|, over the warp, then over
+     * the CTA, on the integer pipe (non-negative doubles order as integers);
+     * a NaN speed is left out ---- */
+    {
+        auto number = [](double x) -> double {
+            return __double_as_longlong(x) <= 0x7ff0000000000000ll ? x : 0.0;
+        };
+        unsigned long long v = dkey(d_max_nn<true>(dtdx * number(smax_x), dtdy * number(smax_y)));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        cx = fmax(cx, __shfl_xor_sync(0xffffffffu, cx, o));
-        cy = fmax(cy, __shfl_xor_sync(0xffffffffu, cy, o));
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        red[warp] = cx;
-        red[32 + warp] = cy;
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
+            v = w > v ? w : v;
+        }
+        if (lane == 0) atomicMax(reinterpret_cast<unsigned long long*>(sc + SC_CFL), v);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double mx = 0.0, my = 0.0;
-        for (int w2 = 0; w2 < NT / 32; ++w2) {
-            mx = fmax(mx, red[w2]);
-            my = fmax(my, red[32 + w2]);
-        }
-        if (part) { /* a window of a split item: the cluster forms the patch CFL */
-            part[0] = mx;
-            part[1] = my;
-        }
-    }
-    if (part) {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncthreads();
-        return true;
-    }
-    if (threadIdx.x == 0) {
-        double mx = 0.0, my = 0.0;
-        for (int w2 = 0; w2 < NT / 32; ++w2) {
-            mx = fmax(mx, red[w2]);
-            my = fmax(my, red[32 + w2]);
-        }
-        double cfl = fmax(dtdx * mx, dtdy * my);
+    if (part) { /* a window of a split item: the cluster forms the patch CFL */
+        if (threadIdx.x == 0) *part = sc[SC_CFL];
+    } else if (threadIdx.x == 0) {
+        double cfl = sc[SC_CFL];
         if (cfl > P.maxcfl_cap) cfl = 0.0;
         if (cfl_out) cfl_out[wi] = cfl;
         if (group_max) atomicMax(group_max + wk.group, dkey(cfl));
@@ -1080,11 +1304,10 @@ __global__ void __cluster_dims__(K, 1, 1) __launch_bounds__(NT, 1)
     const int r = (int)cluster.block_rank();
     const int wi = blockIdx.x / K;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::OFF_BAR);
-    double* part = sm + L::OFF_RED + 62; /* past the warp slots of the CFL reduction */
+    double* part = sm + L::OFF_SC + SC_PART;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
-        part[0] = 0.0;
-        part[1] = 0.0;
+        *part = 0.0;
     }
     __syncthreads();
     /* both tests are the same on every CTA of the cluster: it leaves whole */
@@ -1097,17 +1320,9 @@ __global__ void __cluster_dims__(K, 1, 1) __launch_bounds__(NT, 1)
                                  maux, cfl_out, group_max, err, 1 + r * R, (r + 1) * R, part);
     cluster.sync();
     if (r == 0 && threadIdx.x == 0) {
-        double mx = 0.0, my = 0.0;
-        for (int q = 0; q < K; ++q) {
-            const double* p = cluster.map_shared_rank(part, q);
-            mx = fmax(mx, p[0]);
-            my = fmax(my, p[1]);
-        }
-        const gf_phys& P = phys_table[wk.phys];
-        const double dt = group_dt ? group_dt[wk.group] : dt_uniform;
-        const double dtdx = dt / wk.dx, dtdy = dt / wk.dy;
-        double cfl = fmax(dtdx * mx, dtdy * my);
-        if (cfl > P.maxcfl_cap) cfl = 0.0;
+        double cfl = 0.0;
+        for (int q = 0; q < K; ++q) cfl = d_max_nn<true>(cfl, *cluster.map_shared_rank(part, q));
+        if (cfl > phys_table[wk.phys].maxcfl_cap) cfl = 0.0;
         if (cfl_out) cfl_out[wi] = cfl;
         if (group_max) atomicMax(group_max + wk.group, dkey(cfl));
     }

@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(M) qad_kernel(const gf_qad_dev_task* __restric
             Rc.un = Rc.wet ? Rc.hun / hr : 0.0;
             Rc.ut = Rc.wet ? Rc.hut / hr : 0.0;
             Rc.c = Rc.wet ? sqrt(g * hr) : 0.0;
-            Lc.rh = Lc.rc = Rc.rh = Rc.rc = 0.0;
+            Lc.rc = Rc.rc = 0.0;
             const double c16g = 1.0 / (16.0 * g);
             const double rsg = rsqrt(g);
             const double crit = fmax(drytol * g, 1e-6);
