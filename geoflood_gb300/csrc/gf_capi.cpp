@@ -1338,8 +1338,7 @@ extern "C" int gf_autotune(gf_ctx* c, int reps, gf_tile_result* out)
             result = cuda_fail(c, e, "autotune");
             break;
         }
-        gf::tile_set(m, 0, R.best_throughput);
-        gf::tile_set(m, 1, R.best_latency);
+        gf::tile_install_tuned(m, R.best_throughput, R.best_latency);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

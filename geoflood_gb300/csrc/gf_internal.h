@@ -63,6 +63,7 @@ int tile_get(int m, int goal);
  * cluster of CTAs) are all resident at once on the device, else 0 */
 int latency_goal_fits(int m, long npatch);
 int tile_set(int m, int goal, int v);
+void tile_install_tuned(int m, int throughput, int latency);
 cudaError_t launch_patch_update_tile(int m, int v, const gf_patch_work* work, int nwork,
                                      const gf_phys* phys, double dt, const double* gdt,
                                      const int* gpar, int maux, double* cfl,

@@ -84,9 +84,10 @@ static int window_occupancy()
 }
 
 /* ---- tile shapes (threads per patch x slices per band) per patch size ----
- * Variant 0 of each size is the default; gf_autotune measures them all and
- * installs the fastest for throughput (whole levels) and for latency (a
- * lone small scenario, where one patch's critical path is the step time). */
+ * Without a choice by hand a launch takes its tile by its number of patches
+ * (pick_tile); gf_autotune measures them all and installs the fastest for
+ * throughput (whole levels) and for latency (a lone small scenario, where one
+ * patch's critical path is the step time). */
 using UpdateFn = cudaError_t (*)(const gf_patch_work*, int, const gf_phys*, double, const double*,
                                  const int*, int, double*, unsigned long long*, int*, int, cudaStream_t);
 using OccFn = int (*)();
@@ -126,7 +127,7 @@ static const Tile kTiles16[] = {GF_TILE(16, 128, 6, 3), GF_TILE(16, 256, 13, 1),
                                 GF_WTILE(16, 128, 6, 2), GF_WTILE(16, 128, 6, 4), GF_WTILE(16, 256, 9, 4)};
 static const Tile kTiles32[] = {GF_TILE(32, 256, 7, 1), GF_TILE(32, 256, 5, 1), GF_TILE(32, 384, 7, 1),
                                 GF_TILE(32, 384, 9, 1), GF_TILE(32, 512, 8, 1), GF_TILE(32, 512, 9, 1),
-                                GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8)};
+                                GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8), GF_WTILE(32, 256, 7, 2)};
 #undef GF_TILE
 #undef GF_WTILE
 
@@ -140,11 +141,14 @@ static const Tile* tiles_of(int m, int* n)
     }
 }
 
-/* selected variant per goal (0 throughput, 1 latency) and patch size. 8^2
- * patches start with a whole patch per band and a thread per face: the
- * classes of a band's faces then fill warps better, and the list pass is one
- * round (24 patches 41 us, 4096 patches 361 us; 64 x 5: 58 and 399 us). */
-static int g_tile[2][3] = {{1, 0, 0}, {1, 0, 0}};
+/* Selected variant per goal (0 throughput, 1 latency) and patch size, and the
+ * selection that stands for "by the number of patches" (pick_tile): the
+ * defaults here, or what gf_autotune installed. 8^2 patches take a whole patch
+ * per band and a thread per face (24 patches 39 us, 4096 patches 324 us; 64 x
+ * 5: 55 and 375 us); 32^2 patches 384 x 9 (4096 patches 3.34 ms, 256 x 7 3.61). */
+static int g_tile[2][3] = {{1, 0, 3}, {1, 0, 3}};
+static int g_auto[2][3] = {{1, 0, 3}, {1, 0, 3}};
+static bool g_tuned[3] = {false, false, false};
 static inline int mcls(int m) { return m == 8 ? 0 : m == 16 ? 1 : 2; }
 
 int tile_count(int m)
@@ -167,18 +171,14 @@ int tile_shape(int m, int v, int* nt, int* rb, int* k)
 
 int tile_get(int m, int goal) { return g_tile[goal != 0][mcls(m)]; }
 
-/* The latency tile pays for its split only while every patch of the launch
- * is resident at once; past one wave the throughput tile finishes sooner. */
-int latency_goal_fits(int m, long npatch)
+/* Patches that one launch of variant v runs at once on this device. */
+static long tile_resident(int m, int v)
 {
     int n = 0;
     const Tile* t = tiles_of(m, &n);
-    if (!t) return 0;
-    const int v = g_tile[1][mcls(m)];
     static std::atomic<int> cache[64][3][GF_MAX_TILES] = {};
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || v >= GF_MAX_TILES)
-        return npatch * t[v].k <= (long)sm_count() ? 1 : 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || v >= GF_MAX_TILES) return sm_count() / t[v].k;
     std::atomic<int>& c = cache[dev][mcls(m)][v];
     int slots = c.load(std::memory_order_relaxed);
     if (!slots) {
@@ -187,7 +187,47 @@ int latency_goal_fits(int m, long npatch)
         if (slots <= 0) slots = 1;
         c.store(slots, std::memory_order_relaxed);
     }
-    return npatch <= (long)slots ? 1 : 0;
+    return slots;
+}
+
+/* The latency tile pays for its split only while every patch of the launch
+ * is resident at once; past one wave the throughput tile finishes sooner. */
+int latency_goal_fits(int m, long npatch)
+{
+    int n = 0;
+    if (!tiles_of(m, &n)) return 0;
+    return npatch <= tile_resident(m, g_tile[1][mcls(m)]) ? 1 : 0;
+}
+
+/* Launches that leave SMs idle take a tile that spreads a patch: the first of
+ * these whose CTAs all run at once with at most per_sm of them on an SM (FP64
+ * throughput is the SM's, so a split pays while SMs are free). us for that
+ * many 32^2 patches: K = 8 50 (1), K = 4 76 (24), K = 2 107 (72), one CTA 170
+ * (144); 16^2: 256 x 9 over K = 4 41 (24), 128 x 6 over K = 4 51 (72), 256 x 13
+ * on one CTA 68 (144), 128 x 6 80; past one patch an SM the tile with the most
+ * CTAs resident (16^2, 400 patches: 138 us, 256 x 13 172). The split of an 8^2
+ * patch gains nothing (33 us against 32). */
+struct SmallTile {
+    int v, per_sm;
+};
+static const SmallTile kSmall16[] = {{5, 1}, {4, 2}, {1, 1}};
+static const SmallTile kSmall32[] = {{7, 1}, {6, 1}, {8, 1}};
+
+static int pick_tile(int m, long npatch, int max_ctas, int goal)
+{
+    const int c = mcls(m);
+    goal = goal != 0;
+    /* chosen by hand, or the tuned latency tile asked for */
+    if (g_tile[goal][c] != g_auto[goal][c] || (goal && g_tuned[c])) return g_tile[goal][c];
+    if (max_ctas <= 0 && c != 0) {
+        int nt = 0;
+        const Tile* t = tiles_of(m, &nt);
+        const SmallTile* s = c == 1 ? kSmall16 : kSmall32;
+        for (int i = 0; i < 3; ++i)
+            if (npatch * t[s[i].v].k <= (long)s[i].per_sm * sm_count() && npatch <= tile_resident(m, s[i].v))
+                return s[i].v;
+    }
+    return g_tile[0][c];
 }
 
 int tile_set(int m, int goal, int v)
@@ -197,6 +237,14 @@ int tile_set(int m, int goal, int v)
     if (v < 0 || v >= n) return -1;
     g_tile[goal != 0][mcls(m)] = v;
     return 0;
+}
+
+void tile_install_tuned(int m, int throughput, int latency)
+{
+    const int c = mcls(m);
+    g_tile[0][c] = g_auto[0][c] = throughput;
+    g_tile[1][c] = g_auto[1][c] = latency;
+    g_tuned[c] = true;
 }
 
 cudaError_t launch_patch_update_tile(int m, int v, const gf_patch_work* work, int nwork,
@@ -217,7 +265,17 @@ cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, con
                                 int goal)
 {
     if (!(m == 8 || m == 16 || m == 32)) return cudaErrorInvalidValue;
-    return launch_patch_update_tile(m, g_tile[goal != 0][mcls(m)], work, nwork, phys, dt, gdt, gpar,
+    if (nwork <= 0) { /* set every tile's attributes, ahead of a capture */
+        int n = 0;
+        const Tile* t = tiles_of(m, &n);
+        for (int v = 0; v < n; ++v) {
+            tile_resident(m, v);
+            cudaError_t e = t[v].fn(work, 0, phys, dt, gdt, gpar, maux, cfl, gmax, err, 0, st);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
+    return launch_patch_update_tile(m, pick_tile(m, nwork, max_ctas, goal), work, nwork, phys, dt, gdt, gpar,
                                     maux, cfl, gmax, err, st, max_ctas);
 }
 

@@ -52,6 +52,24 @@ def test_tile_shapes_give_the_same_bits(ctx, m):
         assert np.array_equal(pg, outs[0][2])
 
 
+@pytest.mark.parametrize("m,npx", [(16, 1), (16, 38), (16, 39), (16, 76), (16, 77), (16, 152), (16, 153),
+                                   (32, 19), (32, 20), (32, 38), (32, 39), (32, 76), (32, 77)])
+def test_tile_by_the_number_of_patches_gives_the_same_bits(ctx, m, npx):
+    """Without a choice by hand the tile follows the launch's number of
+    patches: either side of each switch gives the bits of one fixed tile."""
+    keep, other = gf.Context.tile(m, 0), 2
+    q, aux, _, _ = synth.uniform_dam_break_level(npx, 1, m, 1.0, seed=npx, x_dam=0.4 * m * npx)
+    assert keep != other
+    auto = level_vs_oracle(ctx, q, aux, m, 1.0, 0.05, gf.Phys())
+    try:
+        gf.Context.set_tile(m, 0, other)
+        one = level_vs_oracle(ctx, q, aux, m, 1.0, 0.05, gf.Phys())
+    finally:
+        gf.Context.set_tile(m, 0, keep)
+    compare(q, auto[0], auto[1], auto[2], auto[3], m, pcfl_gpu=auto[4], pcfl_ref=auto[5])
+    assert np.array_equal(auto[0], one[0]) and auto[2] == one[2] and np.array_equal(auto[4], one[4])
+
+
 def test_autotune_measures_and_selects(ctx):
     ctx.set_phys(0, gf.Phys())
     res = ctx.autotune(reps=2)
