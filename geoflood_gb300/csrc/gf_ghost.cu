@@ -12,6 +12,7 @@
  */
 #include <cuda_runtime.h>
 
+#include "gf_cmp.cuh"
 #include "gf_internal.h"
 
 namespace gf {
@@ -23,28 +24,58 @@ __device__ __forceinline__ double* plane(double* base, long patch, int field, in
     return base + (patch * nf + field) * (long)S;
 }
 
+/* x^(2/3): for positive x in the single-precision range, x y0 from the
+ * single-precision y0 of x^(-1/3) and one third-order step of the binomial
+ * series, x y0 (1 - e)^(-1/3) with e = 1 - x y0^3; pow otherwise. */
+__device__ __forceinline__ double pow23(double x)
+{
+    if (!(x > 1.0e-30 && x < 1.0e30)) return pow(x, 2.0 / 3.0);
+    const double y0 = gf_f64_pos(rcbrtf(gf_f32(x)));
+    const double e = fma(-x, (y0 * y0) * y0, 1.0);
+    const double t = x * y0;
+    return fma(t * e, fma(2.0 / 9.0, e, 1.0 / 3.0), t);
+}
+__device__ __forceinline__ double root(double a)
+{
+    return gf_pos_normal(a) ? gf_sqrt_n(a) : sqrt(a);
+}
+
 /* Riemann_invariants / two_shock (hydrograh_module.f90:224-331), discharge
- * form; tol is the single-precision literal 1.0e-6 of the Fortran. */
-__device__ void inflow_riemann(double g, double q0hu, double h1, double hu1, double& h0, bool two)
+ * form; tol is the single-precision literal 1.0e-6 of the Fortran. The whole
+ * iteration is one chain of FP64 instructions of 64 clocks each, and a ghost
+ * fill lasts as long as it does: quotients share one refined reciprocal, roots
+ * are refined likewise, what does not change stays outside (a served round's
+ * ghost fill with an inflow side 42-49 us with pow and IEEE quotients). */
+__device__ void inflow_riemann(double g, double rsg, double q0hu, double h1, double u1, double& h0, bool two)
 {
     const double tol = (double)1.0e-6f;
-    const double u1 = hu1 / h1;
-    const double Fr = two ? 1.0 : 0.5;
-    h0 = pow(q0hu / sqrt(g) * Fr, 2.0 / 3.0);
-    for (int i = 1; i <= 100; ++i) {
-        double fxn, dfxn;
-        if (!two) {
-            fxn = q0hu / h0 - 2 * sqrt(g * h0) - u1 + 2 * sqrt(g * h1);
+    const double x = q0hu * rsg;
+    h0 = pow23(two ? x : 0.5 * x);
+    if (!two) {
+        const double fixed = fma(2.0, root(g * h1), -u1);
+        for (int i = 1; i <= 100; ++i) {
+            /* fxn = q0/h0 - 2 sqrt(g h0) - u1 + 2 sqrt(g h1), dfxn = -q0/h0^2 - sqrt(g/h0) */
+            const double r = gf_rcp(h0), s = root(g * h0), q = q0hu * r;
+            const double fxn = fma(-2.0, s, q) + fixed;
             if (fabs(fxn) < tol) return;
-            dfxn = -q0hu / (h0 * h0) - sqrt(g / h0);
-        } else {
-            fxn = q0hu / h0 - u1 - (h0 - h1) * sqrt((g / 2.0) * (1.0 / h0 + 1.0 / h1));
-            if (fabs(fxn) < tol) return;
-            const double num = sqrt(g * (1.0 / h0 + 1.0 / h1));
-            const double deno = 2 * sqrt(2.0) * (h0 * h0) * num;
-            dfxn = -q0hu / (h0 * h0) - num / sqrt(2.0) + g * (h0 - h1) / deno;
+            const double dfxn = -(q + s) * r;
+            h0 = fma(-fxn, gf_rcp(dfxn), h0);
         }
-        h0 = h0 - fxn / dfxn;
+        return;
+    }
+    const double r1 = gf_rcp(h1);
+    constexpr double kR2 = 0.70710678118654752440; /* 1 / sqrt(2) */
+    for (int i = 1; i <= 100; ++i) {
+        /* num = sqrt(g (1/h0 + 1/h1)): fxn = q0/h0 - u1 - (h0 - h1) num / sqrt(2),
+         * dfxn = -q0/h0^2 - num / sqrt(2) + g (h0 - h1) / (2 sqrt(2) h0^2 num) */
+        const double r = gf_rcp(h0), d = h0 - h1, q = q0hu * r;
+        const double a = g * (r + r1);
+        const double ri = gf_pos_normal(a) ? gf_rsqrt_n(a) : rsqrt(a);
+        const double n2 = (a * ri) * kR2;
+        const double fxn = fma(-d, n2, q - u1);
+        if (fabs(fxn) < tol) return;
+        const double dfxn = fma(((0.5 * kR2) * g) * (d * ri), r * r, -fma(q, r, n2));
+        h0 = fma(-fxn, gf_rcp(dfxn), h0);
     }
 }
 
@@ -52,16 +83,18 @@ __device__ void inflow_riemann(double g, double q0hu, double h1, double hu1, dou
 __device__ bool inflow_state(const gf_phys& P, double q0hu, double h1, double hu1, double& h,
                              double& hu)
 {
+    const double g = P.grav;
     if (h1 < P.dry_tolerance) {
-        const double hh = pow(q0hu / sqrt(P.grav), 2.0 / 3.0);
+        const double hh = pow23(q0hu / sqrt(g));
         h = hh > 0.001 ? hh : 0.001;
         hu = q0hu;
         return true;
     }
     if (q0hu != 0.0) {
+        const double rsg = rsqrt(g), u1 = hu1 / h1;
         double h0;
-        inflow_riemann(P.grav, q0hu, h1, hu1, h0, false);
-        if (h0 > h1) inflow_riemann(P.grav, q0hu, h1, hu1, h0, true);
+        inflow_riemann(g, rsg, q0hu, h1, u1, h0, false);
+        if (h0 > h1) inflow_riemann(g, rsg, q0hu, h1, u1, h0, true);
         h = h0;
         hu = q0hu;
         return true;
@@ -69,8 +102,14 @@ __device__ bool inflow_state(const gf_phys& P, double q0hu, double h1, double hu
     return false;
 }
 
+/* Threads of a patch: every ghost cell in at most two rounds, every cell of
+ * the x or the y sides in one (32^2: 272 and 144 cells, 16^2: 144 and 80, 8^2:
+ * 80 and 48). */
 template <int M>
-__global__ void __launch_bounds__(128) ghost_fill_kernel(const gf_ghost_block* __restrict__ blocks,
+constexpr int kGhostThreads = M == 32 ? 160 : M == 16 ? 96 : 96;
+
+template <int M>
+__global__ void __launch_bounds__(kGhostThreads<M>) ghost_fill_kernel(const gf_ghost_block* __restrict__ blocks,
                                                          const gf_ghost_ref* __restrict__ list,
                                                          int nlist,
                                                          const gf_phys* __restrict__ phys_table)
@@ -105,25 +144,49 @@ __global__ void __launch_bounds__(128) ghost_fill_kernel(const gf_ghost_block* _
         if (skip) return;
     }
 
-    /* ---- step 1: same-level face and corner copies ---- */
-    for (int k = threadIdx.x; k < S; k += blockDim.x) {
-        const int i = k % N - 1, j = k / N - 1; /* Fortran indices 1-mbc..M+mbc */
-        const bool L = i <= 0, R = i >= M + 1, B = j <= 0, T = j >= M + 1;
-        if (!(L || R || B || T)) continue;
-        int src;
-        if ((L || R) && (B || T)) src = nb[4 + (T ? 2 : 0) + (R ? 1 : 0)];
-        else src = nb[L ? 0 : R ? 1 : B ? 2 : 3];
-        if (src < 0) continue;
-        const int i2 = i + (L ? M : R ? -M : 0), j2 = j + (B ? M : T ? -M : 0);
-        const int k2 = (j2 + 1) * N + (i2 + 1);
+    /* ---- step 1: same-level face and corner copies: the ghost cells by
+     * number (two rows below, two above, then the sides row by row), all loads
+     * of a thread ahead of its stores ---- */
+    constexpr int NG = S - M * M, NT = kGhostThreads<M>, IT = (NG + NT - 1) / NT;
+    double val[IT][3];
+    int dst[IT];
 #pragma unroll
-        for (int f = 0; f < 3; ++f) plane(q, p, f, S, 3)[k] = plane(q, src, f, S, 3)[k2];
+    for (int it = 0; it < IT; ++it) {
+        const int e = threadIdx.x + it * NT;
+        dst[it] = -1;
+        if (e >= NG) continue;
+        int ii, jj; /* array column and row */
+        if (e < 4 * N) {
+            const int r = e / N;
+            ii = e - r * N;
+            jj = r < 2 ? r : M + r;
+        } else {
+            const int r = (e - 4 * N) / 4, c = (e - 4 * N) % 4;
+            ii = c < 2 ? c : M + c;
+            jj = 2 + r;
+        }
+        const bool L = ii < 2, R = ii >= M + 2, B = jj < 2, T = jj >= M + 2;
+        int src = L ? nb[0] : nb[1];
+        if (B || T) src = L ? (B ? nb[4] : nb[6]) : R ? (B ? nb[5] : nb[7]) : (B ? nb[2] : nb[3]);
+        if (src < 0) continue;
+        const int k2 = (jj + (B ? M : T ? -M : 0)) * N + ii + (L ? M : R ? -M : 0);
+        dst[it] = jj * N + ii;
+        const double* from = plane(q, src, 0, S, 3) + k2;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) val[it][f] = from[f * S];
     }
+    double* own = plane(q, p, 0, S, 3);
+#pragma unroll
+    for (int it = 0; it < IT; ++it)
+        if (dst[it] >= 0) {
+#pragma unroll
+            for (int f = 0; f < 3; ++f) own[f * S + dst[it]] = val[it][f];
+        }
     const bool phys_side[4] = {nb[0] == -1, nb[1] == -1, nb[2] == -1, nb[3] == -1};
     if (!(phys_side[0] || phys_side[1] || phys_side[2] || phys_side[3])) return;
     __syncthreads();
 
-    const gf_phys P = phys_table[blk.phys_of ? blk.phys_of[p] : blk.phys];
+    const gf_phys& P = phys_table[blk.phys_of ? blk.phys_of[p] : blk.phys];
     const gf_patch_geom G = blk.geom[p];
     double* qh = plane(q, p, 0, S, 3);
     double* qu = plane(q, p, 1, S, 3);
@@ -211,9 +274,9 @@ cudaError_t launch_ghost_fill(int m, const gf_ghost_block* blocks, const gf_ghos
 {
     if (nlist <= 0) return cudaSuccess;
     switch (m) {
-    case 32: ghost_fill_kernel<32><<<nlist, 128, 0, st>>>(blocks, list, nlist, phys); break;
-    case 16: ghost_fill_kernel<16><<<nlist, 128, 0, st>>>(blocks, list, nlist, phys); break;
-    case 8: ghost_fill_kernel<8><<<nlist, 128, 0, st>>>(blocks, list, nlist, phys); break;
+    case 32: ghost_fill_kernel<32><<<nlist, kGhostThreads<32>, 0, st>>>(blocks, list, nlist, phys); break;
+    case 16: ghost_fill_kernel<16><<<nlist, kGhostThreads<16>, 0, st>>>(blocks, list, nlist, phys); break;
+    case 8: ghost_fill_kernel<8><<<nlist, kGhostThreads<8>, 0, st>>>(blocks, list, nlist, phys); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
