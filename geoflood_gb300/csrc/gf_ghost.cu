@@ -95,7 +95,10 @@ __device__ bool inflow_state(const gf_phys& P, double q0hu, double h1, double hu
         double h0;
         inflow_riemann(g, rsg, q0hu, h1, u1, h0, false);
         if (h0 > h1) inflow_riemann(g, rsg, q0hu, h1, u1, h0, true);
-        h = h0;
+        /* Where the iteration steps to a negative depth its root is not a
+         * number (the reference's too). It keeps the sign of an invalid root:
+         * the update's integer comparisons then take the ghost cell as dry. */
+        h = h0 == h0 ? h0 : __longlong_as_double(static_cast<long long>(0xfff8000000000000ull));
         hu = q0hu;
         return true;
     }

@@ -128,3 +128,27 @@ def test_level_steps_with_ghost_fill_resynced(ctx, mthbc):
         assert np.abs(out - ref).max() <= 1e-10 * sc
         state = out
         lev.upload(state)
+
+
+@pytest.mark.parametrize("m", [8, 16, 32])
+def test_inflow_without_a_root_is_taken_as_dry(ctx, m):
+    """Fast shallow water behind the inflow side: the two-shock iteration steps
+    to a negative depth, whose root is not a number in the reference too. Such a
+    ghost depth carries the sign of an invalid root, and the update takes the
+    ghost cell as dry: every interior value stays finite."""
+    h, hu, q0 = 0.12307, 0.61017, 0.67769858
+    q = np.zeros((1, m + 4, m + 4, 3))
+    q[..., 0], q[..., 1] = h, hu
+    lev = gf.Level(ctx, 1, m, 1)
+    lev.set_geometry(2.0, 2.0)
+    lev.upload(q, np.zeros(q.shape[:3] + (1,)))
+    lev.set_layout(-np.ones((1, 8), np.int32), np.zeros(1), np.zeros(1))
+    lev.set_hydrograph([0.0, 1.0e3], [q0, q0], [1, 0, 0, 0], 1.0e6, 0.0, 0.0)
+    lev.set_bc((0, 1, 1, 1))
+    lev.ghost_fill(0.0)
+    ghost = lev.download()[0, MBC:MBC + m, :MBC]
+    assert np.isnan(ghost[..., 0]).all() and np.signbit(ghost[..., 0]).all()
+    assert np.all(ghost[..., 1] == q0)
+    lev.step(0.0, 0.1)
+    assert np.isfinite(lev.download()[0, MBC:MBC + m, MBC:MBC + m]).all()
+    lev.close()
