@@ -10,10 +10,12 @@
  */
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "gf_internal.h"
 #include "gf_patch_update.cuh"
+#include "gf_patch_stream.cuh"
 
 namespace gf {
 
@@ -24,6 +26,22 @@ static cudaError_t launch_update(const gf_patch_work* work, int nwork, const gf_
 {
     using L = Smem<M, RB, false>;
     auto kern = patch_update_kernel<M, NT, RB, MINB, false>;
+    static std::atomic<unsigned long long> attr_done{0};
+    cudaError_t ae = smem_attr_per_device(kern, (int)L::BYTES, attr_done);
+    if (ae != cudaSuccess) return ae;
+    if (nwork <= 0) return cudaSuccess;
+    const int grid = (max_ctas > 0 && max_ctas < nwork) ? max_ctas : nwork;
+    kern<<<grid, NT, L::BYTES, st>>>(work, nwork, phys, dt, gdt, gpar, maux, cfl, gmax, err);
+    return cudaGetLastError();
+}
+
+template <int M, int NT, int R, int MINB>
+static cudaError_t launch_stream(const gf_patch_work* work, int nwork, const gf_phys* phys,
+                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
+                                 unsigned long long* gmax, int* err, int max_ctas, cudaStream_t st)
+{
+    using L = StreamSmem<M, R>;
+    auto kern = patch_update_stream_kernel<M, NT, R, MINB>;
     static std::atomic<unsigned long long> attr_done{0};
     cudaError_t ae = smem_attr_per_device(kern, (int)L::BYTES, attr_done);
     if (ae != cudaSuccess) return ae;
@@ -105,6 +123,22 @@ static int occupancy_of()
     return n;
 }
 
+template <int M, int NT, int R, int MINB>
+static int stream_occupancy()
+{
+    using L = StreamSmem<M, R>;
+    auto kern = patch_update_stream_kernel<M, NT, R, MINB>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) !=
+        cudaSuccess)
+        return 0;
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, NT, L::BYTES) != cudaSuccess) return 0;
+    return n;
+}
+
+template <int M, int NT, int R, int MINB>
+static int stream_slots() { return stream_occupancy<M, NT, R, MINB>() * sm_count(); }
+
 template <int M, int NT, int RB, int MINB>
 static int tile_slots() { return occupancy_of<M, NT, RB, MINB>() * sm_count(); }
 
@@ -118,17 +152,21 @@ struct Tile {
 #define GF_TILE(M, NT, RB, MINB)                                                              \
     {NT, RB, 1, &launch_update<M, NT, RB, MINB>, &occupancy_of<M, NT, RB, MINB>,              \
      &tile_slots<M, NT, RB, MINB>}
+#define GF_STILE(M, NT, R, MINB)                                                              \
+    {NT, R, 1, &launch_stream<M, NT, R, MINB>, &stream_occupancy<M, NT, R, MINB>,             \
+     &stream_slots<M, NT, R, MINB>}
 #define GF_WTILE(M, NT, RB, K)                                                                \
     {NT, RB, K, &launch_window<M, NT, RB, K>, &window_occupancy<M, NT, RB, K>,                \
      &window_slots<M, NT, RB, K>}
-static const Tile kTiles8[] = {GF_TILE(8, 64, 5, 6), GF_TILE(8, 128, 10, 4), GF_TILE(8, 128, 5, 3),
+static const Tile kTiles8[] = {GF_TILE(8, 64, 5, 6), GF_TILE(8, 128, 10, 4), GF_STILE(8, 128, 11, 3),
                                GF_WTILE(8, 64, 5, 2), GF_WTILE(8, 64, 5, 4)};
-static const Tile kTiles16[] = {GF_TILE(16, 128, 6, 3), GF_TILE(16, 256, 13, 1), GF_TILE(16, 256, 9, 2),
+static const Tile kTiles16[] = {GF_TILE(16, 128, 6, 3), GF_STILE(16, 192, 7, 2), GF_TILE(16, 256, 9, 2),
                                 GF_WTILE(16, 128, 6, 2), GF_WTILE(16, 128, 6, 4), GF_WTILE(16, 256, 9, 4)};
-static const Tile kTiles32[] = {GF_TILE(32, 256, 7, 1), GF_TILE(32, 256, 5, 1), GF_TILE(32, 384, 7, 1),
-                                GF_TILE(32, 384, 9, 1), GF_TILE(32, 512, 8, 1), GF_TILE(32, 512, 9, 1),
-                                GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8), GF_WTILE(32, 256, 7, 2)};
+static const Tile kTiles32[] = {GF_TILE(32, 256, 7, 1), GF_STILE(32, 256, 4, 2), GF_TILE(32, 384, 7, 1),
+                                GF_TILE(32, 384, 9, 1), GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8),
+                                GF_WTILE(32, 256, 7, 2)};
 #undef GF_TILE
+#undef GF_STILE
 #undef GF_WTILE
 
 static const Tile* tiles_of(int m, int* n)
@@ -143,11 +181,12 @@ static const Tile* tiles_of(int m, int* n)
 
 /* Selected variant per goal (0 throughput, 1 latency) and patch size, and the
  * selection that stands for "by the number of patches" (pick_tile): the
- * defaults here, or what gf_autotune installed. 8^2 patches take a whole patch
- * per band and a thread per face (24 patches 39 us, 4096 patches 324 us; 64 x
- * 5: 55 and 375 us); 32^2 patches 384 x 9 (4096 patches 3.34 ms, 256 x 7 3.61). */
-static int g_tile[2][3] = {{1, 0, 3}, {1, 0, 3}};
-static int g_auto[2][3] = {{1, 0, 3}, {1, 0, 3}};
+ * defaults here, or what gf_autotune installed. 8^2 patches take the
+ * streamed form, a whole patch in its one band (24 patches 33 us, 4096 patches
+ * 310 us; 128 x 10 swept 39 and 323); 32^2 patches 384 x 9 (4096 patches 3.34
+ * ms, 256 x 7 3.61) or the streamed form, pick_tile. */
+static int g_tile[2][3] = {{2, 0, 3}, {2, 0, 3}};
+static int g_auto[2][3] = {{2, 0, 3}, {2, 0, 3}};
 static bool g_tuned[3] = {false, false, false};
 static inline int mcls(int m) { return m == 8 ? 0 : m == 16 ? 1 : 2; }
 
@@ -203,15 +242,19 @@ int latency_goal_fits(int m, long npatch)
  * these whose CTAs all run at once with at most per_sm of them on an SM (FP64
  * throughput is the SM's, so a split pays while SMs are free). us for that
  * many 32^2 patches: K = 8 50 (1), K = 4 76 (24), K = 2 107 (72), one CTA 170
- * (144); 16^2: 256 x 9 over K = 4 41 (24), 128 x 6 over K = 4 51 (72), 256 x 13
- * on one CTA 68 (144), 128 x 6 80; past one patch an SM the tile with the most
- * CTAs resident (16^2, 400 patches: 138 us, 256 x 13 172). The split of an 8^2
- * patch gains nothing (33 us against 32). */
+ * (144); 16^2: 256 x 9 over K = 4 41 (24), 128 x 6 over K = 4 51 (72), the
+ * streamed 192 x 7 60 (152) and 91 (304), 128 x 6 80 and 103. The split of an
+ * 8^2 patch gains nothing (33 us against 32). */
 struct SmallTile {
     int v, per_sm;
 };
-static const SmallTile kSmall16[] = {{5, 1}, {4, 2}, {1, 1}};
-static const SmallTile kSmall32[] = {{7, 1}, {6, 1}, {8, 1}};
+static const SmallTile kSmall16[] = {{5, 1}, {4, 2}, {1, 2}};
+static const SmallTile kSmall32[] = {{5, 1}, {4, 1}, {6, 1}};
+/* Whole 32^2 levels: the streamed tile, two CTAs an SM, when it fills its slots
+ * once (247 patches 286 us, 384 x 9 301) or many times (4096 patches 3.18 ms,
+ * 3.34; 1215 1.07, 1.09); between, its half-empty last wave costs more than it
+ * gains (400 patches 509 us against 445, 760 767 against 732). */
+constexpr int kStream32 = 1, kStream32Waves = 6; /* patches an SM from which it always pays */
 
 static int pick_tile(int m, long npatch, int max_ctas, int goal)
 {
@@ -226,6 +269,9 @@ static int pick_tile(int m, long npatch, int max_ctas, int goal)
         for (int i = 0; i < 3; ++i)
             if (npatch * t[s[i].v].k <= (long)s[i].per_sm * sm_count() && npatch <= tile_resident(m, s[i].v))
                 return s[i].v;
+        if (c == 2 && !g_tuned[c] &&
+            (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
+            return kStream32;
     }
     return g_tile[0][c];
 }
@@ -292,9 +338,12 @@ int sm_count()
     return cache[dev];
 }
 
-/* mixed tile: 256 threads for every size; mx = 8 takes a whole patch per
- * band, mx = 16 its 256-thread variant, mx = 32 the default */
+/* One launch for every size, 256 threads. Uncapped: the streamed form, two
+ * CTAs an SM (rows per band 11, 7, 4). With a cap, which leaves SMs free for
+ * other launches: the swept form, one CTA an SM (mx = 8 a whole patch per band,
+ * mx = 16 its 256-thread variant). */
 constexpr int kMixNT = 256, kMixRB8 = 10, kMixRB16 = 13, kMixRB32 = 7;
+constexpr int kMixR8 = 11, kMixR16 = 7, kMixR32 = 4;
 
 cudaError_t launch_patch_update_mixed(const gf_patch_work* work, const int n[3], const gf_phys* phys,
                                       double dt, const double* gdt, const int* gpar, int maux,
@@ -306,11 +355,19 @@ cudaError_t launch_patch_update_mixed(const gf_patch_work* work, const int n[3],
     static std::atomic<unsigned long long> attr_done{0};
     cudaError_t ae = smem_attr_per_device(kern, (int)X::BYTES, attr_done);
     if (ae != cudaSuccess) return ae;
+    using Y = MixedStreamSmem<kMixR8, kMixR16, kMixR32>;
+    auto skern = patch_update_mixed_stream_kernel<kMixNT, kMixR8, kMixR16, kMixR32>;
+    static std::atomic<unsigned long long> sattr_done{0};
+    if ((ae = smem_attr_per_device(skern, (int)Y::BYTES, sattr_done)) != cudaSuccess) return ae;
     const int nwork = n[0] + n[1] + n[2];
     if (nwork <= 0) return cudaSuccess;
     int grid = sm_count();
-    if (max_ctas > 0 && max_ctas < grid) grid = max_ctas;
-    if (grid > nwork) grid = nwork;
+    if (max_ctas <= 0 || max_ctas >= grid) {
+        grid = std::min(2 * grid, nwork);
+        skern<<<grid, kMixNT, Y::BYTES, st>>>(work, n[0], n[1], n[2], phys, dt, gdt, gpar, maux, cfl, gmax, err, sched);
+        return cudaGetLastError();
+    }
+    grid = std::min(max_ctas, nwork);
     kern<<<grid, kMixNT, X::BYTES, st>>>(work, n[0], n[1], n[2], phys, dt, gdt, gpar, maux, cfl, gmax, err,
                                          sched);
     return cudaGetLastError();

@@ -391,6 +391,102 @@ __device__ __forceinline__ void build_lists_exact(const double* sm, const unsign
     __syncthreads();
 }
 
+/* Fluctuations and limited second-order term of one face in the contracted
+ * build, from its record wc and its neighbours' wl, wr along the sweep (the
+ * middle f-wave is (0, beta2, 0) in local order). Only the upwind neighbour's
+ * projection is formed; the middle wave's ratio of projection and norm is
+ * the quotient of the two beta2. */
+__device__ __forceinline__ void face_terms_fast(const double* wc, const double* wl, const double* wr, const gf_phys& P,
+                                                double dtdn, double amdq[3], double apdq[3], double cq[3])
+{
+    constexpr bool F = true;
+    const double s0 = wc[0], s1 = wc[1], s2 = wc[2];
+    const double f0[3] = {wc[3], wc[4], wc[5]}, f1 = wc[6], f2[3] = {wc[7], wc[8], wc[9]};
+    if (d_ltz<F>(s0) && d_gtz<F>(s2)) { /* one outer wave each way: no sums */
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            amdq[c] = f0[c];
+            apdq[c] = f2[c];
+        }
+    } else {
+        const double w0m = d_ltz<F>(s0) ? 1.0 : d_gtz<F>(s0) ? 0.0 : 0.5;
+        const double w2m = d_ltz<F>(s2) ? 1.0 : d_gtz<F>(s2) ? 0.0 : 0.5;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            amdq[c] = fma(w0m, f0[c], gf_mul(w2m, f2[c]));
+            apdq[c] = fma(1.0 - w0m, f0[c], gf_mul(1.0 - w2m, f2[c]));
+        }
+    }
+    if (d_eqz<F>(s1)) {
+        amdq[1] = fma(0.5, f1, amdq[1]);
+        apdq[1] = fma(0.5, f1, apdq[1]);
+    } else {
+        const bool l = d_ltz<F>(s1);
+        const double v = gf_add(l ? amdq[1] : apdq[1], f1);
+        amdq[1] = l ? v : amdq[1];
+        apdq[1] = l ? apdq[1] : v;
+    }
+    cq[0] = cq[1] = cq[2] = 0.0;
+    if (P.order == 1) return;
+    auto outer = [&](double s, const double* fa, int at, int meth) -> double { /* waves 0 and 2 */
+        double lim = 1.0;
+        if (meth != 0) {
+            const double* pw = (d_gtz<F>(s) ? wl : wr) + at;
+            const double wnorm2 = fma(fa[2], fa[2], fma(fa[1], fa[1], gf_mul(fa[0], fa[0])));
+            if (gf_pos_normal(wnorm2))
+                lim = gf_philim<F>(wnorm2, fma(pw[2], fa[2], fma(pw[1], fa[1], gf_mul(pw[0], fa[0]))), meth);
+        }
+        return gf_mul(with_sign_of(fma(-fabs(s), dtdn, 1.0), s), lim);
+    };
+    {
+        const double fl = outer(s0, f0, 3, P.mthlim[0]);
+        cq[0] = gf_mul(fl, f0[0]); cq[1] = gf_mul(fl, f0[1]); cq[2] = gf_mul(fl, f0[2]);
+    }
+    {
+        double lim = 1.0;
+        if (P.mthlim[1] != 0 && gf_pos_normal(fabs(f1))) {
+            const double up = (d_gtz<F>(s1) ? wl : wr)[6];
+            /* MC: opposite signs, or no upwind wave, give zero without the quotient */
+            lim = P.mthlim[1] == 4 && (d_eqz<F>(up) || opposite_signs(up, f1))
+                      ? 0.0
+                      : gf_philim_r<F>(d_div<F>(up, f1), P.mthlim[1]);
+        }
+        cq[1] = fma(gf_mul(with_sign_of(fma(-fabs(s1), dtdn, 1.0), s1), lim), f1, cq[1]);
+    }
+    {
+        const double fl = outer(s2, f2, 7, P.mthlim[2]);
+        cq[0] = fma(fl, f2[0], cq[0]); cq[1] = fma(fl, f2[1], cq[1]); cq[2] = fma(fl, f2[2], cq[2]);
+    }
+}
+
+/* Per cell of a slice in the contracted build, from the terms of its left and
+ * right face (ol, or): the flux difference N = faddm(right) - faddp(left) =
+ * P + Q/2 with P = amdq(right) + apdq(left), Q = cq(right) - cq(left), and the
+ * transverse split of the fluctuations that enter the cell. rpt2 is linear in
+ * its input and the cell alone decides its branches, so the splits of
+ * amdq(right) and apdq(left) (with the second-order terms for transverse = 2)
+ * are one split of their sum P + Q (P for transverse = 1): bm is the down-going
+ * part, bp the up-going part, equal to the sum of the reference's two splits up
+ * to rounding. Local component order. */
+__device__ __forceinline__ void cell_terms(const double* ol, const double* orr, const gf_cell& cc, double b_lo,
+                                           double b_hi, int transverse, double N[3], double bm[3], double bp[3])
+{
+    double Pv[3], Qv[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        Pv[q] = gf_add(orr[q], ol[3 + q]);
+        Qv[q] = gf_sub(orr[6 + q], ol[6 + q]);
+        N[q] = fma(0.5, Qv[q], Pv[q]);
+        bm[q] = bp[q] = 0.0;
+    }
+    if (transverse != 0 && cc.wet) {
+        double x[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) x[q] = transverse == 2 ? gf_add(Pv[q], Qv[q]) : Pv[q];
+        gf_rpt2_fast(cc, b_lo, b_hi, x, bm, bp);
+    }
+}
+
 /* One sweep direction over all slices, banded. Accumulates into the flux
  * accumulators (contracted build: the x sweep starts them); returns this
  * thread's max |s| over normal faces. side: further work of 32 items a chunk
@@ -668,71 +764,6 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
         }
     };
 
-    /* The same in the contracted build, on its shorter face records (the
-     * middle f-wave is (0, beta2, 0) in local order). Only the upwind neighbour's
-     * projection is formed; the middle wave's ratio of projection and norm is
-     * the quotient of the two beta2. */
-    auto face_terms_fast = [&](const double* wc, double amdq[3], double apdq[3], double cq[3]) {
-        constexpr bool F = true;
-        const double s0 = wc[0], s1 = wc[1], s2 = wc[2];
-        const double f0[3] = {wc[3], wc[4], wc[5]}, f1 = wc[6], f2[3] = {wc[7], wc[8], wc[9]};
-        if (d_ltz<F>(s0) && d_gtz<F>(s2)) { /* one outer wave each way: no sums */
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                amdq[c] = f0[c];
-                apdq[c] = f2[c];
-            }
-        } else {
-            const double w0m = d_ltz<F>(s0) ? 1.0 : d_gtz<F>(s0) ? 0.0 : 0.5;
-            const double w2m = d_ltz<F>(s2) ? 1.0 : d_gtz<F>(s2) ? 0.0 : 0.5;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                amdq[c] = fma(w0m, f0[c], gf_mul(w2m, f2[c]));
-                apdq[c] = fma(1.0 - w0m, f0[c], gf_mul(1.0 - w2m, f2[c]));
-            }
-        }
-        if (d_eqz<F>(s1)) {
-            amdq[1] = fma(0.5, f1, amdq[1]);
-            apdq[1] = fma(0.5, f1, apdq[1]);
-        } else {
-            const bool l = d_ltz<F>(s1);
-            const double v = gf_add(l ? amdq[1] : apdq[1], f1);
-            amdq[1] = l ? v : amdq[1];
-            apdq[1] = l ? apdq[1] : v;
-        }
-        cq[0] = cq[1] = cq[2] = 0.0;
-        if (P.order == 1) return;
-        auto outer = [&](double s, const double* fa, int at, int meth) -> double { /* waves 0 and 2 */
-            double lim = 1.0;
-            if (meth != 0) {
-                const double* pw = (d_gtz<F>(s) ? wc - L::W_STRIDE : wc + L::W_STRIDE) + at;
-                const double wnorm2 = fma(fa[2], fa[2], fma(fa[1], fa[1], gf_mul(fa[0], fa[0])));
-                if (gf_pos_normal(wnorm2))
-                    lim = gf_philim<F>(wnorm2, fma(pw[2], fa[2], fma(pw[1], fa[1], gf_mul(pw[0], fa[0]))), meth);
-            }
-            return gf_mul(with_sign_of(fma(-fabs(s), dtdn, 1.0), s), lim);
-        };
-        {
-            const double fl = outer(s0, f0, 3, P.mthlim[0]);
-            cq[0] = gf_mul(fl, f0[0]); cq[1] = gf_mul(fl, f0[1]); cq[2] = gf_mul(fl, f0[2]);
-        }
-        {
-            double lim = 1.0;
-            if (P.mthlim[1] != 0 && gf_pos_normal(fabs(f1))) {
-                const double up = (d_gtz<F>(s1) ? wc - L::W_STRIDE : wc + L::W_STRIDE)[6];
-                /* MC: opposite signs, or no upwind wave, give zero without the quotient */
-                lim = P.mthlim[1] == 4 && (d_eqz<F>(up) || opposite_signs(up, f1))
-                          ? 0.0
-                          : gf_philim_r<F>(d_div<F>(up, f1), P.mthlim[1]);
-            }
-            cq[1] = fma(gf_mul(with_sign_of(fma(-fabs(s1), dtdn, 1.0), s1), lim), f1, cq[1]);
-        }
-        {
-            const double fl = outer(s2, f2, 7, P.mthlim[2]);
-            cq[0] = fma(fl, f2[0], cq[0]); cq[1] = fma(fl, f2[1], cq[1]); cq[2] = fma(fl, f2[2], cq[2]);
-        }
-    };
-
     /* ---- exact build, stage B: limiter, 2nd-order terms, both transverse
      * splits of every face (flux2's per-face order) ---- */
     auto stage_b_exact = [&](int t0, int band) {
@@ -821,7 +852,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
         const int n = win.nb_lo + (f - ts * fb);
         const double* wc = W + (ts * fa + (n - win.na_lo)) * L::W_STRIDE;
         double amdq[3], apdq[3], cq[3];
-        face_terms_fast(wc, amdq, apdq, cq);
+        face_terms_fast(wc, wc - L::W_STRIDE, wc + L::W_STRIDE, P, dtdn, amdq, apdq, cq);
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             o[k] = amdq[k];
@@ -830,16 +861,8 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
         }
     };
 
-    /* ---- contracted build, stage B2: per cell n of each band slice, from
-     * its faces n (apdq, cq) and n+1 (amdq, cq): the flux difference
-     * N = faddm(n+1) - faddp(n) = P + Q/2 with P = amdq(n+1) + apdq(n),
-     * Q = cq(n+1) - cq(n), and the transverse split of the fluctuations that
-     * enter the cell. rpt2 is linear in its input and the cell alone decides
-     * its branches, so the splits of amdq(n+1) and apdq(n) (with the
-     * second-order terms for transverse = 2) are one split of their sum
-     * P + Q (P for transverse = 1): bm is the down-going part Dn, bp the
-     * up-going part U, equal to the sum of the reference's two splits up to
-     * rounding. ---- */
+    /* ---- contracted build, stage B2: per cell n of each band slice, its
+     * record from its faces n and n+1 (cell_terms) ---- */
     auto chunk_b2 = [&](int t0, int t1, int c) {
         const int ncell = fb - 1;
         const int e = 32 * c + (int)(threadIdx.x & 31);
@@ -857,21 +880,9 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
             }
             const double* orr = O + (ts * fb + (n + 1 - win.nb_lo)) * L::O_STRIDE; /* face n+1 */
             const double* orl = O + (ts * fb + (n - win.nb_lo)) * L::O_STRIDE;     /* face n   */
-            double Pv[3], Qv[3], Nv[3];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) {
-                Pv[q] = gf_add(orr[q], orl[3 + q]);
-                Qv[q] = gf_sub(orr[6 + q], orl[6 + q]);
-                Nv[q] = fma(0.5, Qv[q], Pv[q]);
-            }
-            double bm[3] = {0.0, 0.0, 0.0}, bp[3] = {0.0, 0.0, 0.0};
-            if (P.transverse != 0 && wet[k]) {
-                double x[3];
-#pragma unroll
-                for (int q = 0; q < 3; ++q) x[q] = P.transverse == 2 ? gf_add(Pv[q], Qv[q]) : Pv[q];
-                const gf_cell cc = load_cell<DIR, EXACT, L>(sm, wet, k);
-                gf_rpt2_fast(cc, sm[L::OFF_B + cidx(n, t - 1)], sm[L::OFF_B + cidx(n, t + 1)], x, bm, bp);
-            }
+            double Nv[3], bm[3], bp[3];
+            cell_terms(orl, orr, load_cell<DIR, EXACT, L>(sm, wet, k), sm[L::OFF_B + cidx(n, t - 1)],
+                       sm[L::OFF_B + cidx(n, t + 1)], P.transverse, Nv, bm, bp);
             /* global component order (h, hu, hv) */
             r[0] = Nv[0]; r[G1] = Nv[1]; r[G2] = Nv[2];
             r[3] = bp[0]; r[3 + G1] = bp[1]; r[3 + G2] = bp[2];
