@@ -153,50 +153,172 @@ __device__ bool cell_integral(const Rect& cell, const gf_topo_grid* grids, const
     return false;
 }
 
-__global__ void topo_raster_kernel(const gf_topo_grid* __restrict__ grids, const int* __restrict__ order,
-                                   int n, int nx, int ny, int halo, double xlower, double ylower,
-                                   double dx, double dy, double xupper, double yupper,
-                                   double* __restrict__ out, int* __restrict__ err)
+/* Tile of raster cells of a CTA, and the most node cells of a column (row) of
+ * cells that its tables hold: coarser cells take the general path. */
+constexpr int kTX = 32, kTY = 8, kNodes = 40;
+
+/* One axis of the integral of a column (row) of cells [lo, hi] over a grid:
+ * the node cells i0 .. i1 - 1 it touches, and for each the width of the
+ * overlap and the sum of its two ends in units of the spacing, as
+ * grid_integral forms them. */
+struct AxisNode {
+    double width, sum;
+};
+__device__ __forceinline__ void axis_range(double& lo, double& hi, double low, double d, int n, int* i0, int* i1)
 {
-    const long p = nx + 2 * halo;
-    const long total = p * (ny + 2 * halo);
-    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-        const int gi = (int)(e % p) - halo, gj = (int)(e / p) - halo;
-        Rect cell;
-        cell.x1 = xlower + (double)gi * dx;
-        cell.x2 = xlower + (double)(gi + 1) * dx;
-        cell.y1 = ylower + (double)gj * dy;
-        cell.y2 = ylower + (double)(gj + 1) * dy;
-        const double x = 0.5 * (cell.x1 + cell.x2), y = 0.5 * (cell.y1 + cell.y2);
-        if (y > yupper || y < ylower || x > xupper || x < xlower) continue;
-        double v;
-        if (!cell_integral(cell, grids, order, n, &v)) *err = 1;
-        out[e] = v / (dx * dy);
+    const double top = low + (n - 1) * d;
+    if ((lo - low) < 0.0 || (hi - top) > 0.0) {
+        lo = fmax(low, lo);
+        hi = fmin(top, hi);
     }
+    *i0 = max((int)((lo - low) / d) + 1, 1);
+    *i1 = min((int)ceil((hi - low) / d) + 1, n);
+}
+__device__ __forceinline__ AxisNode axis_node(double lo, double hi, double low, double d, int ii)
+{
+    const double x1 = low + (ii - 1.0) * d, x2 = low + ii * d;
+    const double a = fmax(lo, x1), b = fmin(hi, x2);
+    return {b - a, (b + a - 2.0 * x1) / d};
+}
+
+/* One thread per cell. The kernel is bound by FP64 issue (two lanes a clock),
+ * and most of it went into quotients that depend on the cell's column or row
+ * alone: a tile now forms them once per column and row of cells, in shared
+ * memory, for the cells that lie whole in the finest grid they touch (the
+ * same operations in the same order, so the same bits); the others (cells that
+ * a grid's edge cuts, cells over more node cells than the tables hold) take
+ * cell_integral. */
+__global__ void __launch_bounds__(kTX* kTY)
+    topo_raster_kernel(const gf_topo_grid* __restrict__ grids, const int* __restrict__ order, int n, int nx, int ny,
+                       int halo, double xlower, double ylower, double dx, double dy, double xupper, double yupper,
+                       double* __restrict__ out, int* __restrict__ err)
+{
+    __shared__ AxisNode xt[kNodes][kTX], yt[kTY][kNodes];
+    __shared__ double cx[kTX][2], cy[kTY][2];
+    __shared__ int xr[kTX][2], yr[kTY][2];
+    __shared__ unsigned char outx[kTX], outy[kTY];
+    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * kTX + tx;
+    const long p = nx + 2 * halo;
+    const int tiles = (int)((p + kTX - 1) / kTX), by = blockIdx.x / tiles, bx = blockIdx.x - by * tiles;
+    const int i = bx * kTX + tx, j = by * kTY + ty;
+    if (t < kTX) {
+        const int gi = i - halo;
+        const double x1 = xlower + (double)gi * dx, x2 = xlower + (double)(gi + 1) * dx, x = 0.5 * (x1 + x2);
+        cx[tx][0] = x1;
+        cx[tx][1] = x2;
+        outx[tx] = x > xupper || x < xlower;
+    } else if (t < kTX + kTY) {
+        const int k = t - kTX, gj = by * kTY + k - halo;
+        const double y1 = ylower + (double)gj * dy, y2 = ylower + (double)(gj + 1) * dy, y = 0.5 * (y1 + y2);
+        cy[k][0] = y1;
+        cy[k][1] = y2;
+        outy[k] = y > yupper || y < ylower;
+    }
+    __syncthreads();
+    const Rect cell = {cx[tx][0], cx[tx][1], cy[ty][0], cy[ty][1]};
+    const bool live = i < p && j < ny + 2 * halo && !outx[tx] && !outy[ty];
+    /* 0 no grid yet, 1 done, 2 general path */
+    int state = live ? 0 : 1;
+    double v = 0.0;
+    for (int m = 0; m < n; ++m) {
+        const gf_topo_grid& G = grids[order[m]];
+        const bool meets = state == 0 && fmin(cell.x2, G.xhi) > fmax(cell.x1, G.xlow) &&
+                           fmin(cell.y2, G.yhi) > fmax(cell.y1, G.ylow);
+        const bool whole = meets && cell.x1 >= G.xlow && cell.x2 <= G.xhi && cell.y1 >= G.ylow && cell.y2 <= G.yhi;
+        if (meets && !whole) state = 2;
+        if (!__syncthreads_or(whole)) {
+            if (!__syncthreads_or(state == 0)) break;
+            continue;
+        }
+        if (t < kTX) {
+            double lo = cx[tx][0], hi = cx[tx][1];
+            axis_range(lo, hi, G.xlow, G.dx, G.mx, &xr[tx][0], &xr[tx][1]);
+        } else if (t < kTX + kTY) {
+            const int k = t - kTX;
+            double lo = cy[k][0], hi = cy[k][1];
+            axis_range(lo, hi, G.ylow, G.dy, G.my, &yr[k][0], &yr[k][1]);
+        }
+        __syncthreads();
+        {
+            double lo = cx[tx][0], hi = cx[tx][1];
+            const double top = G.xlow + (G.mx - 1) * G.dx;
+            if ((lo - G.xlow) < 0.0 || (hi - top) > 0.0) {
+                lo = fmax(G.xlow, lo);
+                hi = fmin(top, hi);
+            }
+            const int i0 = xr[tx][0], c = min(xr[tx][1] - i0, kNodes);
+            for (int e = ty; e < c; e += kTY) xt[e][tx] = axis_node(lo, hi, G.xlow, G.dx, i0 + e);
+        }
+        {
+            double lo = cy[ty][0], hi = cy[ty][1];
+            const double top = G.ylow + (G.my - 1) * G.dy;
+            if ((lo - G.ylow) < 0.0 || (hi - top) > 0.0) {
+                lo = fmax(G.ylow, lo);
+                hi = fmin(top, hi);
+            }
+            const int j0 = yr[ty][0], c = min(yr[ty][1] - j0, kNodes);
+            for (int e = tx; e < c; e += kTX) yt[ty][e] = axis_node(lo, hi, G.ylow, G.dy, j0 + e);
+        }
+        __syncthreads();
+        if (whole) {
+            const int i0 = xr[tx][0], nc = xr[tx][1] - i0, j0 = yr[ty][0], nr = yr[ty][1] - j0;
+            if (nc > kNodes || nr > kNodes) {
+                state = 2;
+            } else {
+                double s = 0.0;
+                for (int r = 0; r < nr; ++r) {
+                    /* nodes are stored north to south: row (my - jj) holds the lower ones */
+                    const double* row1 = G.z + (long)(G.my - (j0 + r)) * G.mx + (i0 - 1);
+                    const double* row2 = row1 - G.mx;
+                    const AxisNode Y = yt[ty][r];
+                    double z11 = nc > 0 ? row1[0] : 0.0, z12 = nc > 0 ? row2[0] : 0.0;
+                    for (int c = 0; c < nc; ++c) {
+                        const AxisNode X = xt[c][tx];
+                        const double z21 = row1[c + 1], z22 = row2[c + 1];
+                        const double area = Y.width * X.width;
+                        const double a = z21 - z11, b = z12 - z11, d = z22 - z21 - z12 + z11;
+                        s = s + (0.5 * (a * X.sum + b * Y.sum) + 0.25 * d * X.sum * Y.sum + z11) * area;
+                        z11 = z21;
+                        z12 = z22;
+                    }
+                }
+                v = 0.0 + s;
+                state = 1;
+            }
+        }
+        if (!__syncthreads_or(state == 0)) break;
+    }
+    if (!live) return;
+    if (state == 2) cell_integral(cell, grids, order, n, &v);
+    if (state == 0) *err = 1; /* no grid under the cell */
+    out[(long)j * p + i] = v / (dx * dy);
 }
 
 /* cells outside the domain take the cell inside that setaux's index shift
- * names: i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)) */
-__global__ void topo_outside_kernel(double* __restrict__ out, int nx, int ny, int halo, double xlower,
-                                    double ylower, double dx, double dy, double xupper, double yupper)
+ * names: i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)). A
+ * column's and a row's part of the test are formed once per tile. */
+__global__ void __launch_bounds__(kTX* kTY)
+    topo_outside_kernel(double* __restrict__ out, int nx, int ny, int halo, double xlower, double ylower, double dx,
+                        double dy, double xupper, double yupper)
 {
+    __shared__ unsigned char outx[kTX], outy[kTY];
+    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * kTX + tx;
     const long p = nx + 2 * halo;
-    const long total = p * (ny + 2 * halo);
-    for (long e = blockIdx.x * (long)blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(e % p), j = (int)(e / p);
-        const double x = xlower + ((i - halo) + 0.5) * dx, y = ylower + ((j - halo) + 0.5) * dy;
-        if (!(y < ylower || y > yupper || x < xlower || x > xupper)) continue;
-        const int ii = i + (int)fmax(0.0, ceil((xlower - x) / dx)) - (int)fmax(0.0, ceil((x - xupper) / dx));
-        const int jj = j + (int)fmax(0.0, ceil((ylower - y) / dy)) - (int)fmax(0.0, ceil((y - yupper) / dy));
-        out[e] = out[(long)jj * p + ii];
+    const int tiles = (int)((p + kTX - 1) / kTX), by = blockIdx.x / tiles, bx = blockIdx.x - by * tiles;
+    const int i = bx * kTX + tx, j0 = by * kTY, j = j0 + ty;
+    if (t < kTX) {
+        const double x = xlower + ((i - halo) + 0.5) * dx;
+        outx[tx] = x < xlower || x > xupper;
+    } else if (t < kTX + kTY) {
+        const double y = ylower + ((j0 + (t - kTX) - halo) + 0.5) * dy;
+        outy[t - kTX] = y < ylower || y > yupper;
     }
-}
-
-int grid_of(long total)
-{
-    long b = (total + 127) / 128;
-    if (b > 152L * 32) b = 152L * 32;
-    return (int)(b < 1 ? 1 : b);
+    __syncthreads();
+    if (i >= p || j >= ny + 2 * halo || !(outx[tx] || outy[ty])) return;
+    const double x = xlower + ((i - halo) + 0.5) * dx, y = ylower + ((j - halo) + 0.5) * dy;
+    const int ii = i + (int)fmax(0.0, ceil((xlower - x) / dx)) - (int)fmax(0.0, ceil((x - xupper) / dx));
+    const int jj = j + (int)fmax(0.0, ceil((ylower - y) / dy)) - (int)fmax(0.0, ceil((y - yupper) / dy));
+    out[(long)j * p + i] = out[(long)jj * p + ii];
 }
 
 } // namespace
@@ -206,12 +328,14 @@ cudaError_t launch_topo_raster(const gf_topo_grid* grids, const int* order, int 
                                double yupper, double* out, int* err, cudaStream_t st)
 {
     if (n < 1 || n > GF_TOPO_MAX_FILES) return cudaErrorInvalidValue;
-    const long total = (long)(nx + 2 * halo) * (ny + 2 * halo);
-    topo_raster_kernel<<<grid_of(total), 128, 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy,
-                                                       xupper, yupper, out, err);
+    const long tiles = (long)((nx + 2 * halo + kTX - 1) / kTX) * ((ny + 2 * halo + kTY - 1) / kTY);
+    if (tiles > 0x7fffffffL) return cudaErrorInvalidValue; /* 5e11 cells */
+    const dim3 block(kTX, kTY), grid((unsigned)tiles);
+    topo_raster_kernel<<<grid, block, 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper,
+                                               out, err);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || halo == 0) return e;
-    topo_outside_kernel<<<grid_of(total), 128, 0, st>>>(out, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper);
+    topo_outside_kernel<<<grid, block, 0, st>>>(out, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper);
     return cudaGetLastError();
 }
 

@@ -39,6 +39,20 @@ def test_raster_matches_oracle(ctx, nx, ny, dx):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("nx,ny", [(1, 1), (31, 7), (32, 8), (33, 9), (65, 40), (300, 5), (3, 120)])
+def test_raster_tiles_match_oracle(ctx, nx, ny):
+    """Rasters at the edges of the kernel's tiles, cells from a fraction of a
+    spacing to 90 of them, over an inset whose edge cuts cells: bit for bit."""
+    g = np.random.default_rng(nx * 1000 + ny)
+    t = Topo()
+    t.add_grid(g.uniform(0.0, 40.0, (101, 91)), 0.0, 0.0, 10.0, 10.0)
+    t.add_grid(g.uniform(0.0, 40.0, (67, 81)), 203.7, 301.1, 3.3, 3.3)
+    ts = ot.TopoSet([t.grid(k) for k in range(len(t))])
+    dx, dy = 900.0 / nx, 1000.0 / ny
+    got = t.raster(ctx, nx, ny, 2, 0.0, 0.0, dx, dy, 900.0, 1000.0)
+    assert np.array_equal(got, ts.raster(nx, ny, 2, 0.0, 0.0, dx, dy, 900.0, 1000.0))
+
+
 def test_uncovered_cell_is_an_error(ctx):
     t, _ = sets()
     with pytest.raises(gf.GeoFloodError):
