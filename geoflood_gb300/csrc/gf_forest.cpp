@@ -1737,26 +1737,42 @@ namespace {
 /* planes of the leaves' slots <-> Fortran layout in canonical order */
 int move_leaves(gf_forest* f, double* host, int nfield, bool to_host, bool aux)
 {
-    const size_t per = (size_t)nfield * f->S;
-    const size_t n = f->leaves.size();
-    std::vector<double> tmp(per);
+    const size_t per = (size_t)nfield * f->S, n = f->leaves.size();
+    if (n == 0) return GF_OK;
     cudaStream_t st = gf::ctx_stream(f->ctx);
-    for (size_t k = 0; k < n; ++k) {
-        const int s = f->leaves[k].slot;
-        double* dev = aux ? aslot(f, s) : qslot(f, f->par, s);
-        double* h = host + k * per;
+    std::vector<int> slots(n);
+    for (size_t k = 0; k < n; ++k) slots[k] = f->leaves[k].slot;
+    double* base = aux ? aslot(f, 0) : qslot(f, f->par, 0);
+    /* the leaves change layout on the device, through a buffer of at most 64
+     * MB (less where memory is short), one copy per bufferful */
+    int* d_slots = nullptr;
+    double* d_buf = nullptr;
+    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d_slots), n * sizeof(int), st);
+    size_t chunk = std::min(n, std::max<size_t>(1, ((size_t)64 << 20) / (per * sizeof(double))));
+    if (e == cudaSuccess)
+        while ((e = cudaMallocAsync(reinterpret_cast<void**>(&d_buf), chunk * per * sizeof(double), st)) ==
+                   cudaErrorMemoryAllocation &&
+               chunk > 1) {
+            cudaGetLastError();
+            chunk = (chunk + 1) / 2;
+        }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_slots, slots.data(), n * sizeof(int), cudaMemcpyHostToDevice, st);
+    for (size_t k = 0; k < n && e == cudaSuccess; k += chunk) {
+        const int m = (int)std::min(chunk, n - k);
+        const size_t bytes = (size_t)m * per * sizeof(double);
         if (to_host) {
-            FK(f, cudaMemcpyAsync(tmp.data(), dev, per * sizeof(double), cudaMemcpyDeviceToHost, st));
-            FK(f, cudaStreamSynchronize(st));
-            for (long c = 0; c < f->S; ++c)
-                for (int m = 0; m < nfield; ++m) h[(size_t)c * nfield + m] = tmp[(size_t)m * f->S + c];
+            e = gf::launch_leaf_layout(true, d_slots + k, m, base, d_buf, (int)f->S, nfield, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(host + k * per, d_buf, bytes, cudaMemcpyDeviceToHost, st);
         } else {
-            for (long c = 0; c < f->S; ++c)
-                for (int m = 0; m < nfield; ++m) tmp[(size_t)m * f->S + c] = h[(size_t)c * nfield + m];
-            FK(f, cudaMemcpyAsync(dev, tmp.data(), per * sizeof(double), cudaMemcpyHostToDevice, st));
-            FK(f, cudaStreamSynchronize(st));
+            e = cudaMemcpyAsync(d_buf, host + k * per, bytes, cudaMemcpyHostToDevice, st);
+            if (e == cudaSuccess) e = gf::launch_leaf_layout(false, d_slots + k, m, base, d_buf, (int)f->S, nfield, st);
         }
     }
+    if (d_buf) cudaFreeAsync(d_buf, st);
+    if (d_slots) cudaFreeAsync(d_slots, st);
+    const cudaError_t es = cudaStreamSynchronize(st);
+    FK(f, e);
+    FK(f, es);
     return GF_OK;
 }
 

@@ -183,6 +183,22 @@ __global__ void __launch_bounds__(128) slot_copy_kernel(const gf_slot_task* __re
     for (int k = threadIdx.x; k < 3 * S; k += blockDim.x) T.c[k] = T.a[k];
 }
 
+/* Leaves between their slots (planes) and a dense buffer in the Fortran
+ * layout (field fastest), one CTA per leaf: slot s holds nf planes of S cells
+ * at base + s nf S. */
+template <bool TO_DENSE>
+__global__ void __launch_bounds__(256) leaf_layout_kernel(const int* __restrict__ slots, double* __restrict__ base,
+                                                          double* __restrict__ dense, int S, int nf)
+{
+    double* planes = base + (long)slots[blockIdx.x] * nf * S;
+    double* d = dense + (long)blockIdx.x * nf * S;
+    for (int e = threadIdx.x; e < nf * S; e += blockDim.x) {
+        const int c = e / nf, m = e - c * nf;
+        if (TO_DENSE) d[e] = planes[(long)m * S + c];
+        else planes[(long)m * S + c] = d[e];
+    }
+}
+
 int grid_for(long total)
 {
     long b = (total + 255) / 256;
@@ -245,6 +261,15 @@ cudaError_t launch_slot_copy(int m, const gf_slot_task* tasks, int ntask, cudaSt
     case 8: slot_copy_kernel<8><<<ntask, 128, 0, st>>>(tasks, ntask); break;
     default: return cudaErrorInvalidValue;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_leaf_layout(bool to_dense, const int* slots, int n, double* base, double* dense, int S, int nf,
+                               cudaStream_t st)
+{
+    if (n <= 0) return cudaSuccess;
+    if (to_dense) leaf_layout_kernel<true><<<n, 256, 0, st>>>(slots, base, dense, S, nf);
+    else leaf_layout_kernel<false><<<n, 256, 0, st>>>(slots, base, dense, S, nf);
     return cudaGetLastError();
 }
 

@@ -155,6 +155,8 @@ int topo_raster_device(gf_ctx* c, gf_topo* t, int nx, int ny, int halo, double x
                        double* out, cudaStream_t st);
 cudaError_t launch_tinterp_strip(int m, const gf_slot_task* tasks, int ntask, double alpha,
                                  cudaStream_t st);
+cudaError_t launch_leaf_layout(bool to_dense, const int* slots, int n, double* base, double* dense, int S, int nf,
+                               cudaStream_t st);
 cudaError_t launch_slot_copy(int m, const gf_slot_task* tasks, int ntask, cudaStream_t st);
 cudaError_t launch_qinit_sea_level(const double* b, double* h, double* hu, double* hv, long cells,
                                    double sea_level, cudaStream_t st);
