@@ -23,7 +23,7 @@ from dataclasses import dataclass, field
 import numpy as np
 
 from . import _lib
-from ._lib import STATUS_NAMES, dptr, iptr
+from ._lib import STATUS_NAMES, dptr, dptrs, iptr
 
 MBC = 2
 MEQN = 3
@@ -227,8 +227,7 @@ class Context:
         maux = auxs[0].shape[-1]
         dxa = np.ascontiguousarray(np.broadcast_to(np.asarray(dx, np.float64), (n,)))
         dya = np.ascontiguousarray(np.broadcast_to(np.asarray(dy, np.float64), (n,)))
-        qp = (_lib._dp * n)(*[dptr(a) for a in qs])
-        ap = (_lib._dp * n)(*[dptr(a) for a in auxs])
+        qp, ap = dptrs(qs), dptrs(auxs)
         cfl = np.zeros(n)
         mc = C.c_double()
         _check(self.h, self._lib.gf_patch_update_batch(

@@ -350,6 +350,17 @@ def dptr(a: np.ndarray | None):
     return a.ctypes.data_as(_dp)
 
 
+_f8 = np.dtype(np.float64)
+
+
+def dptrs(arrays):
+    """dptr of every array, as the pointer array of a batch: plain addresses,
+    without a pointer object each (half of what 129 patches' call spent)."""
+    for a in arrays:
+        assert a.dtype == _f8 and a.flags.c_contiguous, "need contiguous float64"
+    return C.cast((_vp * len(arrays))(*[a.ctypes.data for a in arrays]), C.POINTER(_dp))
+
+
 def iptr(a: np.ndarray | None):
     if a is None:
         return None
