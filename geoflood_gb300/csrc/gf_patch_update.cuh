@@ -1088,6 +1088,7 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         }
         if (lane == 16) sc[SC_CFL] = 0.0;
     }
+    const int k_lo = (rlo - 1) * N, k_hi = (rhi + 4) * N;
     for (int k = threadIdx.x; k < S; k += NT) {
         double h = sm[L::OFF_H + k];
         if (d_lt<FAST>(h, drytol)) {
@@ -1102,6 +1103,7 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         const bool w = d_gt<FAST>(h, drytol);
         wet[k] = w ? 1 : 0;
         any_wet |= w;
+        if (k < k_lo || k >= k_hi) continue; /* rows that this window's faces do not read */
         double u = 0.0, v = 0.0, c = 0.0, rc = 0.0;
         if (w) {
             if (FAST) {
