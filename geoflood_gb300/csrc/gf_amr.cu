@@ -20,6 +20,7 @@
  */
 #include <cuda_runtime.h>
 
+#include "gf_cmp.cuh"
 #include "gf_internal.h"
 
 namespace gf {
@@ -33,10 +34,49 @@ struct AmrGeo {
     __device__ static int at(int i, int j) { return (j + 1) * N + (i + 1); }
 };
 
+/* The comparisons below are the IEEE ones, taken from the bit patterns where
+ * those decide: an FP64 comparison costs as much as a product here (64 clocks
+ * a warp), and half of a transfer's FP64 instructions were comparisons. */
+
+/* x < d for a positive d (NaN: false) */
+__device__ __forceinline__ bool below(double x, double d)
+{
+    if (!d_gtz<true>(d)) return x < d;
+    const long long b = __double_as_longlong(x);
+    return b < __double_as_longlong(d) && (b & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL;
+}
+/* x > d for a positive d (NaN: false) */
+__device__ __forceinline__ bool above(double x, double d)
+{
+    if (!d_gtz<true>(d)) return x > d;
+    const long long b = __double_as_longlong(x);
+    return b > __double_as_longlong(d) && b <= 0x7ff0000000000000LL;
+}
+/* zero, or far enough from the ends of the range that a product of two such
+ * values neither underflows nor overflows */
+__device__ __forceinline__ bool tame(double x)
+{
+    const unsigned a = static_cast<unsigned>(__double2hiint(x)) & 0x7fffffffu;
+    return a - 0x20000000u < 0x3f000000u || (__double_as_longlong(x) << 1) == 0;
+}
+
 __device__ __forceinline__ double slope_minmod(double sl, double sr)
 {
+    const long long a = __double_as_longlong(sl), b = __double_as_longlong(sr);
+    const long long ma = a & 0x7fffffffffffffffLL, mb = b & 0x7fffffffffffffffLL;
+    if (tame(sl) && tame(sr)) { /* sl sr <= 0 by sign */
+        if ((a ^ b) < 0 || ma == 0 || mb == 0) return 0.0;
+        return ma < mb ? sl : sr;
+    }
     if (sl * sr <= 0.0) return 0.0;
     return fabs(sl) < fabs(sr) ? sl : sr;
+}
+
+/* x / n for n = 1 .. 4: the product with the exact 1, 1/2, 1/4 where it is one */
+__device__ __forceinline__ double over(double x, int n)
+{
+    if (n == 3) return x / 3.0;
+    return x * (n == 1 ? 1.0 : n == 2 ? 0.5 : 0.25);
 }
 
 /* wet-weighted average of 4 fine cells (average_fort.f:154-198) */
@@ -54,7 +94,7 @@ __device__ void avg4(double drytol, const double* qf, const double* bf, const in
         double huf = qf[G::S + k4[m]];
         double hvf = qf[2 * G::S + k4[m]];
         double etaf;
-        if (hf > drytol) {
+        if (above(hf, drytol)) {
             etaf = hf + b;
             nwet = nwet + 1;
         } else {
@@ -68,12 +108,13 @@ __device__ void avg4(double drytol, const double* qf, const double* bf, const in
         etasum = etasum + etaf;
     }
     if (nwet > 0) {
-        const double etaav = etasum / (double)nwet;
-        const double hav = hsum / (double)nwet;
+        const double etaav = over(etasum, nwet);
+        const double hav = over(hsum, nwet);
         const double hc = fmin(hav, fmax(etaav - bc, 0.0));
+        const double f = hc / hsum;
         h = hc;
-        hu = (hc / hsum) * husum;
-        hv = (hc / hsum) * hvsum;
+        hu = f * husum;
+        hv = f * hvsum;
     } else {
         h = hu = hv = 0.0;
     }
@@ -86,37 +127,31 @@ __device__ void interp_cell(double drytol, double sea, const double* qc, const d
                             double* qf, const double* bfp, int ic, int jc, const int* k4, bool clip)
 {
     using G = AmrGeo<M>;
-    for (int mq = 0; mq < 3; ++mq) {
-        double qcv, gx, gy;
-        if (mq == 0) {
-            double eb[3][3];
+    double v[3][4], bed[4];
 #pragma unroll
-            for (int ii = -1; ii <= 1; ++ii)
+    for (int m = 0; m < 4; ++m) bed[m] = bfp[k4[m]];
 #pragma unroll
-                for (int jj = -1; jj <= 1; ++jj) {
-                    const int k = G::at(ic + ii, jc + jj);
-                    const double h = qc[k];
-                    eb[ii + 1][jj + 1] = (h < drytol) ? sea : h + bcp[k];
-                }
-            qcv = eb[1][1];
-            gx = slope_minmod(qcv - eb[0][1], eb[2][1] - qcv);
-            gy = slope_minmod(qcv - eb[1][0], eb[1][2] - qcv);
-        } else {
-            const double* p = qc + mq * G::S;
-            qcv = p[G::at(ic, jc)];
-            gx = slope_minmod(qcv - p[G::at(ic - 1, jc)], p[G::at(ic + 1, jc)] - qcv);
-            gy = slope_minmod(qcv - p[G::at(ic, jc - 1)], p[G::at(ic, jc + 1)] - qcv);
-        }
+    for (int mq = 0; mq < 3; ++mq) { /* all loads before the stores */
+        const double* p = qc + mq * G::S;
+        auto at = [&](int di, int dj) -> double {
+            const int k = G::at(ic + di, jc + dj);
+            const double x = p[k];
+            return mq ? x : below(x, drytol) ? sea : x + bcp[k];
+        };
+        const double qcv = at(0, 0);
+        const double gx = slope_minmod(qcv - at(-1, 0), at(1, 0) - qcv);
+        const double gy = slope_minmod(qcv - at(0, -1), at(0, 1) - qcv);
+        /* a quarter of the slopes either way (exact), x first */
+        const double ax = gx * 0.25, ay = gy * 0.25;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const double sx = ((m & 1) - 0.5) / 2.0, sy = ((m >> 1) - 0.5) / 2.0;
-            double v = qcv + gx * sx + gy * sy;
-            if (mq == 0) {
-                v = v - bfp[k4[m]];
-                if (clip) v = fmax(v, 0.0);
-            }
-            qf[mq * G::S + k4[m]] = v;
-        }
+        for (int m = 0; m < 4; ++m) v[mq][m] = (qcv + ((m & 1) ? ax : -ax)) + ((m >> 1) ? ay : -ay);
+    }
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+        v[0][m] = v[0][m] - bed[m];
+        if (clip) v[0][m] = fmax(v[0][m], 0.0);
+#pragma unroll
+        for (int mq = 0; mq < 3; ++mq) qf[mq * G::S + k4[m]] = v[mq][m];
     }
 }
 
@@ -325,37 +360,66 @@ __device__ int test_regions(const gf_refine& rf, int level, double xl, double yl
     return -1;
 }
 
+/* x > thr for a value x >= 0 known to better than 1e-5 as xf (zero: x = 0):
+ * 1 yes, 0 no, -1 look closer. */
+__device__ __forceinline__ int surely_above(float xf, bool zero, double thr)
+{
+    if (zero) return thr >= 0.0 ? 0 : -1;
+    if (!(xf < 1.0e30f)) return -1;
+    if (thr == 0.0) return xf > 1.0e-20f ? 1 : -1;
+    const float tf = gf_f32(thr);
+    if (!(tf > 1.0e-30f)) return -1;
+    if (!(tf < 1.0e30f)) return 0; /* far above any such value */
+    return xf > tf * 1.0001f ? 1 : xf < tf * 0.9999f ? 0 : -1;
+}
+
 /* fc2d_geoflood_flag2refine.f90:7-130 for one interior cell (allowflag is
- * always true; the legacy regions.i block is never filled). */
+ * always true; the legacy regions.i block is never filled). Momentum and speed
+ * enter as comparisons alone: single-precision values decide them where they
+ * are clear, and only the others take the FP64 root and quotient (with them a
+ * tag launch was bound by FP64 issue, 15 us for 622 patches of 16^2). */
 __device__ int flag2refine(double drytol, double sea, const gf_refine& rf, double h, double hu,
                            double hv, double b, int level, int maxlevel, int init_flag,
                            bool coarsening)
 {
     if (init_flag != 0 && coarsening) return 0;
     const int max_num_speeds = min(rf.num_speed_tolerance, maxlevel);
-    const double momentum = sqrt(hu * hu + hv * hv);
     const double depth = h;
     const double eta = depth + b;
+    const bool wet = above(depth, drytol);
     const int th_factor = coarsening ? 0 : 1; /* integer variable assigned 0.5 */
+    const float ax = fabsf(gf_f32(hu)), ay = fabsf(gf_f32(hv));
+    const float big = fmaxf(ax, ay), ratio = big > 0.0f ? __fdividef(fminf(ax, ay), big) : 0.0f;
+    const float momf = big * sqrtf(1.0f + ratio * ratio);
+    const bool still = ((__double_as_longlong(hu) | __double_as_longlong(hv)) << 1) == 0;
+    auto momentum = [&]() -> double { return sqrt(hu * hu + hv * hv); };
+    auto momentum_above = [&](double v) -> bool {
+        const int s = surely_above(momf, still, v);
+        return s >= 0 ? s != 0 : momentum() > v;
+    };
     for (int m = 0; m < rf.num_flowgrades; ++m) {
         bool needed = false;
         const int var = rf.flowgradevariable[m];
         if (var == 1) needed = depth > rf.flowgradevalue[m];
-        else if (var == 2) needed = momentum > rf.flowgradevalue[m];
-        else if (var == 3 && depth > drytol) needed = fabs(eta) > rf.flowgradevalue[m];
+        else if (var == 2) needed = momentum_above(rf.flowgradevalue[m]);
+        else if (var == 3 && wet) needed = fabs(eta) > rf.flowgradevalue[m];
         if (needed && level < rf.flowgrademinlevel[m]) return 1;
     }
-    double speed = 0.0;
-    if (depth > drytol) {
-        speed = momentum / depth;
+    const float df = gf_f32(depth);
+    const float speedf = df > 1.0e-25f && df < 1.0e25f && big > 1.0e-25f ? __fdividef(momf, df) : 1.0e38f;
+    auto speed_above = [&](double v) -> bool {
+        const int s = surely_above(speedf, still, v);
+        return s >= 0 ? s != 0 : momentum() / depth > v;
+    };
+    if (wet)
         for (int n = 1; n <= max_num_speeds; ++n)
-            if (speed > th_factor * rf.speed_tolerance[n - 1] && level <= n) return 1;
-    }
-    if (rf.num_flowgrades == 0 && depth > drytol) {
+            if (level <= n && speed_above(th_factor * rf.speed_tolerance[n - 1])) return 1;
+    if (rf.num_flowgrades == 0 && wet) {
         if (fabs(eta - sea) > th_factor * rf.wave_tolerance) {
             if (level < rf.max_level_deep) return 1;
             if (fabs(b) < rf.deep_depth) return 1;
         }
+        const double speed = momentum() / depth;
         if (fabs(b) > rf.deep_depth && speed < rf.speed_tolerance[0]) return 0;
         if (speed / depth > rf.max_velocity_depth_product) return 1;
     }
@@ -366,7 +430,7 @@ __device__ int flag2refine(double drytol, double sea, const gf_refine& rf, doubl
  * four siblings of a family. */
 template <int M>
 __global__ void __launch_bounds__(128) tag_kernel(const gf_tag_task* __restrict__ tasks, int ntask,
-                                                  const gf_refine* __restrict__ rfp,
+                                                  const __grid_constant__ gf_refine launch_rf,
                                                   const gf_phys* __restrict__ phys_table,
                                                   int maxlevel, int init_flag, double t,
                                                   int* __restrict__ tags)
@@ -374,8 +438,14 @@ __global__ void __launch_bounds__(128) tag_kernel(const gf_tag_task* __restrict_
     using G = AmrGeo<M>;
     const int ti = blockIdx.x;
     if (ti >= ntask) return;
-    const gf_tag_task T = tasks[ti];
-    const gf_refine& rf = T.rf ? *T.rf : *rfp;
+    /* the task (it may lie in host memory) comes in once, a word a thread */
+    __shared__ gf_tag_task T;
+    static_assert(sizeof(gf_tag_task) % 8 == 0 && sizeof(gf_tag_task) / 8 <= 128, "one word a thread");
+    if (threadIdx.x < sizeof(gf_tag_task) / 8)
+        reinterpret_cast<unsigned long long*>(&T)[threadIdx.x] =
+            reinterpret_cast<const unsigned long long*>(tasks + ti)[threadIdx.x];
+    __syncthreads();
+    const gf_refine& rf = T.rf ? *T.rf : launch_rf;
     if (T.rf) {
         maxlevel = T.maxlevel;
         init_flag = T.init_flag;
@@ -442,10 +512,11 @@ cudaError_t launch_tags(int m, const gf_tag_task* tasks, int ntask, const gf_ref
                         cudaStream_t st)
 {
     if (ntask <= 0) return cudaSuccess;
+    const gf_refine r = rf ? *rf : gf_refine{};
     switch (m) {
-    case 32: tag_kernel<32><<<ntask, 128, 0, st>>>(tasks, ntask, rf, phys, maxlevel, init_flag, t, tags); break;
-    case 16: tag_kernel<16><<<ntask, 128, 0, st>>>(tasks, ntask, rf, phys, maxlevel, init_flag, t, tags); break;
-    case 8: tag_kernel<8><<<ntask, 128, 0, st>>>(tasks, ntask, rf, phys, maxlevel, init_flag, t, tags); break;
+    case 32: tag_kernel<32><<<ntask, 128, 0, st>>>(tasks, ntask, r, phys, maxlevel, init_flag, t, tags); break;
+    case 16: tag_kernel<16><<<ntask, 128, 0, st>>>(tasks, ntask, r, phys, maxlevel, init_flag, t, tags); break;
+    case 8: tag_kernel<8><<<ntask, 128, 0, st>>>(tasks, ntask, r, phys, maxlevel, init_flag, t, tags); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

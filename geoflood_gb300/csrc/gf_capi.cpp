@@ -91,15 +91,14 @@ struct gf_ctx {
     /* scratch for the host-buffer drop-in paths */
     DevBuf<double> q_soa, aux_soa, cfl;
     HostBuf<double> h_cfl;
-    /* a host batch's traffic in one block each side (io_layout) */
-    DevBuf<char> io_dev;
-    HostBuf<char> io_host;
+    HostBuf<char> io_host; /* a host batch's traffic */
     /* coarse/fine transfers and tags */
-    DevBuf<gf_xfer_task> xfer;
+    /* (pinned host memory that the kernels read and write in place: a few
+     * dozen bytes a CTA, cheaper than a copy each way) */
+    HostBuf<gf_xfer_task> xfer;
     DevBuf<gf_tinterp_task> tint;
-    DevBuf<gf_tag_task> tagt;
-    DevBuf<int> tags;
-    DevBuf<gf_refine> refine;
+    HostBuf<gf_tag_task> tagt;
+    HostBuf<int> tags;
     /* qad */
     DevBuf<gf_qad_dev_task> qad;
     DevBuf<double> qad_flux;
@@ -281,13 +280,11 @@ void gf_ctx_destroy(gf_ctx* c)
     c->aux_soa.release();
     c->cfl.release();
     c->h_cfl.release();
-    c->io_dev.release();
     c->io_host.release();
     c->xfer.release();
     c->tint.release();
     c->tagt.release();
     c->tags.release();
-    c->refine.release();
     c->qad.release();
     c->qad_flux.release();
     if (c->d_phys) cudaFree(c->d_phys);
@@ -350,24 +347,19 @@ int gf_patch_update_batch(gf_ctx* c, int npatch, int mx, int my, int mbc, int me
     GF_CK(c, c->aux_soa.reserve(an));
     GF_CK(c, c->cfl.reserve(npatch));
     GF_CK(c, c->h_cfl.reserve(npatch));
-    /* One block each side, [aux | work | status | q]: one copy carries the
-     * batch in (the status zeroed on the host) and one brings the status and
-     * q back. */
+    /* One pinned block, [aux | work | status | q]: the kernels read and write it
+     * in place, no copies. */
     auto a256 = [](size_t b) { return (b + 255) / 256 * 256; };
     const size_t o_work = a256(an * sizeof(double));
     const size_t o_status = o_work + a256((size_t)npatch * sizeof(gf_patch_work));
     const size_t o_q = o_status + a256(sizeof(DevStatus));
-    const size_t io_bytes = o_q + qn * sizeof(double);
-    GF_CK(c, c->io_dev.reserve(io_bytes));
-    GF_CK(c, c->io_host.reserve(io_bytes));
+    GF_CK(c, c->io_host.reserve(o_q + qn * sizeof(double)));
     char* hio = c->io_host.p;
-    char* dio = c->io_dev.p;
     double* hq = reinterpret_cast<double*>(hio + o_q);
     double* ha = reinterpret_cast<double*>(hio);
     gf_patch_work* hw = reinterpret_cast<gf_patch_work*>(hio + o_work);
     DevStatus* hs = reinterpret_cast<DevStatus*>(hio + o_status);
-    DevStatus* d_status = reinterpret_cast<DevStatus*>(dio + o_status);
-    const gf_patch_work* d_work = reinterpret_cast<const gf_patch_work*>(dio + o_work);
+    DevStatus* d_status = c->d_status;
 
     /* Gather the patches into the pinned block; large batches gather on
      * several host threads. */
@@ -389,26 +381,18 @@ int gf_patch_update_batch(gf_ctx* c, int npatch, int mx, int my, int mbc, int me
         w.group = 0;
         hw[k] = w;
     }
-    std::memset(hs, 0, sizeof(DevStatus));
-    GF_CK(c, cudaMemcpyAsync(dio, hio, io_bytes, cudaMemcpyHostToDevice, c->stream));
-    GF_CK(c, gf::launch_aos_to_soa_pair(reinterpret_cast<const double*>(dio + o_q), c->q_soa.p, 3,
-                                        reinterpret_cast<const double*>(dio), c->aux_soa.p, maux, npatch,
-                                        (int)S, c->stream));
-    /* update, layout back, results and status out: one wait at the end */
+    GF_CK(c, gf::launch_batch_in(hq, c->q_soa.p, ha, c->aux_soa.p, maux, npatch, (int)S, &d_status->gmax,
+                                 &d_status->err, c->stream));
+    /* update, layout back with the results: one wait at the end */
     if (c->exact)
-        GF_CK(c, gf::launch_patch_update_exact(mx, d_work, npatch, c->d_phys, dt, nullptr, nullptr, maux,
+        GF_CK(c, gf::launch_patch_update_exact(mx, hw, npatch, c->d_phys, dt, nullptr, nullptr, maux,
                                                c->cfl.p, &d_status->gmax, &d_status->err, c->stream));
     else
-        GF_CK(c, gf::launch_patch_update(mx, d_work, npatch, c->d_phys, dt, nullptr, nullptr, maux,
+        GF_CK(c, gf::launch_patch_update(mx, hw, npatch, c->d_phys, dt, nullptr, nullptr, maux,
                                          c->cfl.p, &d_status->gmax, &d_status->err, c->stream, 0,
                                          small_batch_goal(mx, npatch)));
-    GF_CK(c, gf::launch_soa_to_aos(c->q_soa.p, reinterpret_cast<double*>(dio + o_q), npatch, (int)S, 3,
-                                   3 * S, 3 * S, c->stream));
-    GF_CK(c, cudaMemcpyAsync(hio + o_status, dio + o_status, io_bytes - o_status, cudaMemcpyDeviceToHost,
-                             c->stream));
-    if (cfl)
-        GF_CK(c, cudaMemcpyAsync(c->h_cfl.p, c->cfl.p, sizeof(double) * npatch,
-                                 cudaMemcpyDeviceToHost, c->stream));
+    GF_CK(c, gf::launch_batch_out(c->q_soa.p, hq, npatch, (int)S, c->cfl.p, cfl ? c->h_cfl.p : nullptr,
+                                  &d_status->gmax, &d_status->err, &hs->gmax, &hs->err, c->stream));
     GF_CK(c, cudaStreamSynchronize(c->stream));
     if (hs->err) return fail(c, GF_ERR_DEVICE, "patch kernel: bounded wait expired");
     double mc;
@@ -760,7 +744,10 @@ static int level_prepare(gf_level* L)
 {
     gf_ctx* c = L->ctx;
     if (!L->aux_loaded) return fail(c, GF_ERR_STATE, "level aux (bathymetry) not uploaded");
+    /* patches of one slot in a row share its check (5561 patches: 60 us of a
+     * step if each is checked) */
     for (int k = 0; k < L->npatch; ++k) {
+        if (k > 0 && L->phys[k] == L->phys[k - 1]) continue;
         int rc = check_phys_slot(c, L->phys[k], L->maux);
         if (rc) return rc;
     }
@@ -795,7 +782,9 @@ int gf_level_step(gf_level* L, double t, double dt, double* maxcfl)
 int gf_level_ghost_fill_async(gf_level* L, double t);
 
 /* Chunks for the host-buffer step: equal whole waves of the update kernel
- * (its resident CTAs on all SMs), about two waves or more each, at most 8. */
+ * (its resident CTAs on all SMs), about two waves each, at most 8 (1073
+ * patches of 32^2 1077 us in three chunks, 998 in four; 2490 of 16^2 785 in two,
+ * 725 in three). */
 static int level_pipe_setup(gf_level* L)
 {
     if (L->pipe_ready) return GF_OK;
@@ -803,7 +792,7 @@ static int level_pipe_setup(gf_level* L)
     int sms = 0;
     GF_CK(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
     const int wave = std::max(1, gf::patch_update_occupancy(L->mx) * sms);
-    int k = L->pipe_request > 0 ? L->pipe_request : std::max(1, std::min(8, L->npatch / (2 * wave)));
+    int k = L->pipe_request > 0 ? L->pipe_request : std::max(1, std::min(8, (L->npatch + wave) / (2 * wave)));
     k = std::min(k, L->npatch);
     int chunk = (L->npatch + k - 1) / k;
     if (L->pipe_request <= 0 && k > 1) chunk = (chunk + wave - 1) / wave * wave;
@@ -998,7 +987,9 @@ int gf_level_transfer(gf_level* Cl, gf_level* Fl, int ntask, const gf_transfer* 
     if (Cl->mx != Fl->mx || Cl->maux != Fl->maux)
         return fail(c, GF_ERR_ARG, "coarse and fine levels need the same patch size and maux");
     if (ntask == 0) return GF_OK;
-    std::vector<gf_xfer_task> t(ntask);
+    GF_CK(c, cudaSetDevice(c->device));
+    GF_CK(c, c->xfer.reserve(ntask));
+    gf_xfer_task* t = c->xfer.p;
     for (int k = 0; k < ntask; ++k) {
         const gf_transfer& u = tasks[k];
         if (u.coarse < 0 || u.coarse >= Cl->npatch || u.fine < 0 || u.fine >= Fl->npatch)
@@ -1038,14 +1029,12 @@ int gf_level_transfer(gf_level* Cl, gf_level* Fl, int ntask, const gf_transfer* 
         x.ox = u.ox;
         x.oy = u.oy;
         x.phys = Cl->phys[u.coarse];
+        x.group = 0;
+        if (k > 0 && x.phys == t[k - 1].phys) continue; /* checked */
         int rc = check_phys_slot(c, x.phys);
         if (rc) return rc;
     }
-    GF_CK(c, cudaSetDevice(c->device));
-    GF_CK(c, c->xfer.reserve(ntask));
-    GF_CK(c, cudaMemcpyAsync(c->xfer.p, t.data(), ntask * sizeof(gf_xfer_task),
-                             cudaMemcpyHostToDevice, c->stream));
-    GF_CK(c, gf::launch_transfer(Cl->mx, c->xfer.p, ntask, c->d_phys, c->stream));
+    GF_CK(c, gf::launch_transfer(Cl->mx, t, ntask, c->d_phys, c->stream));
     GF_CK(c, cudaStreamSynchronize(c->stream));
     return GF_OK;
 }
@@ -1145,14 +1134,11 @@ static int run_tags(gf_level* L, const gf_refine* rf, std::vector<gf_tag_task>& 
     GF_CK(c, cudaSetDevice(c->device));
     GF_CK(c, c->tagt.reserve(n));
     GF_CK(c, c->tags.reserve(n));
-    GF_CK(c, c->refine.reserve(1));
-    GF_CK(c, cudaMemcpyAsync(c->refine.p, rf, sizeof(gf_refine), cudaMemcpyHostToDevice, c->stream));
-    GF_CK(c, cudaMemcpyAsync(c->tagt.p, t.data(), n * sizeof(gf_tag_task), cudaMemcpyHostToDevice,
-                             c->stream));
-    GF_CK(c, gf::launch_tags(L->mx, c->tagt.p, n, c->refine.p, c->d_phys, maxlevel, init_flag, tm,
+    std::memcpy(c->tagt.p, t.data(), n * sizeof(gf_tag_task));
+    GF_CK(c, gf::launch_tags(L->mx, c->tagt.p, n, rf, c->d_phys, maxlevel, init_flag, tm,
                              c->tags.p, c->stream));
-    GF_CK(c, cudaMemcpyAsync(tags, c->tags.p, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     GF_CK(c, cudaStreamSynchronize(c->stream));
+    std::memcpy(tags, c->tags.p, n * sizeof(int));
     return GF_OK;
 }
 
@@ -1162,8 +1148,8 @@ int gf_level_tag4refinement(gf_level* L, const gf_refine* rf, int level, int max
     if (!L || !rf || !tags) return GF_ERR_ARG;
     std::vector<gf_tag_task> tk(L->npatch);
     for (int k = 0; k < L->npatch; ++k) {
-        int rc = check_phys_slot(L->ctx, L->phys[k]);
-        if (rc) return rc;
+        if (k == 0 || L->phys[k] != L->phys[k - 1])
+            if (int rc = check_phys_slot(L->ctx, L->phys[k])) return rc;
         gf_tag_task& x = tk[k];
         std::memset(&x, 0, sizeof x);
         x.q[0] = L->d_q + (size_t)k * 3 * L->S;

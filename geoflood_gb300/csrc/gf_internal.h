@@ -96,8 +96,11 @@ cudaError_t launch_soa_to_aos(const double* src, double* dst, long npatch, int n
                               long src_stride, long dst_stride, cudaStream_t st);
 /* both of a host batch's layouts (q with nfa fields, aux with nfb) in one
  * launch; each set is npatch contiguous blocks of nf * ncell doubles */
-cudaError_t launch_aos_to_soa_pair(const double* sa, double* da, int nfa, const double* sb, double* db,
-                                   int nfb, long npatch, int ncell, cudaStream_t st);
+cudaError_t launch_batch_in(const double* hq, double* q, const double* ha, double* aux, int maux, long npatch,
+                            int ncell, unsigned long long* gmax, int* err, cudaStream_t st);
+cudaError_t launch_batch_out(const double* q, double* hq, long npatch, int ncell, const double* cfl, double* hcfl,
+                             const unsigned long long* gmax, const int* err, unsigned long long* hgmax, int* herr,
+                             cudaStream_t st);
 
 /* Served scenarios: device-side time-step control around a round. */
 cudaError_t launch_served_prepare(gf_group_state* gs, gf_ghost_block* blocks, double* gdt, int* gpar,
