@@ -51,7 +51,6 @@ cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, con
                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                 unsigned long long* gmax, int* err, cudaStream_t st,
                                 int max_ctas = 0, int goal = 0);
-size_t patch_update_smem_bytes(int m);
 int patch_update_occupancy(int m); /* resident CTAs per SM (throughput tile) */
 
 /* Tile shapes of the production patch kernel: variants per patch size, the

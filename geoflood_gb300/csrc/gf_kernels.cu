@@ -51,16 +51,16 @@ static cudaError_t launch_stream(const gf_patch_work* work, int nwork, const gf_
     return cudaGetLastError();
 }
 
-/* The latency form: each work item on a cluster of K CTAs (one window of
+/* The split form: each work item on a cluster of K CTAs (one window of
  * rows each); not persistent, so max_ctas does not apply. */
-template <int M, int NT, int RB, int K>
+template <int M, int NT, int R, int K, int MINB>
 static cudaError_t launch_window(const gf_patch_work* work, int nwork, const gf_phys* phys,
                                  double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                  unsigned long long* gmax, int* err, int max_ctas, cudaStream_t st)
 {
     (void)max_ctas;
-    using L = Smem<M, RB, false>;
-    auto kern = patch_update_window_kernel<M, NT, RB, K, false>;
+    using L = StreamSmem<M, R, K>;
+    auto kern = patch_update_window_kernel<M, NT, R, K, MINB>;
     static std::atomic<unsigned long long> attr_done{0};
     cudaError_t ae = smem_attr_per_device(kern, (int)L::BYTES, attr_done);
     if (ae != cudaSuccess) return ae;
@@ -71,11 +71,11 @@ static cudaError_t launch_window(const gf_patch_work* work, int nwork, const gf_
 
 /* Patches one launch of the window kernel runs at once: the clusters of K
  * CTAs the device holds resident together (placement inside a GPC counted). */
-template <int M, int NT, int RB, int K>
+template <int M, int NT, int R, int K, int MINB>
 static int window_slots()
 {
-    using L = Smem<M, RB, false>;
-    auto kern = patch_update_window_kernel<M, NT, RB, K, false>;
+    using L = StreamSmem<M, R, K>;
+    auto kern = patch_update_window_kernel<M, NT, R, K, MINB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) !=
         cudaSuccess)
         return 0;
@@ -88,11 +88,11 @@ static int window_slots()
     return n;
 }
 
-template <int M, int NT, int RB, int K>
+template <int M, int NT, int R, int K, int MINB>
 static int window_occupancy()
 {
-    using L = Smem<M, RB, false>;
-    auto kern = patch_update_window_kernel<M, NT, RB, K, false>;
+    using L = StreamSmem<M, R, K>;
+    auto kern = patch_update_window_kernel<M, NT, R, K, MINB>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::BYTES) !=
         cudaSuccess)
         return 0;
@@ -155,16 +155,16 @@ struct Tile {
 #define GF_STILE(M, NT, R, MINB)                                                              \
     {NT, R, 1, &launch_stream<M, NT, R, MINB>, &stream_occupancy<M, NT, R, MINB>,             \
      &stream_slots<M, NT, R, MINB>}
-#define GF_WTILE(M, NT, RB, K)                                                                \
-    {NT, RB, K, &launch_window<M, NT, RB, K>, &window_occupancy<M, NT, RB, K>,                \
-     &window_slots<M, NT, RB, K>}
-static const Tile kTiles8[] = {GF_TILE(8, 64, 5, 6), GF_TILE(8, 128, 10, 4), GF_STILE(8, 128, 11, 3),
-                               GF_WTILE(8, 64, 5, 2), GF_WTILE(8, 64, 5, 4)};
-static const Tile kTiles16[] = {GF_TILE(16, 128, 6, 3), GF_STILE(16, 192, 7, 2), GF_TILE(16, 256, 9, 2),
-                                GF_WTILE(16, 128, 6, 2), GF_WTILE(16, 128, 6, 4), GF_WTILE(16, 256, 9, 4)};
+#define GF_WTILE(M, NT, R, K, MINB)                                                           \
+    {NT, R, K, &launch_window<M, NT, R, K, MINB>, &window_occupancy<M, NT, R, K, MINB>,       \
+     &window_slots<M, NT, R, K, MINB>}
+static const Tile kTiles8[] = {GF_TILE(8, 64, 5, 6), GF_TILE(8, 128, 10, 4), GF_STILE(8, 128, 11, 4),
+                               GF_WTILE(8, 128, 7, 2, 2), GF_WTILE(8, 128, 5, 4, 2)};
+static const Tile kTiles16[] = {GF_STILE(16, 128, 5, 3), GF_STILE(16, 192, 7, 2), GF_TILE(16, 256, 9, 2),
+                                GF_WTILE(16, 256, 11, 2, 2), GF_WTILE(16, 256, 7, 4, 1), GF_WTILE(16, 256, 5, 8, 1)};
 static const Tile kTiles32[] = {GF_TILE(32, 256, 7, 1), GF_STILE(32, 256, 4, 2), GF_TILE(32, 384, 7, 1),
-                                GF_TILE(32, 384, 9, 1), GF_WTILE(32, 256, 7, 4), GF_WTILE(32, 256, 7, 8),
-                                GF_WTILE(32, 256, 7, 2)};
+                                GF_TILE(32, 384, 9, 1), GF_WTILE(32, 384, 11, 4, 1), GF_WTILE(32, 384, 7, 8, 1),
+                                GF_WTILE(32, 384, 10, 2, 1)};
 #undef GF_TILE
 #undef GF_STILE
 #undef GF_WTILE
@@ -182,9 +182,11 @@ static const Tile* tiles_of(int m, int* n)
 /* Selected variant per goal (0 throughput, 1 latency) and patch size, and the
  * selection that stands for "by the number of patches" (pick_tile): the
  * defaults here, or what gf_autotune installed. 8^2 patches take the
- * streamed form, a whole patch in its one band (24 patches 33 us, 4096 patches
- * 310 us; 128 x 10 swept 39 and 323); 32^2 patches 384 x 9 (4096 patches 3.34
- * ms, 256 x 7 3.61) or the streamed form, pick_tile. */
+ * streamed form, a whole patch in its one band, four CTAs an SM (4096 patches
+ * 288 us, three CTAs 305, 128 x 10 swept 323), 16^2 its bands of five rows,
+ * three CTAs an SM (5561 patches 1.27 ms at 80 % wet and 0.85 at 50 %, swept
+ * 128 x 6 1.31 and 0.92, streamed 192 x 7 1.34 and 0.93), 32^2 patches 384 x 9
+ * (4096 patches 3.43 ms, 256 x 7 3.61) or the streamed form, pick_tile. */
 static int g_tile[2][3] = {{2, 0, 3}, {2, 0, 3}};
 static int g_auto[2][3] = {{2, 0, 3}, {2, 0, 3}};
 static bool g_tuned[3] = {false, false, false};
@@ -239,17 +241,20 @@ int latency_goal_fits(int m, long npatch)
 }
 
 /* Launches that leave SMs idle take a tile that spreads a patch: the first of
- * these whose CTAs all run at once with at most per_sm of them on an SM (FP64
- * throughput is the SM's, so a split pays while SMs are free). us for that
- * many 32^2 patches: K = 8 50 (1), K = 4 76 (24), K = 2 107 (72), one CTA 170
- * (144); 16^2: 256 x 9 over K = 4 41 (24), 128 x 6 over K = 4 51 (72), the
- * streamed 192 x 7 60 (152) and 91 (304), 128 x 6 80 and 103. The split of an
- * 8^2 patch gains nothing (33 us against 32). */
+ * these with at most per_2sm CTAs for two SMs (FP64 throughput is the SM's, so a
+ * split pays while SMs are free), and, for one_wave, all of them resident at
+ * once. us for that many 32^2 patches, the next choice beside it: K = 8 42 (1;
+ * 56), K = 4 55 (24; 90), K = 2 90 (72; 171), 167 (152; 188), 251 (247; 288), but
+ * 325 (304; 289); 16^2: K = 8 29 (1; 31), K = 4 33 (24; 40), K = 2 41 (72; 64), 54
+ * (152; 64), the streamed 192 x 7 94 (304; 102) and 166 (400; 134); 8^2: K = 4 29
+ * (24; 35) and 31 (72; 31). */
 struct SmallTile {
-    int v, per_sm;
+    int v, per_2sm;
+    bool one_wave;
 };
-static const SmallTile kSmall16[] = {{5, 1}, {4, 2}, {1, 2}};
-static const SmallTile kSmall32[] = {{5, 1}, {4, 1}, {6, 1}};
+static const SmallTile kSmall8[] = {{4, 2, true}};
+static const SmallTile kSmall16[] = {{5, 2, true}, {4, 2, true}, {3, 4, true}, {1, 4, true}};
+static const SmallTile kSmall32[] = {{5, 2, true}, {4, 2, true}, {6, 7, false}};
 /* Whole 32^2 levels: the streamed tile, two CTAs an SM, when it fills its slots
  * once (247 patches 286 us, 384 x 9 301) or many times (4096 patches 3.18 ms,
  * 3.34; 1215 1.07, 1.09); between, its half-empty last wave costs more than it
@@ -262,12 +267,14 @@ static int pick_tile(int m, long npatch, int max_ctas, int goal)
     goal = goal != 0;
     /* chosen by hand, or the tuned latency tile asked for */
     if (g_tile[goal][c] != g_auto[goal][c] || (goal && g_tuned[c])) return g_tile[goal][c];
-    if (max_ctas <= 0 && c != 0) {
+    if (max_ctas <= 0) {
         int nt = 0;
         const Tile* t = tiles_of(m, &nt);
-        const SmallTile* s = c == 1 ? kSmall16 : kSmall32;
-        for (int i = 0; i < 3; ++i)
-            if (npatch * t[s[i].v].k <= (long)s[i].per_sm * sm_count() && npatch <= tile_resident(m, s[i].v))
+        const SmallTile* s = c == 0 ? kSmall8 : c == 1 ? kSmall16 : kSmall32;
+        const int ns = (int)(c == 0 ? sizeof kSmall8 : c == 1 ? sizeof kSmall16 : sizeof kSmall32) / (int)sizeof *s;
+        for (int i = 0; i < ns; ++i)
+            if (2 * npatch * t[s[i].v].k <= (long)s[i].per_2sm * sm_count() &&
+                (!s[i].one_wave || npatch <= tile_resident(m, s[i].v)))
                 return s[i].v;
         if (c == 2 && !g_tuned[c] &&
             (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
@@ -378,16 +385,6 @@ int patch_update_occupancy(int m)
     int n = 0;
     const Tile* t = tiles_of(m, &n);
     return t ? t[g_tile[0][mcls(m)]].occ() : 0;
-}
-
-size_t patch_update_smem_bytes(int m)
-{
-    switch (m) {
-    case 32: return Smem<32, 7>::BYTES;
-    case 16: return Smem<16, 6>::BYTES;
-    case 8: return Smem<8, 5>::BYTES;
-    default: return 0;
-    }
 }
 
 /* ---- layout conversion at the boundary ----

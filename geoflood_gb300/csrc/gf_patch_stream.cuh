@@ -25,6 +25,14 @@
  * Every value is formed by the same operations and summed in the same order as
  * by the sweeps: the results are the same bits.
  *
+ * The window kernel splits a patch over a cluster of K CTAs, each with the rows
+ * of one window, all staged at its start. x and y faces side by side fill the
+ * warps of an SM that holds one window (14 chunks of normal solves for four
+ * rows of 32^2): a lone 32^2 patch 42 us over K = 8 (the sweeps split over the
+ * same cluster 50), 24 patches 55 us over K = 4 (76), 72 90 us over K = 2 (107).
+ * What is left is the chain of FP64 instructions of one face and one cell, 64
+ * cycles each.
+ *
  * Before a band is staged the item's depths are read once. A patch without
  * water is written at once; else the bands start and end with its wet rows (the
  * records before them are zero), and the rows beyond are written like a dry
@@ -37,26 +45,30 @@
 
 namespace GF_KNS {
 
-template <int M, int R>
+template <int M, int R, int K = 1>
 struct StreamSmem {
     static constexpr int N = M + 2 * GF_MBC;
+    static constexpr int RW = M / K;             /* cell rows that the CTA finishes       */
     static constexpr int FA = M + 3, FB = M + 1; /* x faces of a slice: solved, limited  */
     static constexpr int NC = M + 2;             /* y faces of a row (columns 1 .. M + 2) */
-    static constexpr int NB = (M + 3 + R - 1) / R;
+    static constexpr int NB = (RW + 3 + R - 1) / R;
+    static constexpr bool ONE = NB == 1;
     /* rows in use at once: G of b - 1 reads from a0 - R - 2, staging of b + 1
-     * writes to a0 + 2 R - 1 */
-    static constexpr int ROWS = 3 * R + 2 < N ? 3 * R + 2 : N;
+     * writes to a0 + 2 R - 1; a window stages all its rows at its start */
+    static constexpr int ROWS = K == 1 && 3 * R + 2 < N ? 3 * R + 2 : RW + 4;
     /* one row more of the wet flags: B2 looks below its first row */
-    static constexpr int WROWS = 3 * R + 3 < N ? 3 * R + 3 : N;
+    static constexpr int WROWS = K == 1 && 3 * R + 3 < N ? 3 * R + 3 : RW + 4;
     static constexpr int PL = ROWS * N;
     static constexpr int WS = 11, OS = 9, CS = 9; /* record strides, as in Smem */
     static constexpr int OFF_H = 0, OFF_HU = PL, OFF_HV = 2 * PL, OFF_B = 3 * PL, OFF_U = 4 * PL, OFF_V = 5 * PL,
                          OFF_C = 6 * PL, OFF_RC = 7 * PL;
-    static constexpr int RWY = R + 2, ROY = R + 1, RCX = R + 3, RCY = R; /* rings of rows */
+    /* rings of rows; with one band, its rows */
+    static constexpr int RX = ONE ? RW + 2 : R, RWY = ONE ? RW + 3 : R + 2, ROY = ONE ? RW + 1 : R + 1,
+                         RCX = ONE ? RW + 2 : R + 3, RCY = ONE ? RW : R;
     static constexpr int OFF_WX = 8 * PL;
-    static constexpr int OFF_WY = OFF_WX + R * FA * WS;
+    static constexpr int OFF_WY = OFF_WX + RX * FA * WS;
     static constexpr int OFF_OX = OFF_WY + RWY * NC * WS;
-    static constexpr int OFF_OY = OFF_OX + R * FB * OS;
+    static constexpr int OFF_OY = OFF_OX + RX * FB * OS;
     static constexpr int OFF_CX = OFF_OY + ROY * NC * OS;
     static constexpr int OFF_CY = OFF_CX + RCX * M * CS;
     static constexpr int OFF_SC = OFF_CY + RCY * NC * CS;
@@ -73,21 +85,22 @@ struct StreamSmem {
     static __device__ __forceinline__ int wi(int row, int col) { return (WROWS == N ? row : row % WROWS) * N + col; }
 };
 
-/* Rows of band b: x slices and y faces from a0 (x1, y1 past their ends), y
- * limited faces l0 .. l1 - 1, finished cell rows c0 .. c1 - 1. */
-template <int M, int R>
+/* Rows of band b of the RW rows above array row o + 1: x slices and y faces
+ * from a0 (x1, y1 past their ends), y limited faces l0 .. l1 - 1, finished cell
+ * rows c0 .. c1 - 1. */
+template <int RW, int R>
 struct StreamBand {
     int a0, nx, ny, l0, nl, c0, nc;
-    __device__ __forceinline__ explicit StreamBand(int b)
+    __device__ __forceinline__ StreamBand(int b, int o)
     {
-        a0 = 1 + b * R;
-        const int y1 = min(a0 + R, M + 4);
-        nx = min(a0 + R, M + 3) - a0;
+        a0 = 1 + o + b * R;
+        const int y1 = min(a0 + R, o + RW + 4);
+        nx = min(a0 + R, o + RW + 3) - a0;
         ny = y1 - a0;
-        l0 = max(a0 - 1, 2);
-        nl = max(min(y1 - 1, M + 3) - l0, 0);
-        c0 = max(a0 - 2, 2);
-        nc = max(min(y1 - 2, M + 2) - c0, 0);
+        l0 = max(a0 - 1, o + 2);
+        nl = max(min(y1 - 1, o + RW + 3) - l0, 0);
+        c0 = max(a0 - 2, o + 2);
+        nc = max(min(y1 - 2, o + RW + 2) - c0, 0);
     }
 };
 
@@ -107,16 +120,21 @@ __device__ __forceinline__ gf_cell stream_cell(const double* sm, bool wet, int k
     return c;
 }
 
-/* One work item; as patch_item. */
-template <int M, int NT, int R>
+/* One work item; as patch_item. K > 1: window win of the K windows of rows
+ * whose CTAs form a cluster; its largest speed goes to *part. */
+template <int M, int NT, int R, int K = 1>
 __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t& phase, gf_patch_work wk, int wi,
                                             const gf_phys* __restrict__ phys_table, double dt_uniform,
                                             const double* __restrict__ group_dt, const int* __restrict__ group_par,
                                             int maux, double* __restrict__ cfl_out,
-                                            unsigned long long* __restrict__ group_max, int* __restrict__ err)
+                                            unsigned long long* __restrict__ group_max, int* __restrict__ err,
+                                            int win = 0, double* part = nullptr)
 {
-    using L = StreamSmem<M, R>;
-    constexpr int N = L::N, S = N * N, NB = L::NB;
+    using L = StreamSmem<M, R, K>;
+    using Band = StreamBand<L::RW, R>;
+    constexpr int N = L::N, S = N * N, NB = L::NB, RW = L::RW;
+    const int o = K > 1 ? win * RW : 0; /* first row that the item reads */
+    const int top = o + RW + 4;         /* past the last */
     int* cnt = reinterpret_cast<int*>(sm + L::OFF_INT);
     uint16_t* la = reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(sm) + L::OFF_LIST);
     uint16_t *lm = la + L::LIST_A, *lb = lm + L::LIST_A;
@@ -134,7 +152,13 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     if (wk.fl && wk.fl->skip) return true;
     const gf_phys P = phys_table[wk.phys];
     const double g = P.grav, drytol = P.dry_tolerance;
-    if (__syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<volatile int*>(err) != 0)) return false;
+    if (__syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<volatile int*>(err) != 0)) {
+        if (K > 1) {
+            cluster_arrive();
+            cluster_wait();
+        }
+        return false;
+    }
 
     auto stage = [&](int r0, int r1) { /* one thread */
         mbar_expect_tx(bar, (uint32_t)(4 * (r1 - r0) * N * sizeof(double)));
@@ -148,6 +172,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         }
     };
     int any_wet = 0, changed = 0;
+    unsigned kept = 0; /* K > 1: bit r - o, row r holds a cell b4step2 leaves alone */
     /* b4step2 and the quotients of the cells e0, e0 + step, .. of rows r0 .. */
     auto prepare = [&](int r0, int e0, int e1, int step) {
         for (int e = e0; e < e1; e += step) {
@@ -158,6 +183,8 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
                 sm[L::OFF_H + k] = h;
                 sm[L::OFF_HU + k] = 0.0;
                 sm[L::OFF_HV + k] = 0.0;
+            } else if (K > 1) {
+                kept |= 1u << (r0 + rr - o);
             }
             const bool w = d_gt<true>(h, drytol);
             wet[L::wi(r0 + rr, col)] = w ? 1 : 0;
@@ -185,11 +212,29 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         return false;
     };
 
-    /* the rows that hold a cell b4step2 would leave alone (h >= dry_tolerance) */
     unsigned* rows = reinterpret_cast<unsigned*>(cnt + L::CNT_ROWS);
+    auto constants = [&]() { /* the last warp: the item's constants, one lane each */
+        const double q = (lane < 2 ? dt : 1.0) / (lane == 0 ? wk.dx : lane == 1 ? wk.dy : 16.0 * g);
+        if (lane < 3) sc[SC_DTDX + lane] = q;
+        if (lane == 3) sc[SC_RSG] = rsqrt(g);
+        if (lane == 4) {
+            const double crit = fmax(drytol * g, 1e-6);
+            sc[SC_CRIT] = crit;
+            sc[SC_CRIT2] = sqrt(crit);
+        }
+        if (lane >= 8 && lane < 8 + GF_MAX_MANNING) {
+            const double n = P.manning_coefficient[lane - 8];
+            sc[SC_KF + lane - 8] = gf_mul(gf_mul(dt, g), gf_mul(n, n));
+        }
+        if (lane == 16) sc[SC_CFL] = 0.0;
+    };
     for (int k = threadIdx.x; k < L::CNT_INTS; k += NT) cnt[k] = 0;
     __syncthreads();
-    {
+    if (K > 1) {
+        if (threadIdx.x == 0) stage(o, top);
+        if (warp == NT / 32 - 1) constants();
+    } else {
+        /* the rows that hold a cell b4step2 would leave alone (h >= dry_tolerance) */
         constexpr int IT = (S + NT - 1) / NT;
         double h[IT];
 #pragma unroll
@@ -212,9 +257,8 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
             atomicOr(&rows[0], lo);
             atomicOr(&rows[1], hi);
         }
+        __syncthreads();
     }
-    __syncthreads();
-    const unsigned long long wrows = (unsigned long long)rows[1] << 32 | rows[0];
     double* gq = wk.qout ? wk.qout : wk.q;
     /* interior rows r0 .. r1 - 1 without water: b4step2 alone changes them */
     auto write_dry = [&](int r0, int r1) {
@@ -225,18 +269,44 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
             gq[2 * S + k] = 0.0;
         }
     };
-    if (wk.fl) { /* b4step2 changes a cell's bits unless h >= 0 and both momenta are +0 */
+    if (wk.fl && win == 0) { /* b4step2 changes a cell's bits unless h >= 0 and both momenta are +0 */
+        int water = 0;
         for (int k = threadIdx.x; k < S; k += NT) {
             const double h = wk.q[k];
             if (d_lt<true>(h, drytol))
                 changed |= (__double_as_longlong(h) < 0) | (__double_as_longlong(wk.q[S + k]) != 0) |
                            (__double_as_longlong(wk.q[2 * S + k]) != 0);
+            else if (K > 1) water |= d_gt<true>(h, drytol);
         }
         changed = __syncthreads_or(changed);
+        if (K > 1) {
+            water = __syncthreads_or(water);
+            if (threadIdx.x == 0) {
+                wk.fl->ident = (!water && !changed) ? 1 : 0;
+                wk.fl->wet = water ? 1 : 0;
+            }
+        }
     }
+    if (K > 1) {
+        const bool ok = __syncthreads_and(wait_staged());
+        if (!ok) fail();
+        /* the windows are written in place: none before all are staged */
+        cluster_arrive();
+        if (!ok) {
+            cluster_wait();
+            return false;
+        }
+        staged ^= 1u;
+        prepare(o, threadIdx.x, (RW + 4) * N, NT);
+        kept = __reduce_or_sync(0xffffffffu, kept);
+        if (lane == 0 && kept) atomicOr(&rows[0], kept);
+        __syncthreads();
+    }
+    const unsigned long long wrows = (unsigned long long)rows[1] << 32 | rows[0]; /* from row o */
     if (wrows == 0) {
-        write_dry(2, M + 2);
-        if (threadIdx.x == 0) {
+        if (K > 1) cluster_wait();
+        write_dry(o + 2, o + RW + 2);
+        if (K == 1 && threadIdx.x == 0) {
             if (wk.fl) {
                 wk.fl->ident = !changed ? 1 : 0;
                 wk.fl->wet = 0;
@@ -250,31 +320,18 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     /* bands b0 .. b1: the solves of the first wet row, up to the finish of the
      * row above the last */
     const int w0 = __ffsll((long long)wrows) - 1, w1 = 63 - __clzll((long long)wrows);
-    const int b0 = max(w0 - 1, 0) / R, b1 = min(NB - 1, (min(w1 + 1, M + 1) + 2 + R - 1) / R - 1);
-    const int first = 1 + b0 * R; /* its array row */
-    if (threadIdx.x == 0) stage(max(first - 3, 0), min(first + R, N));
+    const int b0 = max(w0 - 1, 0) / R, b1 = min(NB - 1, (min(w1 + 1, RW + 1) + 2 + R - 1) / R - 1);
+    const int first = o + 1 + b0 * R; /* its array row */
+    if (K == 1 && threadIdx.x == 0) stage(max(first - 3, 0), min(first + R, N));
     if (b0 > 0) /* the records below the first band */
         for (int k = L::OFF_WX + (int)threadIdx.x; k < L::OFF_SC; k += NT) sm[k] = 0.0;
-    if (warp == NT / 32 - 1) {
-        /* the item's constants, one lane each */
-        const double q = (lane < 2 ? dt : 1.0) / (lane == 0 ? wk.dx : lane == 1 ? wk.dy : 16.0 * g);
-        if (lane < 3) sc[SC_DTDX + lane] = q;
-        if (lane == 3) sc[SC_RSG] = rsqrt(g);
-        if (lane == 4) {
-            const double crit = fmax(drytol * g, 1e-6);
-            sc[SC_CRIT] = crit;
-            sc[SC_CRIT2] = sqrt(crit);
-        }
-        if (lane >= 8 && lane < 8 + GF_MAX_MANNING) {
-            const double n = P.manning_coefficient[lane - 8];
-            sc[SC_KF + lane - 8] = gf_mul(gf_mul(dt, g), gf_mul(n, n));
-        }
-        if (lane == 16) sc[SC_CFL] = 0.0;
+    if (K == 1) {
+        if (warp == NT / 32 - 1) constants();
+        if (!__syncthreads_and(wait_staged())) return fail();
+        prepare(max(first - 3, 0), threadIdx.x, (min(first + R, N) - max(first - 3, 0)) * N, NT);
+        staged ^= 1u;
     }
-    if (!__syncthreads_and(wait_staged())) return fail();
-    prepare(max(first - 3, 0), threadIdx.x, (min(first + R, N) - max(first - 3, 0)) * N, NT);
-    __syncthreads();
-    staged ^= 1u;
+    if (K == 1 || b0 > 0) __syncthreads();
 
     const double dtdx = sc[SC_DTDX], dtdy = sc[SC_DTDY], crit = sc[SC_CRIT], crit2 = sc[SC_CRIT2];
     const double hx = gf_mul(0.5, dtdx), hy = gf_mul(0.5, dtdy);
@@ -291,7 +348,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     };
     /* the normal-solve faces of band b by class, as list_chunk: entries number
      * the x faces by row, then the y faces by row */
-    auto list_a = [&](const StreamBand<M, R>& B, int par, int c) {
+    auto list_a = [&](const Band& B, int par, int c) {
         const int na = B.nx * L::FA + B.ny * L::NC;
         const bool act = 32 * c + lane < na;
         const int i = act ? 32 * c + lane : 0;
@@ -328,7 +385,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
             to[cls >= 2 ? na - 1 - pos : pos] = (uint16_t)(i | (flag ? 0x8000 : 0));
         }
     };
-    auto chunk_a = [&](const StreamBand<M, R>& B, int par, int c) {
+    auto chunk_a = [&](const Band& B, int par, int c) {
         const int ns = cnt[4 * par], ne = cnt[4 * par + 1], nh = cnt[4 * par + 2], nd = cnt[4 * par + 3];
         const int nA = ns + ne + nh + nd, idx = 32 * c + lane;
         if (idx >= nA) return;
@@ -376,7 +433,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         else smax_x = d_max_nn<true>(smax_x, m);
     };
     /* limited face i of band b: its records and its cells' wet flags */
-    auto limited = [&](const StreamBand<M, R>& B, int i, int& w, int& wl, int& wr, int& o, int& kl, int& kr) -> bool {
+    auto limited = [&](const Band& B, int i, int& w, int& wl, int& wr, int& o, int& kl, int& kr) -> bool {
         const bool y = i >= B.nx * L::FB;
         if (!y) {
             const int ts = i / L::FB, n = 1 + (i - ts * L::FB);
@@ -397,7 +454,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         }
         return y;
     };
-    auto list_b = [&](const StreamBand<M, R>& B, int par, int c) {
+    auto list_b = [&](const Band& B, int par, int c) {
         const int nb = B.nx * L::FB + B.nl * L::NC, i = 32 * c + lane;
         const bool act = i < nb;
         bool dry = false;
@@ -409,7 +466,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         const int pos = place(cnt + L::CNT_B + 2 * par, act ? (dry ? 1 : 0) : -1);
         if (act) lb[dry ? nb - 1 - pos : pos] = (uint16_t)i;
     };
-    auto chunk_b1 = [&](const StreamBand<M, R>& B, int par, int c) {
+    auto chunk_b1 = [&](const Band& B, int par, int c) {
         const int nw = cnt[L::CNT_B + 2 * par], idx = 32 * c + lane;
         if (idx >= nw + cnt[L::CNT_B + 2 * par + 1]) return;
         int w, wl, wr, o, kl, kr;
@@ -429,7 +486,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
             op[6 + k] = cq[k];
         }
     };
-    auto chunk_b2 = [&](const StreamBand<M, R>& B, int c) {
+    auto chunk_b2 = [&](const Band& B, int c) {
         const int i = 32 * c + lane;
         if (i >= B.nx * M + B.nc * L::NC) return;
         const bool y = i >= B.nx * M;
@@ -475,7 +532,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     };
     /* finished cells: the sums of the sweeps in their order, the update and the
      * friction term */
-    auto chunk_g = [&](const StreamBand<M, R>& B, int c) {
+    auto chunk_g = [&](const Band& B, int c) {
         const int i = 32 * c + lane;
         if (i >= B.nc * M) return;
         const int ts = i / M, n = i - ts * M, row = B.c0 + ts;
@@ -508,7 +565,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     };
 
     {
-        const StreamBand<M, R> B0(b0);
+        const Band B0(b0, o);
         for (int c = warp; 32 * c < B0.nx * L::FA + B0.ny * L::NC; c += NT / 32) list_a(B0, b0 & 1, c);
     }
     __syncthreads();
@@ -522,8 +579,8 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     for (int b = b0;; ++b) {
         /* more: rows above the band still to come (the last band's records need
          * the bathymetry above it); mlist: a next band to list */
-        const bool have = b <= b1, more = have && b + 1 < NB, mlist = b < b1;
-        const StreamBand<M, R> B(b), Bp(b - 1);
+        const bool have = b <= b1, more = K == 1 && have && b + 1 < NB, mlist = b < b1;
+        const Band B(b, o), Bp(b - 1, o);
         const int par = b & 1;
         /* ---- A | B2 of the band before | dry list | next rows ---- */
         const int r0 = 1 + (b + 1) * R, r1 = more ? min(r0 + R, N) : r0;
@@ -550,7 +607,8 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         if (threadIdx.x < 2) cnt[L::CNT_B + 2 * (par ^ 1) + threadIdx.x] = 0;
         /* ---- B1 | class list of the next band | finished rows ---- */
         if (more) staged ^= 1u;
-        const StreamBand<M, R> Bn(b + 1);
+        const Band Bn(b + 1, o);
+        if (K > 1 && b == b0 + 1) cluster_wait(); /* the first rows to be written */
         const int c1 = cl, cn = mlist ? chunks(Bn.nx * L::FA + Bn.ny * L::NC) : 0, cg = b > b0 ? chunks(Bp.nc * M) : 0;
         for (int c; (c = next(2 * b + 1)) < c1 + cn + cg;) {
             if (c < c1) chunk_b1(B, par, c);
@@ -565,12 +623,12 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
     }
     phase = staged;
     {
-        const StreamBand<M, R> B0(b0), B1(b1);
-        write_dry(2, B0.c0);
-        write_dry(B1.c0 + B1.nc, M + 2);
+        const Band B0(b0, o), B1(b1, o);
+        write_dry(o + 2, B0.c0);
+        write_dry(B1.c0 + B1.nc, o + RW + 2);
     }
 
-    if (wk.fl) {
+    if (K == 1 && wk.fl) {
         any_wet = __syncthreads_or(any_wet);
         if (threadIdx.x == 0) {
             wk.fl->ident = (!any_wet && !changed) ? 1 : 0;
@@ -590,7 +648,9 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         if (lane == 0) atomicMax(reinterpret_cast<unsigned long long*>(sc + SC_CFL), v);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (K > 1) { /* the cluster forms the patch CFL */
+        if (threadIdx.x == 0) *part = sc[SC_CFL];
+    } else if (threadIdx.x == 0) {
         double cfl = sc[SC_CFL];
         if (cfl > P.maxcfl_cap) cfl = 0.0;
         if (cfl_out) cfl_out[wi] = cfl;
@@ -619,6 +679,52 @@ __global__ void __launch_bounds__(NT, MINB)
         if (!stream_item<M, NT, R>(sm, bar, phase, work[wi], wi, phys_table, dt_uniform, group_dt, group_par, maux,
                                    cfl_out, group_max, err))
             return;
+}
+
+/* A patch over a cluster of K CTAs on K SMs: CTA r finishes the rows r M / K ..
+ * of the interior and solves the faces that these read, the ones at its edges
+ * once more than its neighbour does, so nothing but the speeds passes between
+ * the CTAs. The patch CFL is the largest of theirs, read by CTA 0 through
+ * distributed shared memory; the last barrier keeps every CTA until then. */
+template <int M, int NT, int R, int K, int MINB>
+__global__ void __cluster_dims__(K, 1, 1) __launch_bounds__(NT, MINB)
+    patch_update_window_kernel(const gf_patch_work* __restrict__ work, int nwork,
+                               const gf_phys* __restrict__ phys_table, double dt_uniform,
+                               const double* __restrict__ group_dt, const int* __restrict__ group_par,
+                               int maux, double* __restrict__ cfl_out,
+                               unsigned long long* __restrict__ group_max, int* __restrict__ err)
+{
+    static_assert(M % K == 0 && M / K + 4 <= 32, "rows split evenly, their flags in one word");
+    namespace cg = cooperative_groups;
+    using L = StreamSmem<M, R, K>;
+    extern __shared__ __align__(128) double sm[];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int r = (int)cluster.block_rank();
+    const int wi = blockIdx.x / K;
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::OFF_BAR);
+    double* part = sm + L::OFF_SC + SC_PART;
+    if (threadIdx.x == 0) {
+        mbar_init(bar, 1);
+        *part = 0.0;
+    }
+    __syncthreads();
+    /* these tests are the same on every CTA of the cluster: it leaves whole */
+    if (wi >= nwork) return;
+    const gf_patch_work wk = work[wi];
+    if (group_dt && !(group_dt[wk.group] > 0.0)) return;
+    if (wk.fl && wk.fl->skip) return;
+    uint32_t phase = 0;
+    stream_item<M, NT, R, K>(sm, bar, phase, wk, wi, phys_table, dt_uniform, group_dt, group_par, maux, cfl_out,
+                             group_max, err, r, part);
+    cluster.sync();
+    if (r == 0 && threadIdx.x == 0) {
+        double cfl = 0.0;
+        for (int q = 0; q < K; ++q) cfl = d_max_nn<true>(cfl, *cluster.map_shared_rank(part, q));
+        if (cfl > phys_table[wk.phys].maxcfl_cap) cfl = 0.0;
+        if (cfl_out) cfl_out[wi] = cfl;
+        if (group_max) atomicMax(group_max + wk.group, dkey(cfl));
+    }
+    cluster.sync();
 }
 
 /* Every patch size in one persistent launch, as patch_update_mixed_kernel,

@@ -208,35 +208,15 @@ __device__ __forceinline__ gf_cell load_cell(const double* sm, const unsigned ch
     return c;
 }
 
-/* The faces one sweep computes when a work item updates only the interior
- * rows rlo..rhi of its patch (the whole patch: rlo = 1, rhi = M). The x
- * sweep takes the slices (rows) rlo-1..rhi+1 with all their faces; the y
- * sweep takes every slice (column) with the normal-solve faces rlo-1..rhi+2
- * and the limited faces rlo..rhi+1, which are exactly the faces whose
- * records the update of rows rlo..rhi reads. Records of a band are packed
- * by the window's faces per slice (fa, fb), so a band holds rb slices
- * within the same shared-memory records as a whole-patch band of RB. For
- * rlo = 1, rhi = M every field is the whole-patch constant. */
-template <int M, int RB, int DIR>
+/* The faces one sweep computes. The x sweep takes the slices (rows) 0..M + 1,
+ * the y sweep the columns; records of a band are packed by the faces of a slice
+ * (fa, fb). */
+template <int M, int RB>
 struct SweepWin {
-    int ts_lo, nsl; /* slices ts_lo .. ts_lo + nsl - 1                  */
-    int na_lo, fa;  /* normal-solve faces na_lo .. na_lo + fa - 1        */
-    int nb_lo, fb;  /* limited faces nb_lo .. nb_lo + fb - 1             */
-    int rb;         /* slices per band                                   */
-    __device__ __forceinline__ SweepWin(int rlo, int rhi)
-    {
-        if (DIR == 0) {
-            ts_lo = rlo - 1; nsl = rhi - rlo + 3;
-            na_lo = 0; fa = M + 3;
-            nb_lo = 1; fb = M + 1;
-            rb = RB;
-        } else {
-            ts_lo = 0; nsl = M + 2;
-            na_lo = rlo - 1; fa = rhi - rlo + 4;
-            nb_lo = rlo; fb = rhi - rlo + 2;
-            rb = min(RB * (M + 3) / fa, RB * (M + 1) / fb);
-        }
-    }
+    static constexpr int ts_lo = 0, nsl = M + 2; /* slices ts_lo .. ts_lo + nsl - 1           */
+    static constexpr int na_lo = 0, fa = M + 3;  /* normal-solve faces na_lo .. na_lo + fa - 1 */
+    static constexpr int nb_lo = 1, fb = M + 1;  /* limited faces nb_lo .. nb_lo + fb - 1      */
+    static constexpr int rb = RB;                /* slices per band                            */
 };
 
 /* The full solve into a face record (contracted build). Not inlined: faces
@@ -270,8 +250,9 @@ struct SweepLists {
  * one atomic. */
 template <int M, int RB, int DIR>
 __device__ __forceinline__ void list_chunk(const double* sm, const unsigned char* wet, const SweepLists& ls, double g,
-                                           double crit, double crit2, const SweepWin<M, RB, DIR>& w, int band, int c)
+                                           double crit, double crit2, int band, int c)
 {
+    constexpr SweepWin<M, RB> w{};
     using L = Smem<M, RB, false>;
     constexpr int N = Geo<M>::N;
     const double* U = sm + (DIR == 0 ? L::OFF_U : L::OFF_V);
@@ -322,8 +303,9 @@ __device__ __forceinline__ void list_chunk(const double* sm, const unsigned char
  * list. Two passes (count, then place) over all faces. */
 template <int M, int NT, int RB, int DIR>
 __device__ __forceinline__ void build_lists_exact(const double* sm, const unsigned char* wet, int* cnt, uint16_t* la,
-                                                  uint16_t* lb, double g, const SweepWin<M, RB, DIR>& w)
+                                                  uint16_t* lb, double g)
 {
+    constexpr SweepWin<M, RB> w{};
     using G = Geo<M>;
     using L = Smem<M, RB, true>;
     constexpr int N = G::N;
@@ -494,7 +476,7 @@ __device__ __forceinline__ void cell_terms(const double* ol, const double* orr, 
  * made). */
 template <int M, int NT, int RB, int DIR, bool EXACT, class Side>
 __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, const SweepLists& ls, const gf_phys& P,
-                                        int rlo, int rhi, const Side& side)
+                                        const Side& side)
 {
     using G = Geo<M>;
     using L = Smem<M, RB, EXACT>;
@@ -526,13 +508,9 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
         return cnt[((band * 2 + list) * L::NCLS + cls) * 2 + 0];
     };
 
-    const SweepWin<M, RB, DIR> win(rlo, rhi);
-    const int fa = win.fa, fb = win.fb;
-    if constexpr (EXACT) build_lists_exact<M, NT, RB, DIR>(sm, wet, cnt, la, lb, g, win);
-    /* cells the gather writes: slice-direction t clamped to the window's rows
-     * in the x sweep, cell-direction n clamped to them in the y sweep */
-    const int gt_lo = DIR == 0 ? rlo : 1, gt_hi = DIR == 0 ? rhi : M;
-    const int gn_lo = DIR == 0 ? 1 : rlo, gn_hi = DIR == 0 ? M : rhi;
+    constexpr SweepWin<M, RB> win{};
+    constexpr int fa = win.fa, fb = win.fb;
+    if constexpr (EXACT) build_lists_exact<M, NT, RB, DIR>(sm, wet, cnt, la, lb, g);
     /* record of limited face `face` (nb_lo..) of band slice ts */
     auto orec = [&](int ts, int face) -> const double* {
         return O + (ts * fb + (face - win.nb_lo)) * L::O_STRIDE;
@@ -557,15 +535,15 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
     /* cells [e0, e0 + step, ..) of those the slices t0..t1 feed: n in [1, M],
      * t in [t0-1, t1+1] (interior), within the window */
     auto gather_cells = [&](int t0, int t1) -> int {
-        return (min(gt_hi, t1 + 1) - max(gt_lo, t0 - 1) + 1) * (gn_hi - gn_lo + 1);
+        return (min(M, t1 + 1) - max(1, t0 - 1) + 1) * M;
     };
     auto gather = [&](int t0, int t1, int e0, int e1, int step) {
-        const int ta = max(gt_lo, t0 - 1);
-        const int nn = gn_hi - gn_lo + 1;
+        const int ta = max(1, t0 - 1);
+        constexpr int nn = M;
         for (int e = e0; e < e1; e += step) {
             const int ts = e / nn;
             const int t = ta + ts;
-            const int n = gn_lo + (e - ts * nn);
+            const int n = 1 + (e - ts * nn);
             const int a = aidx(n, t);
             if (EXACT) {
                 if (t - 1 >= t0 && t - 1 <= t1) { /* slice below: up-going parts */
@@ -1010,8 +988,7 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
                                            double dt_uniform, const double* __restrict__ group_dt,
                                            const int* __restrict__ group_par, int maux,
                                            double* __restrict__ cfl_out,
-                                           unsigned long long* __restrict__ group_max, int* __restrict__ err,
-                                           int rlo = 1, int rhi = M, double* part = nullptr)
+                                           unsigned long long* __restrict__ group_max, int* __restrict__ err)
 {
     using G = Geo<M>;
     using L = Smem<M, RB, EXACT>;
@@ -1041,13 +1018,7 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
     /* after a wait of this launch (or an earlier one of the same step) gave
      * up, the step has failed: later items leave at once */
     const bool failed = __syncthreads_or(threadIdx.x == 0 && err && *reinterpret_cast<volatile int*>(err) != 0);
-    if (failed) {
-        if (part) {
-            cluster_arrive();
-            cluster_wait();
-        }
-        return false;
-    }
+    if (failed) return false;
 
     /* ---- stage the patch (h, hu, hv planes and b) with bulk copies ---- */
     if (threadIdx.x == 0) {
@@ -1061,11 +1032,6 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
     if (!staged) {
         if (threadIdx.x == 0) atomicExch(err, 1);
         mbar_wait(bar, ph, kWaitPolls); /* let any copy in flight land */
-    }
-    /* the CTAs of a split item update it in place: none writes before all have staged it */
-    if (part) cluster_arrive();
-    if (!staged) {
-        if (part) cluster_wait();
         return false;
     }
 
@@ -1088,7 +1054,6 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         }
         if (lane == 16) sc[SC_CFL] = 0.0;
     }
-    const int k_lo = (rlo - 1) * N, k_hi = (rhi + 4) * N;
     for (int k = threadIdx.x; k < S; k += NT) {
         double h = sm[L::OFF_H + k];
         if (d_lt<FAST>(h, drytol)) {
@@ -1103,7 +1068,6 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         const bool w = d_gt<FAST>(h, drytol);
         wet[k] = w ? 1 : 0;
         any_wet |= w;
-        if (k < k_lo || k >= k_hi) continue; /* rows that this window's faces do not read */
         double u = 0.0, v = 0.0, c = 0.0, rc = 0.0;
         if (w) {
             if (FAST) {
@@ -1142,8 +1106,8 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
                 __device__ void run(int, int) const {}
             } none;
             const SweepLists ls = {cnt, nullptr, lists, lists + L::LIST_A, nullptr};
-            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, ls, P, rlo, rhi, none);
-            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, ls, P, rlo, rhi, none);
+            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, ls, P, none);
+            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, ls, P, none);
         } else {
             /* The x sweep's first band is listed before it, every next band's
              * faces during the band before, and the y sweep's spread over all
@@ -1152,8 +1116,6 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
                 const double* sm;
                 const unsigned char* wet;
                 SweepLists x, y;
-                SweepWin<M, RB, 0> wx;
-                SweepWin<M, RB, 1> wy;
                 double g, crit, crit2;
                 int nbx, ncx, ncy, ny; /* x bands, chunks of a band of x and y, chunks of y */
                 __device__ __forceinline__ int xs(int p) const
@@ -1166,10 +1128,10 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
                 {
                     const int nx = xs(p);
                     if (c < nx) {
-                        list_chunk<M, RB, 0>(sm, wet, x, g, crit, crit2, wx, (p >> 1) + 1, (p & 1) ? ncx / 2 + c : c);
+                        list_chunk<M, RB, 0>(sm, wet, x, g, crit, crit2, (p >> 1) + 1, (p & 1) ? ncx / 2 + c : c);
                     } else {
                         const int e = y0(p) + c - nx, band = e / ncy;
-                        list_chunk<M, RB, 1>(sm, wet, y, g, crit, crit2, wy, band, e - band * ncy);
+                        list_chunk<M, RB, 1>(sm, wet, y, g, crit, crit2, band, e - band * ncy);
                     }
                 }
             };
@@ -1182,26 +1144,22 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
                 return {cnt + d * L::CNT_SWEEP, cnt + L::CNT_CUR + d * L::CUR_SWEEP, p, p + L::LIST_A,
                         p + L::LIST_A + L::LIST_B};
             };
-            const SweepWin<M, RB, 0> wx(rlo, rhi);
-            const SweepWin<M, RB, 1> wy(rlo, rhi);
-            Side side = {sm, wet, lists_of(0), lists_of(1), wx, wy, g, sc[SC_CRIT], sc[SC_CRIT2],
-                         (wx.nsl + wx.rb - 1) / wx.rb, (wx.rb * wx.fa + 31) / 32, (wy.rb * wy.fa + 31) / 32, 0};
-            side.ny = (wy.nsl + wy.rb - 1) / wy.rb * side.ncy;
+            constexpr int NBAND = (M + 2 + RB - 1) / RB, NCH = (RB * (M + 3) + 31) / 32;
+            Side side = {sm, wet, lists_of(0), lists_of(1), g, sc[SC_CRIT], sc[SC_CRIT2], NBAND, NCH, NCH, NBAND * NCH};
             for (int c = warp; c < side.ncx; c += NT / 32)
-                list_chunk<M, RB, 0>(sm, wet, side.x, g, side.crit, side.crit2, wx, 0, c);
+                list_chunk<M, RB, 0>(sm, wet, side.x, g, side.crit, side.crit2, 0, c);
             __syncthreads();
-            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, side.x, P, rlo, rhi, side);
-            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, side.y, P, rlo, rhi, None());
+            smax_x = sweep<M, NT, RB, 0, EXACT>(sm, wet, side.x, P, side);
+            smax_y = sweep<M, NT, RB, 1, EXACT>(sm, wet, side.y, P, None());
         }
     }
 
     /* ---- flux-difference update, src2, write interior ---- */
-    if (part) cluster_wait();
     double* gq = wk.qout ? wk.qout : wk.q;
     const double* gaux = wk.aux;
     const int fidx = P.friction_index - 1;
-    for (int e = threadIdx.x; e < (rhi - rlo + 1) * M; e += NT) {
-        const int i = 1 + e % M, j = rlo + e / M;
+    for (int e = threadIdx.x; e < M * M; e += NT) {
+        const int i = 1 + e % M, j = 1 + e / M;
         const int k = (j + 1) * N + (i + 1);
         double h = sm[L::OFF_H + k], hu = sm[L::OFF_HU + k], hv = sm[L::OFF_HV + k];
         constexpr int PL = L::PLANE;
@@ -1254,9 +1212,7 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
         if (lane == 0) atomicMax(reinterpret_cast<unsigned long long*>(sc + SC_CFL), v);
     }
     __syncthreads();
-    if (part) { /* a window of a split item: the cluster forms the patch CFL */
-        if (threadIdx.x == 0) *part = sc[SC_CFL];
-    } else if (threadIdx.x == 0) {
+    if (threadIdx.x == 0) {
         double cfl = sc[SC_CFL];
         if (cfl > P.maxcfl_cap) cfl = 0.0;
         if (cfl_out) cfl_out[wi] = cfl;
@@ -1289,57 +1245,6 @@ __global__ void __launch_bounds__(NT, MINB)
         if (!patch_item<M, NT, RB, EXACT>(sm, bar, phase, work[wi], wi, phys_table, dt_uniform, group_dt,
                                           group_par, maux, cfl_out, group_max, err))
             return;
-}
-
-/* Latency form: one patch split over a thread-block cluster of K CTAs on
- * K SMs. CTA r of a cluster updates interior rows r*M/K+1 .. (r+1)*M/K of
- * the cluster's work item; each stages the whole patch and computes exactly
- * the faces those rows read (SweepWin), so the interior values are the same
- * bits as the one-CTA kernel's (the same operations, summed per cell in the
- * same slice order). The patch CFL is the maximum of the CTAs' partial wave
- * speed maxima, read by rank 0 through distributed shared memory after a
- * cluster barrier; a second barrier keeps every CTA resident until it has
- * been read. A lone patch then runs on K SMs instead of one. */
-template <int M, int NT, int RB, int K, bool EXACT>
-__global__ void __cluster_dims__(K, 1, 1) __launch_bounds__(NT, 1)
-    patch_update_window_kernel(const gf_patch_work* __restrict__ work, int nwork,
-                               const gf_phys* __restrict__ phys_table, double dt_uniform,
-                               const double* __restrict__ group_dt, const int* __restrict__ group_par,
-                               int maux, double* __restrict__ cfl_out,
-                               unsigned long long* __restrict__ group_max, int* __restrict__ err)
-{
-    static_assert(M % K == 0, "the rows split evenly over the cluster");
-    namespace cg = cooperative_groups;
-    using L = Smem<M, RB, EXACT>;
-    constexpr int R = M / K;
-    extern __shared__ __align__(128) double sm[];
-    cg::cluster_group cluster = cg::this_cluster();
-    const int r = (int)cluster.block_rank();
-    const int wi = blockIdx.x / K;
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm + L::OFF_BAR);
-    double* part = sm + L::OFF_SC + SC_PART;
-    if (threadIdx.x == 0) {
-        mbar_init(bar, 1);
-        *part = 0.0;
-    }
-    __syncthreads();
-    /* both tests are the same on every CTA of the cluster: it leaves whole */
-    if (wi >= nwork) return;
-    const gf_patch_work wk = work[wi];
-    if (group_dt && !(group_dt[wk.group] > 0.0)) return;
-    if (wk.fl && wk.fl->skip) return;
-    uint32_t phase = 0;
-    patch_item<M, NT, RB, EXACT>(sm, bar, phase, wk, wi, phys_table, dt_uniform, group_dt, group_par,
-                                 maux, cfl_out, group_max, err, 1 + r * R, (r + 1) * R, part);
-    cluster.sync();
-    if (r == 0 && threadIdx.x == 0) {
-        double cfl = 0.0;
-        for (int q = 0; q < K; ++q) cfl = d_max_nn<true>(cfl, *cluster.map_shared_rank(part, q));
-        if (cfl > phys_table[wk.phys].maxcfl_cap) cfl = 0.0;
-        if (cfl_out) cfl_out[wi] = cfl;
-        if (group_max) atomicMax(group_max + wk.group, dkey(cfl));
-    }
-    cluster.sync();
 }
 
 /* Shared-memory bytes of the mixed kernel: the largest class layout, then

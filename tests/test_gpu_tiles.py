@@ -70,6 +70,61 @@ def test_tile_by_the_number_of_patches_gives_the_same_bits(ctx, m, npx):
     assert np.array_equal(auto[0], one[0]) and auto[2] == one[2] and np.array_equal(auto[4], one[4])
 
 
+@pytest.mark.parametrize("m,npx", [(8, 38), (8, 39), (16, 304), (16, 305), (32, 266), (32, 267), (32, 304), (32, 305)])
+def test_tile_switches_of_wider_launches_give_the_same_bits(ctx, m, npx):
+    """Either side of the remaining switches: the bits of one fixed tile."""
+    keep, other = gf.Context.tile(m, 0), 2 if m == 16 else 0
+    assert keep != other
+    q, aux, _, _ = synth.uniform_dam_break_level(npx, 1, m, 1.0, seed=npx, x_dam=0.4 * m * npx)
+    ctx.set_phys(0, gf.Phys())
+    outs = []
+    try:
+        for v in (keep, other):
+            gf.Context.set_tile(m, 0, v)
+            lev = gf.Level(ctx, npx, m, 1)
+            lev.set_geometry(1.0, 1.0)
+            lev.upload(q, aux)
+            cfl = lev.step(0.0, 0.05)
+            outs.append((lev.download(), cfl, lev.patch_cfl()))
+            lev.close()
+    finally:
+        gf.Context.set_tile(m, 0, keep)
+    assert np.array_equal(outs[0][0], outs[1][0]) and outs[0][1] == outs[1][1]
+    assert np.array_equal(outs[0][2], outs[1][2])
+
+
+@pytest.mark.parametrize("m", [8, 16, 32])
+@pytest.mark.parametrize("kind", ["band", "row", "thin"])
+def test_dry_rows_and_windows(ctx, m, kind):
+    """Water in some rows only (a band of rows at every height, a single row at
+    every place from ghost to ghost, depths below the tolerance with momentum):
+    rows that a tile passes over, or windows of a split patch without water,
+    come out as the oracle's, and as the same bits from every tile."""
+    n = m + 4
+    q, aux = random_state(n, m, 60 + m)
+    for k in range(n):
+        lo, hi = (k, min(k + 1, n)) if kind == "row" else (k // 2, min(k // 2 + 1 + k % 7, n))
+        if kind == "thin":
+            q[k, :lo, :, 0] = np.minimum(q[k, :lo, :, 0], 5e-4)
+            q[k, hi:, :, 0] = np.minimum(q[k, hi:, :, 0], 1e-3)
+        else:
+            q[k, :lo] = 0.0
+            q[k, hi:] = 0.0
+    keep = gf.Context.tile(m, 0)
+    outs = []
+    try:
+        for v in variants(m):
+            gf.Context.set_tile(m, 0, v)
+            out, ref, cg, cr, pg, pr = level_vs_oracle(ctx, q, aux, m, 2.0, 0.02, gf.Phys())
+            compare(q, out, ref, cg, cr, m, pcfl_gpu=pg, pcfl_ref=pr)
+            outs.append((out, cg, pg))
+    finally:
+        gf.Context.set_tile(m, 0, keep)
+    for out, cg, pg in outs[1:]:
+        assert np.array_equal(out, outs[0][0]) and cg == outs[0][1]
+        assert np.array_equal(pg, outs[0][2])
+
+
 def test_autotune_measures_and_selects(ctx):
     ctx.set_phys(0, gf.Phys())
     res = ctx.autotune(reps=2)
