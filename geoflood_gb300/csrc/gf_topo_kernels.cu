@@ -2,7 +2,7 @@
  * Cell-averaged topography on the device: setaux's bathymetry for every
  * cell of a raster (a level of a forest, or any uniform grid).
  *
- * One thread per cell. The cell's integral follows cellgridintegrate
+ * The cell's integral follows cellgridintegrate
  * (src/fc2d_geoclaw/geolib_source/cellgridintegrate2.f:1-90): the finest
  * grid overlapping the cell alone if it holds the whole cell, else the
  * inclusion-exclusion over the ranked grids of rectintegral
@@ -153,172 +153,188 @@ __device__ bool cell_integral(const Rect& cell, const gf_topo_grid* grids, const
     return false;
 }
 
-/* Tile of raster cells of a CTA, and the most node cells of a column (row) of
- * cells that its tables hold: coarser cells take the general path. */
-constexpr int kTX = 32, kTY = 8, kNodes = 40;
+/* Tile of raster cells of a CTA of kTX x kTY threads (kRows rows of cells, some
+ * for each thread), and the most node cells of a column (row) of cells that its
+ * tables hold: coarser cells take the general path. */
+constexpr int kTX = 32, kTY = 8, kRows = 32, kPer = kRows / kTY, kNodes = 40;
+static_assert(kRows == kTX, "one warp per axis");
 
 /* One axis of the integral of a column (row) of cells [lo, hi] over a grid:
  * the node cells i0 .. i1 - 1 it touches, and for each the width of the
- * overlap and the sum of its two ends in units of the spacing, as
- * grid_integral forms them. */
+ * overlap and half the sum of its two ends in units of the spacing. */
 struct AxisNode {
-    double width, sum;
+    double width, half;
 };
-__device__ __forceinline__ void axis_range(double& lo, double& hi, double low, double d, int n, int* i0, int* i1)
+struct AxisCell {
+    double lo, hi;   /* the cell's sides                          */
+    double clo, chi; /* clamped to the grid                       */
+    int i0, i1;      /* its node cells                            */
+    int meets;       /* bit 0: overlaps the grid, bit 1: inside it */
+};
+__device__ __forceinline__ void axis_range(AxisCell& A, double low, double d, int n)
 {
     const double top = low + (n - 1) * d;
+    double lo = A.lo, hi = A.hi;
     if ((lo - low) < 0.0 || (hi - top) > 0.0) {
         lo = fmax(low, lo);
         hi = fmin(top, hi);
     }
-    *i0 = max((int)((lo - low) / d) + 1, 1);
-    *i1 = min((int)ceil((hi - low) / d) + 1, n);
+    A.clo = lo;
+    A.chi = hi;
+    A.i0 = max((int)((lo - low) / d) + 1, 1);
+    A.i1 = min((int)ceil((hi - low) / d) + 1, n);
 }
 __device__ __forceinline__ AxisNode axis_node(double lo, double hi, double low, double d, int ii)
 {
     const double x1 = low + (ii - 1.0) * d, x2 = low + ii * d;
     const double a = fmax(lo, x1), b = fmin(hi, x2);
-    return {b - a, (b + a - 2.0 * x1) / d};
+    return {b - a, 0.5 * ((b + a - 2.0 * x1) / d)};
 }
 
-/* One thread per cell. The kernel is bound by FP64 issue (two lanes a clock),
- * and most of it went into quotients that depend on the cell's column or row
- * alone: a tile now forms them once per column and row of cells, in shared
- * memory, for the cells that lie whole in the finest grid they touch (the
- * same operations in the same order, so the same bits); the others (cells that
- * a grid's edge cuts, cells over more node cells than the tables hold) take
- * cell_integral. */
+/* v / area, correctly rounded, from the rounded reciprocal of area (Markstein,
+ * "Computation of elementary functions on the IBM RISC System/6000 processor",
+ * 1990): the first step makes the quotient faithful, the second exact. Five FP64
+ * operations; the general quotient takes about twice as many. Out of the range
+ * where no step can over- or underflow, or without a reciprocal (0): the
+ * quotient itself. */
+__device__ __forceinline__ double over_area(double v, double area, double rarea)
+{
+    const unsigned e = (unsigned)(__double_as_longlong(v) >> 52) & 0x7ff;
+    if (e - 512u > 1024u || rarea == 0.0) return v / area;
+    double q = v * rarea;
+    q = fma(fma(-area, q, v), rarea, q);
+    return fma(fma(-area, q, v), rarea, q);
+}
+
+/* The kernel is bound by FP64 issue (two lanes a clock), and most of it would go
+ * into tests and quotients that depend on a cell's column or row alone. A tile of
+ * 32 x 32 cells forms them once per column and row, one warp an axis, in shared
+ * memory, for the cells that lie whole in the finest grid they touch; what is
+ * left for a cell are the 14 operations of each node cell under it and the last
+ * quotient. Halves of the axis sums stand for the factors 1/2 and 1/4 of the
+ * bilinear form (powers of two, which no rounding sees), and the difference of a
+ * node column serves both cells beside it: the same bits. The other cells (cells
+ * that a grid's edge cuts, cells over more node cells than the tables hold) are
+ * gathered, so that the column under an edge fills one warp, and take
+ * cell_integral. 1535^2 cells over a 1025^2 grid with a 513^2 inset, ncu: 625 us
+ * with a warp for each row of them, 422 us gathered (82 % FP64 pipe, 89 FP64
+ * instructions for 32 cells). Cells outside the domain are cells inside to this
+ * kernel (a pass of its own over the raster took 31 us). */
 __global__ void __launch_bounds__(kTX* kTY)
     topo_raster_kernel(const gf_topo_grid* __restrict__ grids, const int* __restrict__ order, int n, int nx, int ny,
                        int halo, double xlower, double ylower, double dx, double dy, double xupper, double yupper,
-                       double* __restrict__ out, int* __restrict__ err)
+                       double area, double rarea, double* __restrict__ out, int* __restrict__ err)
 {
-    __shared__ AxisNode xt[kNodes][kTX], yt[kTY][kNodes];
-    __shared__ double cx[kTX][2], cy[kTY][2];
-    __shared__ int xr[kTX][2], yr[kTY][2];
-    __shared__ unsigned char outx[kTX], outy[kTY];
-    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * kTX + tx;
+    __shared__ AxisNode xt[kNodes][kTX], yt[kNodes][kRows];
+    __shared__ AxisCell ax[kTX], ay[kRows];
+    __shared__ unsigned short rest[kTX * kRows]; /* cells of the general path */
+    __shared__ int nrest;
+    const int tx = threadIdx.x, ty = threadIdx.y;
     const long p = nx + 2 * halo;
     const int tiles = (int)((p + kTX - 1) / kTX), by = blockIdx.x / tiles, bx = blockIdx.x - by * tiles;
-    const int i = bx * kTX + tx, j = by * kTY + ty;
-    if (t < kTX) {
-        const int gi = i - halo;
-        const double x1 = xlower + (double)gi * dx, x2 = xlower + (double)(gi + 1) * dx, x = 0.5 * (x1 + x2);
-        cx[tx][0] = x1;
-        cx[tx][1] = x2;
-        outx[tx] = x > xupper || x < xlower;
-    } else if (t < kTX + kTY) {
-        const int k = t - kTX, gj = by * kTY + k - halo;
-        const double y1 = ylower + (double)gj * dy, y2 = ylower + (double)(gj + 1) * dy, y = 0.5 * (y1 + y2);
-        cy[k][0] = y1;
-        cy[k][1] = y2;
-        outy[k] = y > yupper || y < ylower;
+    const int i = bx * kTX + tx, jb = by * kRows;
+    if (ty == 2 && tx == 0) nrest = 0;
+    if (ty < 2) { /* warp 0 the columns, warp 1 the rows */
+        int g = (ty ? jb + tx : i) - halo;
+        const double low = ty ? ylower : xlower, d = ty ? dy : dx, up = ty ? yupper : xupper;
+        /* a cell outside the domain takes the cell inside that setaux's index
+         * shift names: i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)) */
+        const double x = low + (g + 0.5) * d;
+        if (x < low || x > up) g += (int)fmax(0.0, ceil((low - x) / d)) - (int)fmax(0.0, ceil((x - up) / d));
+        AxisCell& A = ty ? ay[tx] : ax[tx];
+        A.lo = low + (double)g * d;
+        A.hi = low + (double)(g + 1) * d;
     }
     __syncthreads();
-    const Rect cell = {cx[tx][0], cx[tx][1], cy[ty][0], cy[ty][1]};
-    const bool live = i < p && j < ny + 2 * halo && !outx[tx] && !outy[ty];
-    /* 0 no grid yet, 1 done, 2 general path */
-    int state = live ? 0 : 1;
-    double v = 0.0;
+    /* of this thread's cells, bit q for row ty + q kTY: still without a grid, to
+     * take the general path */
+    unsigned open = 0, general = 0, live;
+    for (int q = 0; q < kPer; ++q) {
+        const int k = ty + q * kTY;
+        if (i < p && jb + k < ny + 2 * halo) open |= 1u << q;
+    }
+    live = open;
+    double v[kPer] = {};
     for (int m = 0; m < n; ++m) {
         const gf_topo_grid& G = grids[order[m]];
-        const bool meets = state == 0 && fmin(cell.x2, G.xhi) > fmax(cell.x1, G.xlow) &&
-                           fmin(cell.y2, G.yhi) > fmax(cell.y1, G.ylow);
-        const bool whole = meets && cell.x1 >= G.xlow && cell.x2 <= G.xhi && cell.y1 >= G.ylow && cell.y2 <= G.yhi;
-        if (meets && !whole) state = 2;
-        if (!__syncthreads_or(whole)) {
-            if (!__syncthreads_or(state == 0)) break;
-            continue;
-        }
-        if (t < kTX) {
-            double lo = cx[tx][0], hi = cx[tx][1];
-            axis_range(lo, hi, G.xlow, G.dx, G.mx, &xr[tx][0], &xr[tx][1]);
-        } else if (t < kTX + kTY) {
-            const int k = t - kTX;
-            double lo = cy[k][0], hi = cy[k][1];
-            axis_range(lo, hi, G.ylow, G.dy, G.my, &yr[k][0], &yr[k][1]);
+        if (ty < 2) {
+            AxisCell& A = ty ? ay[tx] : ax[tx];
+            const double low = ty ? G.ylow : G.xlow, high = ty ? G.yhi : G.xhi;
+            A.meets = (fmin(A.hi, high) > fmax(A.lo, low) ? 1 : 0) | (A.lo >= low && A.hi <= high ? 2 : 0);
         }
         __syncthreads();
-        {
-            double lo = cx[tx][0], hi = cx[tx][1];
-            const double top = G.xlow + (G.mx - 1) * G.dx;
-            if ((lo - G.xlow) < 0.0 || (hi - top) > 0.0) {
-                lo = fmax(G.xlow, lo);
-                hi = fmin(top, hi);
+        unsigned whole = 0;
+        for (int q = 0; q < kPer; ++q) {
+            const int both = ax[tx].meets & ay[ty + q * kTY].meets;
+            if ((both & 1) && (open >> q & 1)) {
+                open &= ~(1u << q);
+                if (both & 2) whole |= 1u << q;
+                else general |= 1u << q;
             }
-            const int i0 = xr[tx][0], c = min(xr[tx][1] - i0, kNodes);
-            for (int e = ty; e < c; e += kTY) xt[e][tx] = axis_node(lo, hi, G.xlow, G.dx, i0 + e);
         }
-        {
-            double lo = cy[ty][0], hi = cy[ty][1];
-            const double top = G.ylow + (G.my - 1) * G.dy;
-            if ((lo - G.ylow) < 0.0 || (hi - top) > 0.0) {
-                lo = fmax(G.ylow, lo);
-                hi = fmin(top, hi);
+        if (__syncthreads_or(whole != 0)) {
+            if (ty == 0) axis_range(ax[tx], G.xlow, G.dx, G.mx);
+            else if (ty == 1) axis_range(ay[tx], G.ylow, G.dy, G.my);
+            __syncthreads();
+            {
+                const AxisCell& A = ax[tx];
+                const int c = min(A.i1 - A.i0, kNodes);
+                for (int e = ty; e < c; e += kTY) xt[e][tx] = axis_node(A.clo, A.chi, G.xlow, G.dx, A.i0 + e);
             }
-            const int j0 = yr[ty][0], c = min(yr[ty][1] - j0, kNodes);
-            for (int e = tx; e < c; e += kTX) yt[ty][e] = axis_node(lo, hi, G.ylow, G.dy, j0 + e);
-        }
-        __syncthreads();
-        if (whole) {
-            const int i0 = xr[tx][0], nc = xr[tx][1] - i0, j0 = yr[ty][0], nr = yr[ty][1] - j0;
-            if (nc > kNodes || nr > kNodes) {
-                state = 2;
-            } else {
+            {
+                const AxisCell& A = ay[tx];
+                const int c = min(A.i1 - A.i0, kNodes);
+                for (int e = kTY - 1 - ty; e < c; e += kTY) yt[e][tx] = axis_node(A.clo, A.chi, G.ylow, G.dy, A.i0 + e);
+            }
+            __syncthreads();
+            const int i0 = ax[tx].i0, nc = ax[tx].i1 - i0;
+#pragma unroll
+            for (int q = 0; q < kPer; ++q) {
+                if (!(whole >> q & 1)) continue;
+                const int k = ty + q * kTY, j0 = ay[k].i0, nr = ay[k].i1 - j0;
+                if (nc > kNodes || nr > kNodes) {
+                    general |= 1u << q;
+                    continue;
+                }
                 double s = 0.0;
                 for (int r = 0; r < nr; ++r) {
                     /* nodes are stored north to south: row (my - jj) holds the lower ones */
                     const double* row1 = G.z + (long)(G.my - (j0 + r)) * G.mx + (i0 - 1);
                     const double* row2 = row1 - G.mx;
-                    const AxisNode Y = yt[ty][r];
+                    const AxisNode Y = yt[r][k];
                     double z11 = nc > 0 ? row1[0] : 0.0, z12 = nc > 0 ? row2[0] : 0.0;
+                    double b = z12 - z11;
                     for (int c = 0; c < nc; ++c) {
                         const AxisNode X = xt[c][tx];
                         const double z21 = row1[c + 1], z22 = row2[c + 1];
                         const double area = Y.width * X.width;
-                        const double a = z21 - z11, b = z12 - z11, d = z22 - z21 - z12 + z11;
-                        s = s + (0.5 * (a * X.sum + b * Y.sum) + 0.25 * d * X.sum * Y.sum + z11) * area;
+                        const double a = z21 - z11, bn = z22 - z21, d = bn - z12 + z11;
+                        s = s + ((a * X.half + b * Y.half) + d * X.half * Y.half + z11) * area;
                         z11 = z21;
                         z12 = z22;
+                        b = bn;
                     }
                 }
-                v = 0.0 + s;
-                state = 1;
+                v[q] = 0.0 + s;
             }
         }
-        if (!__syncthreads_or(state == 0)) break;
+        if (!__syncthreads_or(open != 0)) break;
     }
-    if (!live) return;
-    if (state == 2) cell_integral(cell, grids, order, n, &v);
-    if (state == 0) *err = 1; /* no grid under the cell */
-    out[(long)j * p + i] = v / (dx * dy);
-}
-
-/* cells outside the domain take the cell inside that setaux's index shift
- * names: i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)). A
- * column's and a row's part of the test are formed once per tile. */
-__global__ void __launch_bounds__(kTX* kTY)
-    topo_outside_kernel(double* __restrict__ out, int nx, int ny, int halo, double xlower, double ylower, double dx,
-                        double dy, double xupper, double yupper)
-{
-    __shared__ unsigned char outx[kTX], outy[kTY];
-    const int tx = threadIdx.x, ty = threadIdx.y, t = ty * kTX + tx;
-    const long p = nx + 2 * halo;
-    const int tiles = (int)((p + kTX - 1) / kTX), by = blockIdx.x / tiles, bx = blockIdx.x - by * tiles;
-    const int i = bx * kTX + tx, j0 = by * kTY, j = j0 + ty;
-    if (t < kTX) {
-        const double x = xlower + ((i - halo) + 0.5) * dx;
-        outx[tx] = x < xlower || x > xupper;
-    } else if (t < kTX + kTY) {
-        const double y = ylower + ((j0 + (t - kTX) - halo) + 0.5) * dy;
-        outy[t - kTX] = y < ylower || y > yupper;
+    if (open) *err = 1; /* no grid under a cell */
+#pragma unroll
+    for (int q = 0; q < kPer; ++q) {
+        const int k = ty + q * kTY;
+        if (general >> q & 1) rest[atomicAdd(&nrest, 1)] = (unsigned short)(k * kTX + tx);
+        else if (live >> q & 1) out[(long)(jb + k) * p + i] = over_area(v[q], area, rarea);
     }
     __syncthreads();
-    if (i >= p || j >= ny + 2 * halo || !(outx[tx] || outy[ty])) return;
-    const double x = xlower + ((i - halo) + 0.5) * dx, y = ylower + ((j - halo) + 0.5) * dy;
-    const int ii = i + (int)fmax(0.0, ceil((xlower - x) / dx)) - (int)fmax(0.0, ceil((x - xupper) / dx));
-    const int jj = j + (int)fmax(0.0, ceil((ylower - y) / dy)) - (int)fmax(0.0, ceil((y - yupper) / dy));
-    out[(long)j * p + i] = out[(long)jj * p + ii];
+    for (int e = ty * kTX + tx; e < nrest; e += kTX * kTY) {
+        const int k = rest[e] / kTX, c = rest[e] % kTX;
+        const Rect cell = {ax[c].lo, ax[c].hi, ay[k].lo, ay[k].hi};
+        double w = 0.0;
+        cell_integral(cell, grids, order, n, &w);
+        out[(long)(jb + k) * p + bx * kTX + c] = over_area(w, area, rarea);
+    }
 }
 
 } // namespace
@@ -328,14 +344,14 @@ cudaError_t launch_topo_raster(const gf_topo_grid* grids, const int* order, int 
                                double yupper, double* out, int* err, cudaStream_t st)
 {
     if (n < 1 || n > GF_TOPO_MAX_FILES) return cudaErrorInvalidValue;
-    const long tiles = (long)((nx + 2 * halo + kTX - 1) / kTX) * ((ny + 2 * halo + kTY - 1) / kTY);
-    if (tiles > 0x7fffffffL) return cudaErrorInvalidValue; /* 5e11 cells */
-    const dim3 block(kTX, kTY), grid((unsigned)tiles);
-    topo_raster_kernel<<<grid, block, 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper,
-                                               out, err);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess || halo == 0) return e;
-    topo_outside_kernel<<<grid, block, 0, st>>>(out, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper);
+    const long cols = (nx + 2 * halo + kTX - 1) / kTX;
+    const long tiles = cols * ((ny + 2 * halo + kRows - 1) / kRows);
+    if (tiles > 0x7fffffffL) return cudaErrorInvalidValue; /* 2e12 cells */
+    const dim3 block(kTX, kTY);
+    const double area = dx * dy;
+    const double rarea = area > 0x1p-500 && area < 0x1p500 ? 1.0 / area : 0.0;
+    topo_raster_kernel<<<(unsigned)tiles, block, 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy,
+                                                          xupper, yupper, area, rarea, out, err);
     return cudaGetLastError();
 }
 

@@ -53,6 +53,23 @@ def test_raster_tiles_match_oracle(ctx, nx, ny):
     assert np.array_equal(got, ts.raster(nx, ny, 2, 0.0, 0.0, dx, dy, 900.0, 1000.0))
 
 
+@pytest.mark.parametrize("nx,ny,halo,short", [(28, 27, 2, 0.0), (27, 28, 2, 0.0), (29, 29, 2, 0.0), (62, 61, 1, 0.0),
+                                              (95, 97, 8, 0.0), (40, 70, 2, 2.6), (70, 40, 1, 5.0)])
+def test_raster_tile_rows_and_cells_outside_match_oracle(ctx, nx, ny, halo, short):
+    """Tiles of 32 rows at their edges, columns and rows that an inset's edges
+    cut (gathered into full warps), and a domain that ends `short` cells inside
+    the raster (its outer cells take the nearest cell inside): bit for bit."""
+    g = np.random.default_rng(nx * 1000 + ny)
+    t = Topo()
+    t.add_grid(g.uniform(0.0, 40.0, (101, 91)), 0.0, 0.0, 10.0, 10.0)
+    t.add_grid(g.uniform(0.0, 40.0, (67, 81)), 203.7, 301.1, 3.3, 3.3)
+    ts = ot.TopoSet([t.grid(k) for k in range(len(t))])
+    dx, dy = 900.0 / nx, 1000.0 / ny
+    xu, yu = 900.0 - short * dx, 1000.0 - short * dy
+    got = t.raster(ctx, nx, ny, halo, 0.0, 0.0, dx, dy, xu, yu)
+    assert np.array_equal(got, ts.raster(nx, ny, halo, 0.0, 0.0, dx, dy, xu, yu))
+
+
 def test_uncovered_cell_is_an_error(ctx):
     t, _ = sets()
     with pytest.raises(gf.GeoFloodError):
