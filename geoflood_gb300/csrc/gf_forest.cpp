@@ -2338,7 +2338,10 @@ int batch_launch(BatchRun& R, int* live_out)
     }
     const int ng = (int)B.fs.size();
     int rounds = (int)std::ceil(0.5 / std::max(R.round_ms, 1e-3));
-    rounds = std::max(1, std::min(64, rounds));
+    int left = 1; /* rounds past the members' next stops would run empty */
+    for (const gf_forest* f : B.fs)
+        if (!f->gst.paused) left = std::max(left, gf::rounds_left(f->gst, 64));
+    rounds = std::max(1, std::min(left, rounds));
     R.t_launch = clk::now();
     const cudaStream_t cst = gf::ctx_stream(B.ctx);
     if (B.st != cst) {

@@ -101,6 +101,23 @@ cudaError_t launch_batch_out(const double* q, double* hq, long npatch, int ncell
                              const unsigned long long* gmax, const int* err, unsigned long long* hgmax, int* herr,
                              cudaStream_t st);
 
+/* Rounds that a scenario still takes part in, at its present time step: its
+ * steps, the round after the last that ends it, no further than the round that
+ * stops it for a regrid. An estimate for the number of rounds to launch ahead
+ * (the time step changes on the way); max at most. */
+inline int rounds_left(const gf_group_state& s, int max)
+{
+    if (!s.active) return 0;
+    const int intervals = s.nout - 1 - s.nint;
+    const double dt = s.dt_minlevel / s.level_factor;
+    const double n = (s.tend + intervals * s.dt_outer - s.t_curr) / dt + intervals;
+    int left = n < max ? (n > 0.0 ? (int)n + 2 : 1) : max; /* NaN: max */
+    if (s.regrid_interval > 0 && s.regrid_interval - s.since_regrid + 1 < left)
+        left = s.regrid_interval - s.since_regrid + 1;
+    return left < 1 ? 1 : left > max ? max : left;
+}
+
+
 /* Served scenarios: device-side time-step control around a round. */
 cudaError_t launch_served_prepare(gf_group_state* gs, gf_ghost_block* blocks, double* gdt, int* gpar,
                                   unsigned long long* gmax, const double* hy_t,

@@ -638,6 +638,16 @@ int capture_round(gf_server* srv, Lane& L)
     return GF_OK;
 }
 
+/* Rounds the lane's members still need beyond those in flight (an estimate):
+ * a round past the last member's end runs empty, about 15 us each. */
+int lane_rounds_left(const Lane& L)
+{
+    int left = 0;
+    for (const Scen* s : L.members) left = std::max(left, gf::rounds_left(s->gst, kMaxRounds));
+    for (const Chunk& c : L.inflight) left -= c.rounds;
+    return left;
+}
+
 /* Enqueue a chunk of rounds (epoch unchanged) and the controllers' readback. */
 int launch_chunk(gf_server* srv, Lane& L)
 {
@@ -646,7 +656,7 @@ int launch_chunk(gf_server* srv, Lane& L)
     const gf_group_state* gs = reinterpret_cast<const gf_group_state*>(d + L.off_gs);
     const unsigned long long* rb = reinterpret_cast<const unsigned long long*>(d + L.off_rb);
     int rounds = (int)std::ceil(kChunkTargetMs / std::max(L.round_ms, 1e-3));
-    rounds = std::max(1, std::min(kMaxRounds, rounds));
+    rounds = std::max(1, std::min(lane_rounds_left(L), rounds));
     const int slot = L.next_slot;
     L.next_slot ^= 1;
     SV_CK(srv, cudaEventRecord(L.ev_start[slot], L.st));
@@ -724,7 +734,7 @@ int pump_locked(gf_server* srv, int* busy)
             if (rc) return rc;
         }
         if (L.members.empty()) continue;
-        while (L.inflight.size() < 2) {
+        while (L.inflight.size() < 2 && (L.inflight.empty() || lane_rounds_left(L) > 0)) {
             rc = launch_chunk(srv, L);
             if (rc) return rc;
         }
