@@ -40,15 +40,14 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "cell-updates/s"
 BYTES_PER_CELL_UPDATE = 56  # read h, hu, hv, b; write h, hu, hv (FP64)
-# Per tile shape of the mx = 32 update (threads, slices per band), from one ncu
-# capture each of the launch this bench times first in its kernel-only loop
-# (update launch 24 of `--steps 20 --warmup 3`, the same state): DRAM
-# traffic (dram__bytes_read.sum + dram__bytes_write.sum, against 234.9 MB
-# algorithmic) and FP64 warp instructions (sm__inst_executed_pipe_fp64.sum;
+# Per tile shape of the mx = 32 update (threads, rows per band), from one ncu
+# capture of the launch this bench times first in its kernel-only loop (update
+# launch 24 of `--steps 20 --warmup 3`, the same state): DRAM traffic
+# (dram__bytes_read.sum + dram__bytes_write.sum; below the 234.9 MB algorithmic,
+# since rows without water are read for their depth alone) and FP64 warp instructions (sm__inst_executed_pipe_fp64.sum;
 # x 32 lanes / 4 194 304 cell-updates = FP64 issue slots per cell-update)
-NCU_COUNTS = {(256, 7): (170.886912e6 + 62.938880e6, 29.892596e6),
-              (384, 9): (170.445312e6 + 66.367744e6, 29.903210e6)}
-NCU_DEFAULT_TILE = (384, 9)
+NCU_COUNTS = {(256, 4): (90.650368e6 + 89.671680e6, 18.152225e6)}
+NCU_DEFAULT_TILE = (256, 4)
 M = 32
 NPX = NPY = 64
 DX = 1.0
@@ -695,7 +694,7 @@ def run_gpu(args):
     lone_us = lone_patch_latency_us(ctx, q, aux)
 
     hbm_peak, peak_kind = load_peaks()
-    tile32 = (384, 9)
+    tile32 = NCU_DEFAULT_TILE  # what a launch of this many patches takes by itself
     tsel = next((t for t in (tiles or []) if t["mx"] == M), None)
     if tsel is not None:
         tile32 = tuple(tsel["tiles"][tsel["best_throughput"]][:2])
@@ -703,7 +702,7 @@ def run_gpu(args):
         for spec in filter(None, args.tiles.split(",")):
             mx_s, thr, _ = (int(v) for v in spec.split(":"))
             if mx_s == M:
-                tile32 = {0: (256, 7), 1: (256, 5), 2: (384, 7), 3: (384, 9)}.get(thr, tile32)
+                tile32 = {0: (256, 7), 1: (256, 4), 2: (384, 7), 3: (384, 9)}.get(thr, tile32)
     traffic, fp64_warp_inst = NCU_COUNTS.get(tile32, NCU_COUNTS[NCU_DEFAULT_TILE])
     algo = BYTES_PER_CELL_UPDATE * ncell
     achieved = algo / (kernel_ms * 1e-3) / 1e9
@@ -1405,7 +1404,7 @@ def main():
     ap.add_argument("--no-autotune", action="store_true")
     ap.add_argument("--tiles", default="",
                     help="pin tile variants instead of autotuning: mx:throughput:latency,... "
-                         "(e.g. 32:3:7)")
+                         "(e.g. 32:1:5)")
     ap.add_argument("--large-only", action="store_true")
     ap.add_argument("--large-steps", type=int, default=24)
     ap.add_argument("--no-dem", action="store_true")

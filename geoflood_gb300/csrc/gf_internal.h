@@ -164,10 +164,10 @@ cudaError_t launch_pyramid_down(const double* fine, double* coarse, int nxc, int
 cudaError_t launch_patch_fill(int m, const gf_fill_task* tasks, int ntask, cudaStream_t st);
 /* cell averages of topo grids over a raster (interior cells inside the
  * domain, then the cells outside copy the nearest inside); *err = 1 when a
- * cell overlaps no grid */
+ * cell overlaps no grid; finest: the smallest spacing of the grids */
 cudaError_t launch_topo_raster(const gf_topo_grid* grids, const int* order, int n, int nx, int ny,
                                int halo, double xlower, double ylower, double dx, double dy,
-                               double xupper, double yupper, double* out, int* err,
+                               double xupper, double yupper, double finest, double* out, int* err,
                                cudaStream_t st);
 int topo_raster_device(gf_ctx* c, gf_topo* t, int nx, int ny, int halo, double xlower,
                        double ylower, double dx, double dy, double xupper, double yupper,

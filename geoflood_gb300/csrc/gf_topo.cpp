@@ -588,12 +588,14 @@ int topo_raster_device(gf_ctx* c, gf_topo* t, int nx, int ny, int halo, double x
     int rc = topo_device(t, ctx_device(c), st, &grid, &order, &n);
     if (rc == GF_ERR_STATE) return ctx_fail(c, rc, "the topo set has no grids");
     if (rc) return ctx_fail(c, rc, "topo upload failed");
+    double finest = t->grids[0].dx;
+    for (const TopoGrid& g : t->grids) finest = std::min(finest, std::min(g.dx, g.dy));
     int* d_err = nullptr;
     cudaError_t e = cudaMallocAsync(&d_err, sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(d_err, 0, sizeof(int), st);
     if (e == cudaSuccess)
-        e = launch_topo_raster(grid, order, n, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper, out, d_err,
-                               st);
+        e = launch_topo_raster(grid, order, n, nx, ny, halo, xlower, ylower, dx, dy, xupper, yupper, finest, out,
+                               d_err, st);
     int h_err = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -135,8 +135,8 @@ __device__ double ranked_integral(Rect r0, int m0, const gf_topo_grid* grids, co
     return ret;
 }
 
-__device__ bool cell_integral(const Rect& cell, const gf_topo_grid* grids, const int* order, int n,
-                              double* out)
+__device__ __forceinline__ bool cell_integral_inline(const Rect& cell, const gf_topo_grid* grids, const int* order,
+                                                     int n, double* out)
 {
     for (int m = 0; m < n; ++m) {
         const gf_topo_grid& G = grids[order[m]];
@@ -153,11 +153,44 @@ __device__ bool cell_integral(const Rect& cell, const gf_topo_grid* grids, const
     return false;
 }
 
-/* Tile of raster cells of a CTA of kTX x kTY threads (kRows rows of cells, some
- * for each thread), and the most node cells of a column (row) of cells that its
- * tables hold: coarser cells take the general path. */
-constexpr int kTX = 32, kTY = 8, kRows = 32, kPer = kRows / kTY, kNodes = 40;
-static_assert(kRows == kTX, "one warp per axis");
+__device__ __noinline__ bool cell_integral(const Rect& cell, const gf_topo_grid* grids, const int* order, int n,
+                                           double* out)
+{
+    return cell_integral_inline(cell, grids, order, n, out);
+}
+
+/* raster index g along an axis, a cell outside the domain taken as the
+ * cell inside that setaux's index shift names:
+ * i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)) */
+__device__ __forceinline__ int inside_index(int g, double low, double d, double up)
+{
+    const double x = low + (g + 0.5) * d;
+    if (x < low || x > up) g += (int)fmax(0.0, ceil((low - x) / d)) - (int)fmax(0.0, ceil((x - up) / d));
+    return g;
+}
+
+/* Cells over more nodes of the finest grid than the tiles' tables hold: one
+ * thread per cell, a chain of thousands of node cells each. */
+__global__ void __launch_bounds__(128)
+    topo_coarse_kernel(const gf_topo_grid* __restrict__ grids, const int* __restrict__ order, int n, int nx, int ny,
+                       int halo, double xlower, double ylower, double dx, double dy, double xupper, double yupper,
+                       double* __restrict__ out, int* __restrict__ err)
+{
+    const long p = nx + 2 * halo, e = blockIdx.x * (long)blockDim.x + threadIdx.x;
+    if (e >= p * (ny + 2 * halo)) return;
+    const int gi = inside_index((int)(e % p) - halo, xlower, dx, xupper);
+    const int gj = inside_index((int)(e / p) - halo, ylower, dy, yupper);
+    const Rect cell = {xlower + (double)gi * dx, xlower + (double)(gi + 1) * dx, ylower + (double)gj * dy,
+                       ylower + (double)(gj + 1) * dy};
+    double v;
+    if (!cell_integral_inline(cell, grids, order, n, &v)) *err = 1;
+    out[e] = v / (dx * dy);
+}
+
+/* Tile of raster cells of a CTA of kTX x kTY threads: kRows rows, some for each
+ * thread. kNodes: the most node cells of a column (row) of cells that its tables
+ * hold; coarser cells take the general path. */
+constexpr int kTX = 32, kNodes = 40;
 
 /* One axis of the integral of a column (row) of cells [lo, hi] over a grid:
  * the node cells i0 .. i1 - 1 it touches, and for each the width of the
@@ -220,13 +253,16 @@ __device__ __forceinline__ double over_area(double v, double area, double rarea)
  * with a warp for each row of them, 422 us gathered (82 % FP64 pipe, 89 FP64
  * instructions for 32 cells). Cells outside the domain are cells inside to this
  * kernel (a pass of its own over the raster took 31 us). */
+template <int kTY, int kRows>
 __global__ void __launch_bounds__(kTX* kTY)
     topo_raster_kernel(const gf_topo_grid* __restrict__ grids, const int* __restrict__ order, int n, int nx, int ny,
                        int halo, double xlower, double ylower, double dx, double dy, double xupper, double yupper,
                        double area, double rarea, double* __restrict__ out, int* __restrict__ err)
 {
-    __shared__ AxisNode xt[kNodes][kTX], yt[kNodes][kRows];
-    __shared__ AxisCell ax[kTX], ay[kRows];
+    constexpr int kPer = kRows / kTY;
+    constexpr bool kGather = kRows > 4;
+    __shared__ AxisNode xt[kNodes][kTX], yt[kNodes][kTX];
+    __shared__ AxisCell ax[kTX], ay[kTX];
     __shared__ unsigned short rest[kTX * kRows]; /* cells of the general path */
     __shared__ int nrest;
     const int tx = threadIdx.x, ty = threadIdx.y;
@@ -235,12 +271,8 @@ __global__ void __launch_bounds__(kTX* kTY)
     const int i = bx * kTX + tx, jb = by * kRows;
     if (ty == 2 && tx == 0) nrest = 0;
     if (ty < 2) { /* warp 0 the columns, warp 1 the rows */
-        int g = (ty ? jb + tx : i) - halo;
         const double low = ty ? ylower : xlower, d = ty ? dy : dx, up = ty ? yupper : xupper;
-        /* a cell outside the domain takes the cell inside that setaux's index
-         * shift names: i + max(0, ceil((xlower - x)/dx)) - max(0, ceil((x - xupper)/dx)) */
-        const double x = low + (g + 0.5) * d;
-        if (x < low || x > up) g += (int)fmax(0.0, ceil((low - x) / d)) - (int)fmax(0.0, ceil((x - up) / d));
+        const int g = inside_index((ty ? jb + tx : i) - halo, low, d, up);
         AxisCell& A = ty ? ay[tx] : ax[tx];
         A.lo = low + (double)g * d;
         A.hi = low + (double)(g + 1) * d;
@@ -278,12 +310,12 @@ __global__ void __launch_bounds__(kTX* kTY)
             __syncthreads();
             {
                 const AxisCell& A = ax[tx];
-                const int c = min(A.i1 - A.i0, kNodes);
+                const int c = A.i1 - A.i0 <= kNodes ? A.i1 - A.i0 : 0;
                 for (int e = ty; e < c; e += kTY) xt[e][tx] = axis_node(A.clo, A.chi, G.xlow, G.dx, A.i0 + e);
             }
             {
                 const AxisCell& A = ay[tx];
-                const int c = min(A.i1 - A.i0, kNodes);
+                const int c = A.i1 - A.i0 <= kNodes ? A.i1 - A.i0 : 0;
                 for (int e = kTY - 1 - ty; e < c; e += kTY) yt[e][tx] = axis_node(A.clo, A.chi, G.ylow, G.dy, A.i0 + e);
             }
             __syncthreads();
@@ -321,12 +353,22 @@ __global__ void __launch_bounds__(kTX* kTY)
         if (!__syncthreads_or(open != 0)) break;
     }
     if (open) *err = 1; /* no grid under a cell */
-#pragma unroll
     for (int q = 0; q < kPer; ++q) {
         const int k = ty + q * kTY;
-        if (general >> q & 1) rest[atomicAdd(&nrest, 1)] = (unsigned short)(k * kTX + tx);
-        else if (live >> q & 1) out[(long)(jb + k) * p + i] = over_area(v[q], area, rarea);
+        __syncwarp();
+        const bool cutc = general >> q & 1;
+        const int ncut = __popc(__ballot_sync(0xffffffffu, cutc));
+        if (kGather && cutc && ncut < kTX / 4) {
+            rest[atomicAdd(&nrest, 1)] = (unsigned short)(k * kTX + tx);
+            continue;
+        }
+        if (cutc) {
+            const Rect cell = {ax[tx].lo, ax[tx].hi, ay[k].lo, ay[k].hi};
+            cell_integral(cell, grids, order, n, &v[q]);
+        }
+        if (live >> q & 1) out[(long)(jb + k) * p + i] = over_area(v[q], area, rarea);
     }
+    if (!kGather) return;
     __syncthreads();
     for (int e = ty * kTX + tx; e < nrest; e += kTX * kTY) {
         const int k = rest[e] / kTX, c = rest[e] % kTX;
@@ -341,18 +383,37 @@ __global__ void __launch_bounds__(kTX* kTY)
 
 cudaError_t launch_topo_raster(const gf_topo_grid* grids, const int* order, int n, int nx, int ny, int halo,
                                double xlower, double ylower, double dx, double dy, double xupper,
-                               double yupper, double* out, int* err, cudaStream_t st)
+                               double yupper, double finest, double* out, int* err, cudaStream_t st)
 {
     if (n < 1 || n > GF_TOPO_MAX_FILES) return cudaErrorInvalidValue;
     const long cols = (nx + 2 * halo + kTX - 1) / kTX;
-    const long tiles = cols * ((ny + 2 * halo + kRows - 1) / kRows);
-    if (tiles > 0x7fffffffL) return cudaErrorInvalidValue; /* 2e12 cells */
-    const dim3 block(kTX, kTY);
     const double area = dx * dy;
-    const double rarea = area > 0x1p-500 && area < 0x1p500 ? 1.0 / area : 0.0;
-    topo_raster_kernel<<<(unsigned)tiles, block, 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy,
-                                                          xupper, yupper, area, rarea, out, err);
-    return cudaGetLastError();
+    const double rarea = area > 1e-150 && area < 1e150 ? 1.0 / area : 0.0;
+    const long cells = (long)(nx + 2 * halo) * (ny + 2 * halo);
+    /* cells beyond the tables gain nothing from tiles (64^2 and 128^2 cells of 64
+     * and 32 m over a 0.5 m inset 35.0 and 10.2 ms so, 37.8 and 11.0 in tiles;
+     * 256^2 of 16 m 2.84 and 2.16) */
+    if (fmax(dx, dy) > (kNodes - 2) * finest) {
+        if (cells > 128L * 0x7fffffffL) return cudaErrorInvalidValue;
+        topo_coarse_kernel<<<(unsigned)((cells + 127) / 128), 128, 0, st>>>(grids, order, n, nx, ny, halo, xlower,
+                                                                            ylower, dx, dy, xupper, yupper, out, err);
+        return cudaGetLastError();
+    }
+    /* 32 rows a CTA share most of what belongs to a column, but leave SMs idle on
+     * small rasters, and so do 8 on smaller ones, where a gathered warp of cut
+     * cells is a longer chain than each cell in its place: us for 64^2 / 512^2 /
+     * 2048^2 cells with 4 rows 1650 / 460 / -, 8 rows 1775 / 350 / 2410, 32 rows
+     * 3314 / 369 / 2275 */
+    auto run = [&](auto* kern, int ty, int rows) -> cudaError_t {
+        const long tiles = cols * ((ny + 2 * halo + rows - 1) / rows);
+        if (tiles > 0x7fffffffL) return cudaErrorInvalidValue; /* 3e11 cells */
+        kern<<<(unsigned)tiles, dim3(kTX, ty), 0, st>>>(grids, order, n, nx, ny, halo, xlower, ylower, dx, dy, xupper,
+                                                        yupper, area, rarea, out, err);
+        return cudaGetLastError();
+    };
+    if (cells >= 8L * sm_count() * kTX * 32) return run(topo_raster_kernel<8, 32>, 8, 32);
+    if (cells >= 2L * sm_count() * kTX * 8) return run(topo_raster_kernel<8, 8>, 8, 8);
+    return run(topo_raster_kernel<4, 4>, 4, 4);
 }
 
 } // namespace gf
