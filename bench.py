@@ -44,8 +44,8 @@ BYTES_PER_CELL_UPDATE = 56  # read h, hu, hv, b; write h, hu, hv (FP64)
 # capture of the launch this bench times first in its kernel-only loop (update
 # launch 24 of `--steps 20 --warmup 3`, the same state): DRAM traffic
 # (dram__bytes_read.sum + dram__bytes_write.sum; below the 234.9 MB algorithmic,
-# since rows without water are read for their depth alone) and FP64 warp instructions (sm__inst_executed_pipe_fp64.sum;
-# x 32 lanes / 4 194 304 cell-updates = FP64 issue slots per cell-update)
+# since rows without water are read for their depth alone) and FP64 warp
+# instructions (sm__inst_executed_pipe_fp64.sum; x 32 lanes / 4 194 304 cell-updates = FP64 issue slots per cell-update)
 NCU_COUNTS = {(256, 4): (90.650368e6 + 89.671680e6, 18.152225e6)}
 NCU_DEFAULT_TILE = (256, 4)
 M = 32

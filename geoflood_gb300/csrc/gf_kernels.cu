@@ -2,11 +2,8 @@
  * Kernel instantiations and launchers for the patch update and the
  * host-layout conversions used at the drop-in boundary.
  *
- * Tile shapes per patch size m (threads per CTA, slices per band):
- *   m = 32: 256 threads, 7 slices  (245 / 231 faces per band stage)
- *   m = 16: 128 threads, 6 slices  (114 / 102)
- *   m =  8: 128 threads, 10 slices (110 /  90)
- * chosen so the flattened face loops of a band fill the CTA.
+ * The tile shapes per patch size and the choice among them stand at kTiles8 ..
+ * kTiles32 and pick_tile.
  */
 #include <cuda_runtime.h>
 

@@ -533,7 +533,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
     double* TP = TM + 3 * MM;
 
     /* cells [e0, e0 + step, ..) of those the slices t0..t1 feed: n in [1, M],
-     * t in [t0-1, t1+1] (interior), within the window */
+     * t in [t0-1, t1+1] (interior) */
     auto gather_cells = [&](int t0, int t1) -> int {
         return (min(M, t1 + 1) - max(1, t0 - 1) + 1) * M;
     };

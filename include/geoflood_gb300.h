@@ -799,9 +799,10 @@ double gf_fserver_clock(const gf_fserver* s);
 
 /* ------------------------------------------------------------ tiling */
 /* Tile shapes of the production patch kernel (threads per patch x slices
- * per band) per patch size, measured on this device: the fastest for whole
+ * or rows per band) per patch size. A launch takes its tile by its number of
+ * patches; gf_autotune measures them on this device, and the fastest for whole
  * levels (throughput) and the fastest lone small batch (latency) become
- * the process-wide choice; the served form's smallest lane uses the
+ * the process-wide choice for launches that fill the device; the served form's smallest lane uses the
  * latency choice, everything else the throughput choice. Synthetic
  * all-wet patches, physics slot 0 of the context, `reps` timed launches
  * per variant. No reference counterpart (tuning support). */
