@@ -27,6 +27,7 @@ from ._lib import STATUS_NAMES, dptr, dptrs, iptr
 
 MBC = 2
 MEQN = 3
+TILE_AUTO = -100  # set_tile: the launch's number of patches decides
 
 
 class GeoFloodError(RuntimeError):
@@ -182,11 +183,31 @@ class Context:
 
     @staticmethod
     def tile(mx: int, goal: int = 0) -> int:
-        """Selected tile variant for patch size mx (goal 0 throughput, 1 latency)."""
+        """Tile variant chosen by hand or by autotune for patch size mx (goal 0
+        throughput, 1 latency); TILE_AUTO without a choice."""
         return int(_lib.load().gf_tile_get(int(mx), int(goal)))
 
     @staticmethod
+    def tile_of(mx: int, npatch: int, goal: int = 0) -> int:
+        """Tile variant that a launch of npatch patches takes."""
+        v = int(_lib.load().gf_tile_of(int(mx), int(npatch), int(goal)))
+        if v < 0:
+            raise GeoFloodError(v, "no such patch size or number of patches")
+        return v
+
+    @staticmethod
+    def tile_shape(mx: int, variant: int) -> tuple:
+        """(threads, slices or rows per band, cluster) of a variant."""
+        t = (C.c_int * 3)()
+        p = [C.cast(C.byref(t, 4 * k), C.POINTER(C.c_int)) for k in range(3)]
+        rc = _lib.load().gf_tile_shape(int(mx), int(variant), *p)
+        if rc != 0:
+            raise GeoFloodError(rc, "no such tile variant")
+        return tuple(t)
+
+    @staticmethod
     def set_tile(mx: int, goal: int, variant: int):
+        """Pin a tile variant by hand; TILE_AUTO takes the choice back."""
         rc = _lib.load().gf_tile_set(int(mx), int(goal), int(variant))
         if rc != 0:
             raise GeoFloodError(rc, "no such tile variant")

@@ -285,6 +285,8 @@ SIGNATURES = [
     ("gf_tile_count", C.c_int, [C.c_int]),
     ("gf_tile_get", C.c_int, [C.c_int, C.c_int]),
     ("gf_tile_set", C.c_int, [C.c_int, C.c_int, C.c_int]),
+    ("gf_tile_of", C.c_int, [C.c_int, C.c_int, C.c_int]),
+    ("gf_tile_shape", C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
     ("gf_server_opts_default", None, [C.POINTER(gf_server_opts)]),
     ("gf_server_create", C.c_int, [C.c_int, C.POINTER(gf_server_opts), C.POINTER(_vp)]),
     ("gf_server_destroy", None, [_vp]),

@@ -1240,6 +1240,18 @@ extern "C" int gf_tile_set(int mx, int goal, int variant)
     return gf::tile_set(mx, goal, variant) ? GF_ERR_ARG : GF_OK;
 }
 
+extern "C" int gf_tile_of(int mx, int npatch, int goal)
+{
+    if (!(mx == 8 || mx == 16 || mx == 32) || npatch < 1) return GF_ERR_ARG;
+    return gf::tile_of(mx, npatch, goal);
+}
+
+extern "C" int gf_tile_shape(int mx, int variant, int* threads, int* band, int* cluster)
+{
+    if (!threads || !band || !cluster) return GF_ERR_ARG;
+    return gf::tile_shape(mx, variant, threads, band, cluster) ? GF_ERR_ARG : GF_OK;
+}
+
 extern "C" int gf_autotune(gf_ctx* c, int reps, gf_tile_result* out)
 {
     if (!c || !out || reps < 1) return GF_ERR_ARG;

@@ -51,13 +51,17 @@ cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, con
                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                 unsigned long long* gmax, int* err, cudaStream_t st,
                                 int max_ctas = 0, int goal = 0);
-int patch_update_occupancy(int m); /* resident CTAs per SM (throughput tile) */
+/* resident CTAs per SM of the chosen throughput tile, else of the default one */
+int patch_update_occupancy(int m);
 
 /* Tile shapes of the production patch kernel: variants per patch size, the
- * selection per goal (0 throughput, 1 latency) used by launch_patch_update. */
+ * choice per goal (0 throughput, 1 latency) that launch_patch_update honours
+ * (GF_TILE_AUTO: none, the number of patches decides), and the tile that an
+ * uncapped launch of npatch patches takes. */
 int tile_count(int m);
 int tile_shape(int m, int v, int* nt, int* rb, int* k = nullptr);
 int tile_get(int m, int goal);
+int tile_of(int m, long npatch, int goal);
 /* 1 when npatch patches of size m on the latency tile (each over its
  * cluster of CTAs) are all resident at once on the device, else 0 */
 int latency_goal_fits(int m, long npatch);

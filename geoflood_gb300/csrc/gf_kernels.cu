@@ -176,17 +176,18 @@ static const Tile* tiles_of(int m, int* n)
     }
 }
 
-/* Selected variant per goal (0 throughput, 1 latency) and patch size, and the
- * selection that stands for "by the number of patches" (pick_tile): the
- * defaults here, or what gf_autotune installed. 8^2 patches take the
+/* Tile of a launch without a choice by hand, where the number of patches does
+ * not name another one (pick_tile). 8^2 patches take the
  * streamed form, a whole patch in its one band, four CTAs an SM (4096 patches
  * 288 us, three CTAs 305, 128 x 10 swept 323), 16^2 its bands of five rows,
  * three CTAs an SM (5561 patches 1.27 ms at 80 % wet and 0.85 at 50 %, swept
  * 128 x 6 1.31 and 0.92, streamed 192 x 7 1.34 and 0.93), 32^2 patches 384 x 9
  * (4096 patches 3.43 ms, 256 x 7 3.61) or the streamed form, pick_tile. */
-static int g_tile[2][3] = {{2, 0, 3}, {2, 0, 3}};
-static int g_auto[2][3] = {{2, 0, 3}, {2, 0, 3}};
-static bool g_tuned[3] = {false, false, false};
+static const int kDefault[3] = {2, 0, 3};
+/* Chosen per goal (0 throughput, 1 latency) and patch size: by hand (tile_set),
+ * by gf_autotune; -1: not. */
+static std::atomic<int> g_pin[2][3] = {{-1, -1, -1}, {-1, -1, -1}};
+static std::atomic<int> g_tuned[2][3] = {{-1, -1, -1}, {-1, -1, -1}};
 static inline int mcls(int m) { return m == 8 ? 0 : m == 16 ? 1 : 2; }
 
 int tile_count(int m)
@@ -207,7 +208,17 @@ int tile_shape(int m, int v, int* nt, int* rb, int* k)
     return 0;
 }
 
-int tile_get(int m, int goal) { return g_tile[goal != 0][mcls(m)]; }
+static int chosen(int m, int goal) /* by hand, else tuned, else -1 */
+{
+    const int pin = g_pin[goal != 0][mcls(m)];
+    return pin >= 0 ? pin : g_tuned[goal != 0][mcls(m)].load();
+}
+
+int tile_get(int m, int goal)
+{
+    const int v = chosen(m, goal);
+    return v >= 0 ? v : GF_TILE_AUTO;
+}
 
 /* Patches that one launch of variant v runs at once on this device. */
 static long tile_resident(int m, int v)
@@ -234,7 +245,8 @@ int latency_goal_fits(int m, long npatch)
 {
     int n = 0;
     if (!tiles_of(m, &n)) return 0;
-    return npatch <= tile_resident(m, g_tile[1][mcls(m)]) ? 1 : 0;
+    const int v = chosen(m, 1);
+    return npatch <= tile_resident(m, v >= 0 ? v : kDefault[mcls(m)]) ? 1 : 0;
 }
 
 /* Launches that leave SMs idle take a tile that spreads a patch: the first of
@@ -258,43 +270,61 @@ static const SmallTile kSmall32[] = {{5, 2, true}, {4, 2, true}, {6, 7, false}};
  * gains (400 patches 509 us against 445, 760 767 against 732). */
 constexpr int kStream32 = 1, kStream32Waves = 6; /* patches an SM from which it always pays */
 
+/* Tile of a capped launch, whose CTAs walk the list on part of the SMs: no rule
+ * by the number of patches. */
+static int capped_tile(int m)
+{
+    const int v = chosen(m, 0);
+    return v >= 0 ? v : kDefault[mcls(m)];
+}
+
+/* A choice by hand always stands, the tuned latency tile where it is asked for;
+ * the tuned throughput tile where no patch is split. */
 static int pick_tile(int m, long npatch, int max_ctas, int goal)
 {
     const int c = mcls(m);
     goal = goal != 0;
-    /* chosen by hand, or the tuned latency tile asked for */
-    if (g_tile[goal][c] != g_auto[goal][c] || (goal && g_tuned[c])) return g_tile[goal][c];
-    if (max_ctas <= 0) {
-        int nt = 0;
-        const Tile* t = tiles_of(m, &nt);
-        const SmallTile* s = c == 0 ? kSmall8 : c == 1 ? kSmall16 : kSmall32;
-        const int ns = (int)(c == 0 ? sizeof kSmall8 : c == 1 ? sizeof kSmall16 : sizeof kSmall32) / (int)sizeof *s;
-        for (int i = 0; i < ns; ++i)
-            if (2 * npatch * t[s[i].v].k <= (long)s[i].per_2sm * sm_count() &&
-                (!s[i].one_wave || npatch <= tile_resident(m, s[i].v)))
-                return s[i].v;
-        if (c == 2 && !g_tuned[c] &&
-            (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
-            return kStream32;
-    }
-    return g_tile[0][c];
+    const int pin = g_pin[goal][c], best = g_tuned[goal][c];
+    if (pin >= 0) return pin;
+    if (goal && best >= 0) return best;
+    if (max_ctas > 0) return capped_tile(m);
+    int nt = 0;
+    const Tile* t = tiles_of(m, &nt);
+    const SmallTile* s = c == 0 ? kSmall8 : c == 1 ? kSmall16 : kSmall32;
+    const int ns = (int)(c == 0 ? sizeof kSmall8 : c == 1 ? sizeof kSmall16 : sizeof kSmall32) / (int)sizeof *s;
+    for (int i = 0; i < ns; ++i)
+        if (2 * npatch * t[s[i].v].k <= (long)s[i].per_2sm * sm_count() &&
+            (!s[i].one_wave || npatch <= tile_resident(m, s[i].v)))
+            return s[i].v;
+    if (const int by_hand = g_pin[0][c]; by_hand >= 0) return by_hand; /* goal 1 */
+    if (const int tuned = g_tuned[0][c]; tuned >= 0) return tuned;
+    if (c == 2 && (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
+        return kStream32;
+    return kDefault[c];
 }
+
+int tile_of(int m, long npatch, int goal) { return pick_tile(m, npatch, 0, goal); }
 
 int tile_set(int m, int goal, int v)
 {
     int n = 0;
     tiles_of(m, &n);
+    if (v == GF_TILE_AUTO) {
+        g_pin[goal != 0][mcls(m)] = -1;
+        g_tuned[goal != 0][mcls(m)] = -1;
+        return 0;
+    }
     if (v < 0 || v >= n) return -1;
-    g_tile[goal != 0][mcls(m)] = v;
+    g_pin[goal != 0][mcls(m)] = v;
     return 0;
 }
 
 void tile_install_tuned(int m, int throughput, int latency)
 {
     const int c = mcls(m);
-    g_tile[0][c] = g_auto[0][c] = throughput;
-    g_tile[1][c] = g_auto[1][c] = latency;
-    g_tuned[c] = true;
+    g_tuned[0][c] = throughput;
+    g_tuned[1][c] = latency;
+    g_pin[0][c] = g_pin[1][c] = -1;
 }
 
 cudaError_t launch_patch_update_tile(int m, int v, const gf_patch_work* work, int nwork,
@@ -381,7 +411,7 @@ int patch_update_occupancy(int m)
 {
     int n = 0;
     const Tile* t = tiles_of(m, &n);
-    return t ? t[g_tile[0][mcls(m)]].occ() : 0;
+    return t ? t[capped_tile(m)].occ() : 0;
 }
 
 /* ---- layout conversion at the boundary ----

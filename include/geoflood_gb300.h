@@ -799,11 +799,11 @@ double gf_fserver_clock(const gf_fserver* s);
 
 /* ------------------------------------------------------------ tiling */
 /* Tile shapes of the production patch kernel (threads per patch x slices
- * or rows per band) per patch size. A launch takes its tile by its number of
- * patches; gf_autotune measures them on this device, and the fastest for whole
- * levels (throughput) and the fastest lone small batch (latency) become
- * the process-wide choice for launches that fill the device; the served form's smallest lane uses the
- * latency choice, everything else the throughput choice. Synthetic
+ * or rows per band, split of a patch over a cluster) per patch size. Without a
+ * choice a launch takes its tile by its number of patches. gf_autotune times
+ * every shape on this device and chooses, for the process, the fastest for a
+ * level of 4 million cells (throughput: launches that split no patch) and the
+ * fastest for 8 patches (latency). It takes back choices by hand. Synthetic
  * all-wet patches, physics slot 0 of the context, `reps` timed launches
  * per variant. No reference counterpart (tuning support). */
 #define GF_MAX_TILES 12
@@ -820,14 +820,23 @@ typedef struct gf_tile_result {
 int gf_autotune(gf_ctx* ctx, int reps, gf_tile_result* out /* [3]: mx 8, 16, 32 */);
 /* Number of tile variants of patch size mx. */
 int gf_tile_count(int mx);
-/* Current choice (goal 0 throughput, 1 latency) or a manual one. Levels,
- * forests and batched rounds take the throughput choice; a batch through
+/* Threads, slices or rows per band and cluster of a variant. */
+int gf_tile_shape(int mx, int variant, int* threads, int* band, int* cluster);
+/* Choice per goal (0 throughput, 1 latency). gf_tile_set pins a variant by hand:
+ * every launch of the goal takes it, whatever its number of patches.
+ * GF_TILE_AUTO takes a pin and a tuned choice back. gf_tile_get returns the
+ * pinned variant, else the tuned one, else GF_TILE_AUTO. Levels,
+ * forests and batched rounds ask for goal 0; a batch through
  * gf_patch_update / gf_patch_update_batch / gf_step_buffer_update, and a
- * step of the served form's smallest lane, take the latency choice when
- * all their patches run in one wave of it (no more patches than the
- * clusters of that tile the GPU holds resident at once). */
+ * step of the served form's smallest lane, ask for goal 1 when
+ * all their patches run in one wave of its variant (no more patches than the
+ * clusters of that tile the GPU holds resident at once; without a choice, the
+ * tile of whole levels). */
+#define GF_TILE_AUTO (-100)
 int gf_tile_get(int mx, int goal);
 int gf_tile_set(int mx, int goal, int variant);
+/* Variant that a launch of npatch patches takes on the current device. */
+int gf_tile_of(int mx, int npatch, int goal);
 
 /* ----------------------------------------------------------- probes */
 /* Measured FP64 pipe rates of `device` in operations per second:

@@ -94,6 +94,22 @@ def test_tile_switches_of_wider_launches_give_the_same_bits(ctx, m, npx):
 
 
 @pytest.mark.parametrize("m", [8, 16, 32])
+def test_every_switch_of_the_tile_gives_the_same_bits(ctx, m):
+    """The numbers of patches at which the tile changes, clusters resident at
+    once on this device among them: either side has the bits of one fixed tile."""
+    keep = gf.Context.tile(m, 0)
+    gf.Context.set_tile(m, 0, gf.TILE_AUTO)
+    try:
+        of = [gf.Context.tile_of(m, n) for n in range(1, 1001)]
+        counts = [n + d for n in range(1, 1000) if of[n - 1] != of[n] for d in (0, 1)]
+        assert len(counts) >= 2
+        for n in counts:
+            test_tile_switches_of_wider_launches_give_the_same_bits(ctx, m, n)
+    finally:
+        gf.Context.set_tile(m, 0, keep)
+
+
+@pytest.mark.parametrize("m", [8, 16, 32])
 @pytest.mark.parametrize("kind", ["band", "row", "thin"])
 def test_dry_rows_and_windows(ctx, m, kind):
     """Water in some rows only (a band of rows at every height, a single row at
