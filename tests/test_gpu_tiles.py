@@ -103,8 +103,20 @@ def test_every_switch_of_the_tile_gives_the_same_bits(ctx, m):
         of = [gf.Context.tile_of(m, n) for n in range(1, 1001)]
         counts = [n + d for n in range(1, 1000) if of[n - 1] != of[n] for d in (0, 1)]
         assert len(counts) >= 2
+        q, aux, _, _ = synth.uniform_dam_break_level(32, -(-max(counts) // 32), m, 1.0, seed=m, x_dam=12.8 * m)
+        ctx.set_phys(0, gf.Phys())
         for n in counts:
-            test_tile_switches_of_wider_launches_give_the_same_bits(ctx, m, n)
+            outs = []
+            for v in (gf.TILE_AUTO, 2 if m == 16 else 0):
+                gf.Context.set_tile(m, 0, v)
+                lev = gf.Level(ctx, n, m, 1)
+                lev.set_geometry(1.0, 1.0)
+                lev.upload(np.ascontiguousarray(q[:n]), np.ascontiguousarray(aux[:n]))
+                cfl = lev.step(0.0, 0.05)
+                outs.append((lev.download(), cfl, lev.patch_cfl()))
+                lev.close()
+            assert np.array_equal(outs[0][0], outs[1][0]) and outs[0][1] == outs[1][1]
+            assert np.array_equal(outs[0][2], outs[1][2])
     finally:
         gf.Context.set_tile(m, 0, keep)
 
