@@ -1259,8 +1259,7 @@ extern "C" int gf_autotune(gf_ctx* c, int reps, gf_tile_result* out)
     if (rc) return rc;
     GF_CK(c, cudaSetDevice(c->device));
     static const int ms[3] = {8, 16, 32};
-    const long target_cells = 4L << 20;
-    const int nsmall = 8;
+        const int nsmall = 8;
     cudaEvent_t e0, e1;
     GF_CK(c, cudaEventCreate(&e0));
     GF_CK(c, cudaEventCreate(&e1));
@@ -1268,7 +1267,7 @@ extern "C" int gf_autotune(gf_ctx* c, int reps, gf_tile_result* out)
     for (int k = 0; k < 3 && result == GF_OK; ++k) {
         const int m = ms[k];
         const long S = cells_of(m, m);
-        const int np = (int)(target_cells / ((long)m * m));
+        const int np = (int)(gf::kTuneCells / ((long)m * m));
         gf_tile_result& R = out[k];
         std::memset(&R, 0, sizeof R);
         R.mx = m;

@@ -51,8 +51,9 @@ cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, con
                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                 unsigned long long* gmax, int* err, cudaStream_t st,
                                 int max_ctas = 0, int goal = 0);
-/* resident CTAs per SM of the chosen throughput tile, else of the default one */
-int patch_update_occupancy(int m);
+/* resident CTAs per SM of the tile of capped launches, or of the one chosen by
+ * hand or, without, by default for whole levels */
+int patch_update_occupancy(int m, bool capped = false);
 
 /* Tile shapes of the production patch kernel: variants per patch size, the
  * choice per goal (0 throughput, 1 latency) that launch_patch_update honours
@@ -62,6 +63,7 @@ int tile_count(int m);
 int tile_shape(int m, int v, int* nt, int* rb, int* k = nullptr);
 int tile_get(int m, int goal);
 int tile_of(int m, long npatch, int goal);
+constexpr long kTuneCells = 4L << 20; /* cells of the level that gf_autotune times */
 /* 1 when npatch patches of size m on the latency tile (each over its
  * cluster of CTAs) are all resident at once on the device, else 0 */
 int latency_goal_fits(int m, long npatch);

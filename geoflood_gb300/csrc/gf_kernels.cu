@@ -278,8 +278,10 @@ static int capped_tile(int m)
     return v >= 0 ? v : kDefault[mcls(m)];
 }
 
-/* A choice by hand always stands, the tuned latency tile where it is asked for;
- * the tuned throughput tile where no patch is split. */
+/* A choice by hand always stands, the tuned latency tile where it is asked for.
+ * The tuned throughput tile serves launches of the size it was measured on:
+ * below, the number of patches decides as without it (400 patches of 32^2 442 us
+ * so, 504 by the tile that is the fastest for 4096; 760 612 and 671). */
 static int pick_tile(int m, long npatch, int max_ctas, int goal)
 {
     const int c = mcls(m);
@@ -297,7 +299,7 @@ static int pick_tile(int m, long npatch, int max_ctas, int goal)
             (!s[i].one_wave || npatch <= tile_resident(m, s[i].v)))
             return s[i].v;
     if (const int by_hand = g_pin[0][c]; by_hand >= 0) return by_hand; /* goal 1 */
-    if (const int tuned = g_tuned[0][c]; tuned >= 0) return tuned;
+    if (const int tuned = g_tuned[0][c]; tuned >= 0 && npatch * m * m >= kTuneCells) return tuned;
     if (c == 2 && (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
         return kStream32;
     return kDefault[c];
@@ -407,11 +409,13 @@ cudaError_t launch_patch_update_mixed(const gf_patch_work* work, const int n[3],
     return cudaGetLastError();
 }
 
-int patch_update_occupancy(int m)
+int patch_update_occupancy(int m, bool capped)
 {
     int n = 0;
     const Tile* t = tiles_of(m, &n);
-    return t ? t[capped_tile(m)].occ() : 0;
+    if (!t) return 0;
+    const int pin = g_pin[0][mcls(m)];
+    return t[capped ? capped_tile(m) : pin >= 0 ? pin : kDefault[mcls(m)]].occ();
 }
 
 /* ---- layout conversion at the boundary ----

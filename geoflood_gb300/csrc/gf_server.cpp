@@ -855,7 +855,7 @@ int gf_server_create(int device, const gf_server_opts* opts, gf_server** out)
     for (int k = 1; k < o.nlanes; ++k) {
         const int sms = nsm - o.reserve_sms;
         for (int c = 0; c < 3; ++c) {
-            const int occ = gf::patch_update_occupancy(ms[c]);
+            const int occ = gf::patch_update_occupancy(ms[c], true);
             s->cta_cap[k][c] = (o.reserve_sms > 0 && sms > 0 && occ > 0) ? sms * occ : 0;
         }
         s->mix_cap[k] = (o.reserve_sms > 0 && sms > 0) ? sms : 0; /* one CTA per SM */

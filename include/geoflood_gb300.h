@@ -802,8 +802,9 @@ double gf_fserver_clock(const gf_fserver* s);
  * or rows per band, split of a patch over a cluster) per patch size. Without a
  * choice a launch takes its tile by its number of patches. gf_autotune times
  * every shape on this device and chooses, for the process, the fastest for a
- * level of 4 million cells (throughput: launches that split no patch) and the
- * fastest for 8 patches (latency). It takes back choices by hand. Synthetic
+ * level of 4 million cells (throughput: launches of that size and capped ones;
+ * smaller launches go by their number of patches as before) and the fastest for
+ * 8 patches (latency). It takes back choices by hand. Synthetic
  * all-wet patches, physics slot 0 of the context, `reps` timed launches
  * per variant. No reference counterpart (tuning support). */
 #define GF_MAX_TILES 12

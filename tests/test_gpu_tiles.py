@@ -168,6 +168,27 @@ def test_autotune_measures_and_selects(ctx):
         gf.Context.set_tile(8, 0, 9)
 
 
+def test_autotune_leaves_smaller_launches_to_their_number_of_patches(ctx):
+    """The throughput choice is that of a level of 4M cells: it serves launches of
+    that size, and smaller ones take the tiles they take without it."""
+    counts = (1, 100, 247, 300, 400, 760, 911, 1073, 4095)
+    try:
+        for m in (8, 16, 32):
+            for goal in (0, 1):
+                gf.Context.set_tile(m, goal, gf.TILE_AUTO)
+        before = [[gf.Context.tile_of(m, n) for n in counts] for m in (8, 16, 32)]
+        ctx.set_phys(0, gf.Phys())
+        res = ctx.autotune(reps=1)
+        assert [[gf.Context.tile_of(m, n) for n in counts] for m in (8, 16, 32)] == before
+        for r in res:
+            assert gf.Context.tile_of(r["mx"], (4 << 20) // r["mx"] ** 2) == r["best_throughput"]
+            assert gf.Context.tile_of(r["mx"], 8, 1) == r["best_latency"]
+    finally:
+        for m in (8, 16, 32):
+            for goal in (0, 1):
+                gf.Context.set_tile(m, goal, gf.TILE_AUTO)
+
+
 @pytest.mark.parametrize("m", [8, 16, 32])
 def test_small_host_batches_take_the_latency_tile_with_the_same_bits(ctx, m):
     """gf_patch_update_batch on a handful of patches runs the latency
