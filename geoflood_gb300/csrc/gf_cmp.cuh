@@ -9,7 +9,10 @@
  *   - against zero they are exact (x > 0, x < 0, x == 0 with either zero);
  *   - between two values they use the order-preserving integer key of the
  *     bit pattern, which agrees with IEEE ordering except that -0 sorts
- *     below +0 (IEEE: equal). Inputs are never NaN here.
+ *     below +0 (IEEE: equal). A NaN sorts by its sign, above infinity or below
+ *     minus infinity, where IEEE comparisons are false: a depth that is a
+ *     negative NaN is dry (the inflow states without a root, gf_ghost.cu), a
+ *     positive one wet. d_max_abs leaves a NaN out.
  * With FAST = false they are the IEEE operations themselves, so the
  * contraction-free build keeps the reference's arithmetic bit for bit.
  */
@@ -75,6 +78,16 @@ template <bool F> __device__ __forceinline__ double d_max_nn(double a, double b)
 {
     if (F) return gf_bits(a) < gf_bits(b) ? b : a;
     return fmax(a, b);
+}
+
+/* the larger of a (a number >= 0) and |x|; a where x is not a number, as fmax */
+template <bool F> __device__ __forceinline__ double d_max_abs(double a, double x)
+{
+    if (F) {
+        const long long b = gf_bits(x) & 0x7fffffffffffffffLL;
+        return b > gf_bits(a) && b <= 0x7ff0000000000000LL ? __longlong_as_double(b) : a;
+    }
+    return fmax(a, fabs(x));
 }
 
 /* The hardware's approximate FP64 reciprocal and reciprocal root (subnormal

@@ -428,9 +428,9 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
             w[6] = fw[1][1];
             w[7] = fw[2][0]; w[8] = fw[2][1]; w[9] = fw[2][2];
         }
-        const double m = d_max_nn<true>(d_max_nn<true>(fabs(s[0]), fabs(s[1])), fabs(s[2]));
-        if (y) smax_y = d_max_nn<true>(smax_y, m);
-        else smax_x = d_max_nn<true>(smax_x, m);
+        const double m = d_max_abs<true>(d_max_abs<true>(d_max_abs<true>(y ? smax_y : smax_x, s[0]), s[1]), s[2]);
+        if (y) smax_y = m;
+        else smax_x = m;
     };
     /* limited face i of band b: its records and its cells' wet flags */
     auto limited = [&](const Band& B, int i, int& w, int& wl, int& wr, int& o, int& kl, int& kr) -> bool {
@@ -636,10 +636,7 @@ __device__ __forceinline__ bool stream_item(double* sm, uint64_t* bar, uint32_t&
         }
     }
     {
-        auto number = [](double x) -> double {
-            return __double_as_longlong(x) <= 0x7ff0000000000000ll ? x : 0.0;
-        };
-        unsigned long long v = dkey(d_max_nn<true>(dtdx * number(smax_x), dtdy * number(smax_y)));
+        unsigned long long v = dkey(d_max_nn<true>(dtdx * smax_x, dtdy * smax_y));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);

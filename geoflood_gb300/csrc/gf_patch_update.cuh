@@ -642,7 +642,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
                 w[3 + 3 * mw + 0] = fw[mw][0];
                 w[3 + 3 * mw + 1] = fw[mw][1];
                 w[3 + 3 * mw + 2] = fw[mw][2];
-                smax = fmax(smax, fabs(s[mw]));
+                smax = d_max_abs<FAST>(smax, s[mw]);
             }
         }
     };
@@ -671,7 +671,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
         if (idx < nh) {
             full_solve(cl, cr, g, drytol, sc, w);
 #pragma unroll
-            for (int mw = 0; mw < 3; ++mw) smax = d_max_nn<FAST>(smax, fabs(w[mw]));
+            for (int mw = 0; mw < 3; ++mw) smax = d_max_abs<FAST>(smax, w[mw]);
             return;
         }
         double s[3], fw[3][3];
@@ -680,7 +680,7 @@ __device__ __forceinline__ double sweep(double* sm, const unsigned char* wet, co
 #pragma unroll
         for (int mw = 0; mw < 3; ++mw) {
             w[mw] = s[mw];
-            smax = d_max_nn<FAST>(smax, fabs(s[mw]));
+            smax = d_max_abs<FAST>(smax, s[mw]);
         }
         w[3] = fw[0][0]; w[4] = fw[0][1]; w[5] = fw[0][2];
         w[6] = fw[1][1];
@@ -1198,12 +1198,9 @@ __device__ __forceinline__ bool patch_item(double* sm, uint64_t* bar, uint32_t& 
 
     /* ---- CFL: the largest of dt/dx |s| and dt/dy |s|, over the warp, then over
      * the CTA, on the integer pipe (non-negative doubles order as integers);
-     * a NaN speed is left out ---- */
+     * NaN speeds were left out face by face ---- */
     {
-        auto number = [](double x) -> double {
-            return __double_as_longlong(x) <= 0x7ff0000000000000ll ? x : 0.0;
-        };
-        unsigned long long v = dkey(d_max_nn<true>(dtdx * number(smax_x), dtdy * number(smax_y)));
+        unsigned long long v = dkey(d_max_nn<true>(dtdx * smax_x, dtdy * smax_y));
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             const unsigned long long w = __shfl_xor_sync(0xffffffffu, v, o);
