@@ -516,8 +516,13 @@ int gf_level_create(gf_ctx* c, int npatch, int mx, int my, int maux, gf_level** 
     if (e == cudaSuccess) e = cudaMalloc(&L->d_geom, (size_t)npatch * sizeof(gf_patch_geom));
     if (e == cudaSuccess) e = cudaMalloc(&L->d_phys_of, (size_t)npatch * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&L->d_ghost, sizeof(gf_ghost_block));
-    if (e == cudaSuccess) e = cudaMemset(L->d_aux, 0, an * sizeof(double));
-    if (e == cudaSuccess) e = cudaMemset(L->d_q, 0, qn * sizeof(double));
+    /* done before any stream, the context's or the caller's, uses the planes; the
+     * status and CFLs too, which a wait or a read before the first step returns */
+    if (e == cudaSuccess) e = cudaMemsetAsync(L->d_aux, 0, an * sizeof(double), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(L->d_q, 0, qn * sizeof(double), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(L->d_status, 0, sizeof(DevStatus), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(L->d_cfl, 0, npatch * sizeof(double), c->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) {
         gf_level_destroy(L);
         return cuda_fail(c, e, "gf_level_create");
