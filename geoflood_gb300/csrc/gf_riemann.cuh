@@ -360,11 +360,34 @@ __device__ __forceinline__ void gf_rpn2_face(const gf_cell& Lc, const gf_cell& R
     fw[2][0] = f13 * wall2; fw[2][1] = f23 * wall2; fw[2][2] = f33 * wall2;
 }
 
+/* Single-precision products, fused sums, quotients and roots written as the
+ * operation they become, as gf_mul above: a face has the same class in every
+ * kernel. A host build (tests) brings its own root and __fdividef. */
 #ifndef GF_HOST_MATH
 __device__ __forceinline__ float gf_sqrtf(float x)
 {
     float r;
     asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float gf_fmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float gf_ffma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float gf_fdiv(float a, float b)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
+    return __fmul_rn(a, r);
+}
+#else
+__device__ __forceinline__ float gf_fmul(float a, float b)
+{
+    volatile float r = a * b;
+    return r;
+}
+__device__ __forceinline__ float gf_ffma(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ float gf_fdiv(float a, float b)
+{
+    volatile float r = __fdividef(a, b);
     return r;
 }
 #endif
@@ -397,15 +420,15 @@ __device__ __forceinline__ int gf_face_class(float hL, float hR, float uL, float
          * speeds lie 2 c inside the Einfeldt speeds */
         const float h = wetL ? hL : hR, u = wetL ? uL : -uR, c = wetL ? cL : cR;
         const float bw = wetL ? bL : bR, bd = wetL ? bR : bL;
-        const float r = fmaxf(c + 0.5f * u, 0.0f);
-        const float top = fmaxf(h, __fdividef(r * r, g));
+        const float r = fmaxf(gf_ffma(0.5f, u, c), 0.0f);
+        const float top = fmaxf(h, gf_fdiv(gf_fmul(r, r), g));
         const float gap = bd - (top + bw);
-        const float e = 1.0e-5f * top + 1.0e-6f * (fabsf(bw) + fabsf(bd));
+        const float e = gf_ffma(1.0e-5f, top, gf_fmul(1.0e-6f, fabsf(bw) + fabsf(bd)));
         const bool ok = (h > 1.0e-15f) & (h < 1.0e15f) & (S < 1.0e15f);
         return ok & (gap > e) ? 2 : ok & (gap < -e) ? 1 : 3;
     }
-    const float ghb = 0.5f * g * (hL + hR);
-    const float uhat = __fdividef(cL * uL + cR * uR, cL + cR);
+    const float ghb = gf_fmul(gf_fmul(0.5f, g), hL + hR);
+    const float uhat = gf_fdiv(gf_ffma(cL, uL, gf_fmul(cR, uR)), cL + cR);
     const float chat = gf_sqrtf(ghb);
     const float l1 = fminf(uL - cL, uhat - chat), l3 = fmaxf(uR + cR, uhat + chat);
     /* middle-state speeds: the formulas of gf_riemanntype for two
@@ -415,47 +438,49 @@ __device__ __forceinline__ int gf_face_class(float hL, float hR, float uL, float
     const float hmin = fminf(hL, hR), hmax = fmaxf(hL, hR), dh = hmax - hmin;
     const float cmin = fminf(cL, cR), cmax = fmaxf(cL, cR);
     const float delu = uR - uL;
-    const float Fmin = delu + 2.0f * (cmin - cmax);
-    const float dhs = dh * gf_sqrtf(__fdividef(ghb, hL * hR)); /* dh sqrt(g (1/hL + 1/hR) / 2) */
+    const float Fmin = gf_ffma(2.0f, cmin - cmax, delu);
+    const float dhs = gf_fmul(dh, gf_sqrtf(gf_fdiv(ghb, gf_fmul(hL, hR)))); /* dh sqrt(g (1/hL + 1/hR) / 2) */
     const float Fmax = delu + dhs;
-    const float hm = fminf(fmaxf(hmin - __fdividef(Fmin * dh, Fmax - Fmin), hmin), hmax);
-    const float cm = gf_sqrtf(g * hm);
-    const float c3 = 0.75f * fmaxf(0.0f, 2.0f * (cL + cR) - delu);
+    const float hm = fminf(fmaxf(hmin - gf_fdiv(gf_fmul(Fmin, dh), Fmax - Fmin), hmin), hmax);
+    const float cm = gf_sqrtf(gf_fmul(g, hm));
+    const float c3 = gf_fmul(0.75f, fmaxf(0.0f, gf_ffma(2.0f, cL + cR, -delu)));
+    const float wL = gf_ffma(2.0f, cL, uL), wR = gf_ffma(-2.0f, cR, uR);
     const bool left = hL > hR, rare = Fmin > 0.0f, shock = !rare & (Fmax <= 0.0f);
-    const float s1m = rare    ? uL + 2.0f * cL - c3
+    const float s1m = rare    ? wL - c3
                       : shock ? (left ? uL : uL - dhs) - cmax
-                              : (left ? uL + 2.0f * cL - 3.0f * cm : uR - 2.0f * cR + cm);
-    const float s2m = rare    ? uR - 2.0f * cR + c3
+                              : (left ? gf_ffma(-3.0f, cm, wL) : wR + cm);
+    const float s2m = rare    ? wR + c3
                       : shock ? (left ? uR + dhs : uR) + cmax
-                              : (left ? uL + 2.0f * cL - cm : uR - 2.0f * cR + 3.0f * cm);
-    const float em = 1.0e-4f * (S + fabsf(s1m) + fabsf(s2m)), e = 1.0e-5f * S;
+                              : (left ? wL - cm : gf_ffma(3.0f, cm, wR));
+    const float em = gf_fmul(1.0e-4f, S + fabsf(s1m) + fabsf(s2m)), e = gf_fmul(1.0e-5f, S);
     const bool mid = (hmin > 1.0e-15f) & (hmax < 1.0e15f) & (S < 1.0e15f) & (s2m > l1 + em) & (s1m < l3 - em);
     /* the sonic tests with the middle-state speeds: clearly false, clearly
      * true (a bound of two shocks proves no truth) */
     const bool no1 = (l1 > crit2 + e) | (s1m < -crit2 - em), no2 = (l3 < -crit2 - e) | (s2m > crit2 + em);
     const bool yes = !shock & (((l1 < crit2 - e) & (s1m > -crit2 + em)) | ((l3 > -crit2 + e) & (s2m < crit2 - em)));
     /* the other sonic tests clearly false */
-    const float us = uL + uR, uu = uL * uR;
-    const float sb = 0.25f * us * us - ghb, st = fmaxf(0.0f, uu) - ghb;
-    const float A = 0.25f * us * us + ghb, B = fabsf(uu) + ghb, ab = fabsf(sb);
-    bool ok = no1 & no2 & (ab > crit + 1.0e-3f * A);
-    ok = ok & (sb * st > crit * crit + 1.0e-4f * A * B);
-    ok = ok & (sb * l1 * l3 > crit * crit + 1.0e-4f * A * S * S);
+    const float us = uL + uR, uu = gf_fmul(uL, uR), us4 = gf_fmul(0.25f, us), cc = gf_fmul(crit, crit);
+    const float sb = gf_ffma(us4, us, -ghb), st = fmaxf(0.0f, uu) - ghb;
+    const float A = gf_ffma(us4, us, ghb), B = fabsf(uu) + ghb, ab = fabsf(sb), A4 = gf_fmul(1.0e-4f, A);
+    bool ok = no1 & no2 & (ab > gf_ffma(1.0e-3f, A, crit));
+    ok = ok & (gf_fmul(sb, st) > gf_ffma(A4, B, cc));
+    ok = ok & (gf_fmul(gf_fmul(sb, l1), l3) > gf_ffma(gf_fmul(A4, S), S, cc));
     ok = ok & (fminf(fabsf(l1), fabsf(l3)) > crit2 + e);
     const float pL = uL + cL, pR = uR + cR, mL = uL - cL, mR = uR - cR;
     ok = ok & ((fminf(pL, pR) > e) | (fmaxf(pL, pR) < -e));
     ok = ok & ((fminf(mL, mR) > e) | (fmaxf(mL, mR) < -e));
     /* the jump of h within hsd / l1, hsd / l3 (or -hL, hR) */
-    const float rsb = __fdividef(ghb, sb);
-    const float dd = (bR - bL) * rsb;
-    const float de = 0.02f * fabsf(dd) + 1.0e-5f * (fabsf(bL) + fabsf(bR)) * fabsf(rsb);
-    const float num = hL * (uL - l1) + hR * (l3 - uR);
-    const float en = 1.0e-5f * (hL * (fabsf(uL) + fabsf(l1)) + hR * (fabsf(uR) + fabsf(l3)));
-    const bool t1 = num - dd * l1 - fabsf(l1) * de > en, t3 = num - dd * l3 - fabsf(l3) * de > en;
+    const float rsb = gf_fdiv(ghb, sb);
+    const float dd = gf_fmul(bR - bL, rsb);
+    const float de = gf_ffma(0.02f, fabsf(dd), gf_fmul(gf_fmul(1.0e-5f, fabsf(bL) + fabsf(bR)), fabsf(rsb)));
+    const float num = gf_ffma(hL, uL - l1, gf_fmul(hR, l3 - uR));
+    const float en = gf_fmul(1.0e-5f, gf_ffma(hL, fabsf(uL) + fabsf(l1), gf_fmul(hR, fabsf(uR) + fabsf(l3))));
+    const bool t1 = gf_ffma(-fabsf(l1), de, gf_ffma(-dd, l1, num)) > en;
+    const bool t3 = gf_ffma(-fabsf(l3), de, gf_ffma(-dd, l3, num)) > en;
     const bool sub = (l1 < -crit - e) & (l3 > crit + e), right = l1 > crit + e, leftw = l3 < -crit - e;
     ok = ok & (num > en) & (sub | right | leftw);
     ok = ok & (t1 | !(sub | right)) & (t3 | !(sub | leftw));
-    ok = ok & ((dd - de > -0.999f * hL) | !right) & ((dd + de < 0.999f * hR) | !leftw);
+    ok = ok & ((dd - de > gf_fmul(-0.999f, hL)) | !right) & ((dd + de < gf_fmul(0.999f, hR)) | !leftw);
     return !mid ? 3 : ok ? 0 : yes ? 2 : no1 & no2 ? 1 : 3;
 }
 
