@@ -40,14 +40,21 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "cell-updates/s"
 BYTES_PER_CELL_UPDATE = 56  # read h, hu, hv, b; write h, hu, hv (FP64)
-# Per tile shape of the mx = 32 update (threads, rows per band), from one ncu
+# Per tile shape of the mx = 32 update (threads, rows per band, cluster), from one ncu
 # capture of the launch this bench times first in its kernel-only loop (update
 # launch 24 of `--steps 20 --warmup 3`, the same state): DRAM traffic
 # (dram__bytes_read.sum + dram__bytes_write.sum; below the 234.9 MB algorithmic,
 # since rows without water are read for their depth alone) and FP64 warp
 # instructions (sm__inst_executed_pipe_fp64.sum; x 32 lanes / 4 194 304 cell-updates = FP64 issue slots per cell-update)
-NCU_COUNTS = {(256, 4): (90.650368e6 + 89.671680e6, 18.152225e6)}
-NCU_DEFAULT_TILE = (256, 4)
+NCU_COUNTS = {(256, 4, 1): (90.650368e6 + 89.671680e6, 18.152225e6)}
+
+
+def ncu_counts(tile):
+    """(DRAM bytes, FP64 warp instructions) of a launch of this tile; None for a
+    tile without a capture: another tile's counts are not its."""
+    return NCU_COUNTS.get(tuple(tile), (None, None))
+
+
 M = 32
 NPX = NPY = 64
 DX = 1.0
@@ -551,7 +558,8 @@ def compact(r: dict) -> dict:
         out["cpu_baseline"] = dict(out["cpu_baseline"], value=_sig(out["cpu_baseline"]["value"]))
     rl = r["roofline"]
     out["roofline"] = {"bound": rl["bound"], "achieved": _sig(rl["achieved"]), "peak": rl["peak"],
-                       "unit": rl["unit"], "frac": _sig(rl["frac"], 3), "traffic": int(rl["traffic"])}
+                       "unit": rl["unit"], "frac": _sig(rl["frac"], 3),
+                       "traffic": None if rl["traffic"] is None else int(rl["traffic"])}
     ck = r.get("clocks") or {}
     out["clocks"] = {"sm_mhz": ck.get("sm_mhz"), "sm_max_mhz": ck.get("sm_max_mhz"),
                      "reasons": ck.get("reasons")}
@@ -694,16 +702,8 @@ def run_gpu(args):
     lone_us = lone_patch_latency_us(ctx, q, aux)
 
     hbm_peak, peak_kind = load_peaks()
-    tile32 = NCU_DEFAULT_TILE  # what a launch of this many patches takes by itself
-    tsel = next((t for t in (tiles or []) if t["mx"] == M), None)
-    if tsel is not None:
-        tile32 = tuple(tsel["tiles"][tsel["best_throughput"]][:2])
-    elif args.tiles:
-        for spec in filter(None, args.tiles.split(",")):
-            mx_s, thr, _ = (int(v) for v in spec.split(":"))
-            if mx_s == M:
-                tile32 = {0: (256, 7), 1: (256, 4), 2: (384, 7), 3: (384, 9)}.get(thr, tile32)
-    traffic, fp64_warp_inst = NCU_COUNTS.get(tile32, NCU_COUNTS[NCU_DEFAULT_TILE])
+    tile32 = gf.Context.tile_shape(M, gf.Context.tile_of(M, q.shape[0]))
+    traffic, fp64_warp_inst = ncu_counts(tile32)
     algo = BYTES_PER_CELL_UPDATE * ncell
     achieved = algo / (kernel_ms * 1e-3) / 1e9
     rates = fp64_rates()
@@ -717,12 +717,15 @@ def run_gpu(args):
         # FP64 issue slots (warp instructions x 32 lanes) per cell-update of
         # this workload, from the ncu capture of the same kernel: the achieved
         # FP64 issue rate follows from the live kernel time
-        ops = fp64_warp_inst * 32 / float(ncell)
-        ach = ops * ncell / (kernel_ms * 1e-3) / 1e9
-        fp64.update({"lane_ops_per_cell_update": ops, "achieved_gops": ach,
-                     "frac_of_measured_dfma": ach / (rates["dfma"] / 1e9),
-                     "ops_source": "ncu sm__inst_executed_pipe_fp64.sum of this kernel on "
-                                   "this workload x 32 lanes / cell-updates (one capture)"})
+        if fp64_warp_inst is not None:
+            ops = fp64_warp_inst * 32 / float(ncell)
+            ach = ops * ncell / (kernel_ms * 1e-3) / 1e9
+            fp64.update({"lane_ops_per_cell_update": ops, "achieved_gops": ach,
+                         "frac_of_measured_dfma": ach / (rates["dfma"] / 1e9),
+                         "ops_source": "ncu sm__inst_executed_pipe_fp64.sum of this kernel on "
+                                       "this workload x 32 lanes / cell-updates (one capture)"})
+        else:
+            fp64.update({"frac_of_measured_dfma": None, "ops_source": "no capture of this tile"})
     result = {
         "metric": METRIC, "value": world * ncell / (ms * 1e-3), "unit": METRIC,
         "n_gpus": world, "steps": args.steps, "warmup": max(args.warmup, 3),
@@ -738,7 +741,8 @@ def run_gpu(args):
                      "frac": achieved / hbm_peak, "traffic": traffic, "tile": list(tile32),
                      "traffic_unit": "bytes per launch",
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum "
-                                       "of one launch (one capture)",
+                                       "of one launch (one capture)" if traffic is not None
+                                       else "no capture of this tile",
                      "algorithmic_bytes_per_launch": algo,
                      "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)",
                      "kernel_ms": kernel_ms,
