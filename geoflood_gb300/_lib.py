@@ -357,7 +357,8 @@ _f8 = np.dtype(np.float64)
 
 def dptrs(arrays):
     """dptr of every array, as the pointer array of a batch: plain addresses,
-    without a pointer object each (half of what 129 patches' call spent)."""
+    without a pointer object each (129 patches' two arrays about 600 us so, 250 now,
+    almost all of it numpy's address of an array)."""
     for a in arrays:
         assert a.dtype == _f8 and a.flags.c_contiguous, "need contiguous float64"
     return C.cast((_vp * len(arrays))(*[a.ctypes.data for a in arrays]), C.POINTER(_dp))

@@ -99,8 +99,9 @@ cudaError_t launch_aos_to_soa(const double* src, double* dst, long npatch, int n
                               long src_stride, long dst_stride, cudaStream_t st);
 cudaError_t launch_soa_to_aos(const double* src, double* dst, long npatch, int ncell, int nf,
                               long src_stride, long dst_stride, cudaStream_t st);
-/* both of a host batch's layouts (q with nfa fields, aux with nfb) in one
- * launch; each set is npatch contiguous blocks of nf * ncell doubles */
+/* a host batch from its pinned buffers (npatch blocks of 3 or maux fields by
+ * ncell cells, field fastest) into planes, the status zeroed, in one launch; and
+ * the planes of q back, with the status and, unless hcfl is null, the CFLs */
 cudaError_t launch_batch_in(const double* hq, double* q, const double* ha, double* aux, int maux, long npatch,
                             int ncell, unsigned long long* gmax, int* err, cudaStream_t st);
 cudaError_t launch_batch_out(const double* q, double* hq, long npatch, int ncell, const double* cfl, double* hcfl,
@@ -168,9 +169,9 @@ cudaError_t launch_pyramid_top(const double* src, double* dst, int nx, int ny, c
 cudaError_t launch_pyramid_down(const double* fine, double* coarse, int nxc, int nyc,
                                 cudaStream_t st);
 cudaError_t launch_patch_fill(int m, const gf_fill_task* tasks, int ntask, cudaStream_t st);
-/* cell averages of topo grids over a raster (interior cells inside the
- * domain, then the cells outside copy the nearest inside); *err = 1 when a
- * cell overlaps no grid; finest: the smallest spacing of the grids */
+/* cell averages of topo grids over a raster (a cell outside the domain is
+ * integrated as the nearest inside); *err = 1 when a cell overlaps no grid;
+ * finest: the smallest spacing of the grids */
 cudaError_t launch_topo_raster(const gf_topo_grid* grids, const int* order, int n, int nx, int ny,
                                int halo, double xlower, double ylower, double dx, double dy,
                                double xupper, double yupper, double finest, double* out, int* err,

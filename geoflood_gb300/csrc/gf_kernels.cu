@@ -252,7 +252,7 @@ int latency_goal_fits(int m, long npatch)
 /* Launches that leave SMs idle take a tile that spreads a patch: the first of
  * these with at most per_2sm CTAs for two SMs (FP64 throughput is the SM's, so a
  * split pays while SMs are free), and, for one_wave, all of them resident at
- * once. us for that many 32^2 patches, the next choice beside it: K = 8 42 (1;
+ * once (clusters of 8 of 15 patches on this device, of 4 of 36). us for that many 32^2 patches, the next choice beside it: K = 8 42 (1;
  * 56), K = 4 55 (24; 90), K = 2 90 (72; 171), 167 (152; 188), 251 (247; 288), but
  * 325 (304; 289); 16^2: K = 8 29 (1; 31), K = 4 33 (24; 40), K = 2 41 (72; 64), 54
  * (152; 64), the streamed 192 x 7 94 (304; 102) and 166 (400; 134); 8^2: K = 4 29
@@ -267,7 +267,7 @@ static const SmallTile kSmall32[] = {{5, 2, true}, {4, 2, true}, {6, 7, false}};
 /* Whole 32^2 levels: the streamed tile, two CTAs an SM, when it fills its slots
  * once (247 patches 286 us, 384 x 9 301) or many times (4096 patches 3.18 ms,
  * 3.34; 1215 1.07, 1.09); between, its half-empty last wave costs more than it
- * gains (400 patches 509 us against 445, 760 767 against 732). */
+ * gains (400 patches 504 us against 442, 760 671 against 612). */
 constexpr int kStream32 = 1, kStream32Waves = 6; /* patches an SM from which it always pays */
 
 /* Tile of a capped launch, whose CTAs walk the list on part of the SMs: no rule

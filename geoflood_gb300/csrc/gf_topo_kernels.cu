@@ -241,17 +241,17 @@ __device__ __forceinline__ double over_area(double v, double area, double rarea)
 
 /* The kernel is bound by FP64 issue (two lanes a clock), and most of it would go
  * into tests and quotients that depend on a cell's column or row alone. A tile of
- * 32 x 32 cells forms them once per column and row, one warp an axis, in shared
+ * 32 columns and kRows rows forms them once per column and row, one warp an axis, in shared
  * memory, for the cells that lie whole in the finest grid they touch; what is
  * left for a cell are the 14 operations of each node cell under it and the last
  * quotient. Halves of the axis sums stand for the factors 1/2 and 1/4 of the
  * bilinear form (powers of two, which no rounding sees), and the difference of a
  * node column serves both cells beside it: the same bits. The other cells (cells
  * that a grid's edge cuts, cells over more node cells than the tables hold) are
- * gathered, so that the column under an edge fills one warp, and take
- * cell_integral. 1535^2 cells over a 1025^2 grid with a 513^2 inset, ncu: 625 us
+ * gathered from 8 rows on, so that the column under an edge fills one warp, and
+ * take cell_integral. 1535^2 cells over a 1025^2 grid with a 513^2 inset, ncu: 625 us
  * with a warp for each row of them, 422 us gathered (82 % FP64 pipe, 89 FP64
- * instructions for 32 cells). Cells outside the domain are cells inside to this
+ * instructions for 32 cells; tiles of 32 rows). Cells outside the domain are cells inside to this
  * kernel (a pass of its own over the raster took 31 us). */
 template <int kTY, int kRows>
 __global__ void __launch_bounds__(kTX* kTY)
