@@ -43,10 +43,11 @@ BYTES_PER_CELL_UPDATE = 56  # read h, hu, hv, b; write h, hu, hv (FP64)
 # Per tile shape of the mx = 32 update (threads, rows per band, cluster), from one ncu
 # capture of the launch this bench times first in its kernel-only loop (update
 # launch 24 of `--steps 20 --warmup 3`, the same state): DRAM traffic
-# (dram__bytes_read.sum + dram__bytes_write.sum; below the 234.9 MB algorithmic,
-# since rows without water are read for their depth alone) and FP64 warp
+# (dram__bytes_read.sum + dram__bytes_write.sum; 256 x 4 below the 234.9 MB algorithmic,
+# since it reads rows without water for their depth alone) and FP64 warp
 # instructions (sm__inst_executed_pipe_fp64.sum; x 32 lanes / 4 194 304 cell-updates = FP64 issue slots per cell-update)
-NCU_COUNTS = {(256, 4, 1): (90.650368e6 + 89.671680e6, 18.152225e6)}
+NCU_COUNTS = {(256, 4, 1): (90.599424e6 + 89.816064e6, 18.159435e6),
+              (384, 9, 1): (170.307328e6 + 75.584512e6, 17.745479e6)}
 
 
 def ncu_counts(tile):

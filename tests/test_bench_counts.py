@@ -19,8 +19,8 @@ def bench():
 
 
 def test_a_tile_without_a_capture_has_no_counts(bench):
-    assert all(v > 0 for v in bench.ncu_counts([256, 4, 1]))
-    for tile in ((384, 9, 1), (256, 7, 1), (384, 10, 2)):
+    assert all(v > 0 for tile in ([256, 4, 1], [384, 9, 1]) for v in bench.ncu_counts(tile))
+    for tile in ((256, 7, 1), (384, 7, 1), (384, 10, 2)):
         assert bench.ncu_counts(tile) == (None, None)
 
 
