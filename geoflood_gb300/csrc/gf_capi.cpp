@@ -262,7 +262,7 @@ int gf_ctx_create(int device, gf_ctx** out)
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_status, sizeof(DevStatus));
     if (e == cudaSuccess) e = cudaMalloc(&c->d_gdt, sizeof(double) * 64);
     if (e == cudaSuccess) e = cudaMallocHost(&c->h_gdt, sizeof(double) * 64);
-    if (e == cudaSuccess) e = cudaMemset(c->d_status, 0, sizeof(DevStatus));
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->d_status, 0, sizeof(DevStatus), c->stream);
     if (e != cudaSuccess) {
         gf_ctx_destroy(c);
         return e == cudaErrorMemoryAllocation ? GF_ERR_NOMEM : GF_ERR_CUDA;
@@ -833,7 +833,8 @@ static int level_pipe_setup(gf_level* L)
         std::vector<gf_ghost_ref> r(L->npatch);
         for (int p = 0; p < L->npatch; ++p) r[p] = gf_ghost_ref{0, p};
         GF_CK(c, cudaMalloc(&L->d_refs, r.size() * sizeof(gf_ghost_ref)));
-        GF_CK(c, cudaMemcpy(L->d_refs, r.data(), r.size() * sizeof(gf_ghost_ref), cudaMemcpyHostToDevice));
+        GF_CK(c, cudaMemcpyAsync(L->d_refs, r.data(), r.size() * sizeof(gf_ghost_ref), cudaMemcpyHostToDevice,
+                                 c->stream));
     }
     L->pipe_ready = true;
     return GF_OK;
@@ -1301,9 +1302,12 @@ extern "C" int gf_autotune(gf_ctx* c, int reps, gf_tile_result* out)
             w[p].aux = db + (size_t)p * S;
             w[p].dx = w[p].dy = 1.0;
         }
-        if (e == cudaSuccess) e = cudaMemcpy(dq, hq.data(), hq.size() * sizeof(double), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(db, hb.data(), hb.size() * sizeof(double), cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(dw, w.data(), w.size() * sizeof(gf_patch_work), cudaMemcpyHostToDevice);
+        auto up = [&](void* to, const void* from, size_t bytes) {
+            if (e == cudaSuccess) e = cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, c->stream);
+        };
+        up(dq, hq.data(), hq.size() * sizeof(double));
+        up(db, hb.data(), hb.size() * sizeof(double));
+        up(dw, w.data(), w.size() * sizeof(gf_patch_work));
         double best_t = -1.0, best_l = 1e300;
         for (int v = 0; v < R.nvariant && e == cudaSuccess; ++v) {
             gf::tile_shape(m, v, &R.threads[v], &R.band[v], &R.cluster[v]);

@@ -974,8 +974,8 @@ int place_gauges(gf_forest* f)
         if (ii >= M || jj >= M) f->gauge_ghosts = true;
     }
     FK(f, f->d_gtask.reserve(f->gauges.size()));
-    FK(f, cudaMemcpy(f->d_gtask.p, f->gauges.data(), f->gauges.size() * sizeof(gf_gauge_task),
-                     cudaMemcpyHostToDevice));
+    FK(f, cudaMemcpyAsync(f->d_gtask.p, f->gauges.data(), f->gauges.size() * sizeof(gf_gauge_task),
+                          cudaMemcpyHostToDevice, gf::ctx_stream(f->ctx)));
     f->gauges_placed = true;
     return GF_OK;
 }
@@ -1566,10 +1566,12 @@ int gf_forest_create(gf_ctx* c, const gf_forest_opts* o, const double* fields, g
         gf_forest_destroy(f);
         return rc;
     }
-    /* the refinement criteria live on the device for the tag launches */
+    /* the refinement criteria live on the device for the tag launches, whose
+     * stream may be another one */
     e = f->d_refine.reserve(1);
     if (e == cudaSuccess)
-        e = cudaMemcpy(f->d_refine.p, &o->refine, sizeof(gf_refine), cudaMemcpyHostToDevice);
+        e = cudaMemcpyAsync(f->d_refine.p, &o->refine, sizeof(gf_refine), cudaMemcpyHostToDevice, gf::ctx_stream(c));
+    if (e == cudaSuccess) e = cudaStreamSynchronize(gf::ctx_stream(c));
     if (e != cudaSuccess) {
         gf_forest_destroy(f);
         return gf::ctx_cuda_fail(c, e, "forest refinement criteria");
@@ -1914,7 +1916,8 @@ int gf_forest_set_gauges(gf_forest* f, int n, const int* id, const double* xc, c
         FK(f, f->d_glast.reserve(n));
         FK(f, f->d_grec.reserve((size_t)f->grec_cap * n * 6));
         const std::vector<double> never(n, -INFINITY);
-        FK(f, cudaMemcpy(f->d_glast.p, never.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+        FK(f, cudaMemcpyAsync(f->d_glast.p, never.data(), n * sizeof(double), cudaMemcpyHostToDevice,
+                              gf::ctx_stream(f->ctx)));
     }
     return GF_OK;
 }

@@ -559,20 +559,21 @@ int topo_device(gf_topo* t, int dev, cudaStream_t st, const gf_topo_grid** grid,
         size_t off = 0;
         for (size_t k = 0; k < t->grids.size(); ++k) {
             const TopoGrid& g = t->grids[k];
-            if (cudaMemcpy(t->d_z + off, g.z.data(), g.z.size() * sizeof(double), cudaMemcpyHostToDevice) !=
+            if (cudaMemcpyAsync(t->d_z + off, g.z.data(), g.z.size() * sizeof(double), cudaMemcpyHostToDevice, st) !=
                 cudaSuccess)
                 return GF_ERR_CUDA;
             hg[k] = gf_topo_grid{t->d_z + off, g.mx, g.my, g.xlow, g.ylow, g.xhi, g.yhi, g.dx, g.dy};
             off += g.z.size();
         }
-        if (cudaMemcpy(t->d_grid, hg.data(), hg.size() * sizeof(gf_topo_grid), cudaMemcpyHostToDevice) !=
+        /* done before any stream reads them: the set may be used on another one */
+        if (cudaMemcpyAsync(t->d_grid, hg.data(), hg.size() * sizeof(gf_topo_grid), cudaMemcpyHostToDevice, st) !=
                 cudaSuccess ||
-            cudaMemcpy(t->d_order, t->order.data(), t->order.size() * sizeof(int), cudaMemcpyHostToDevice) !=
-                cudaSuccess)
+            cudaMemcpyAsync(t->d_order, t->order.data(), t->order.size() * sizeof(int), cudaMemcpyHostToDevice, st) !=
+                cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
             return GF_ERR_CUDA;
         t->stale = false;
     }
-    (void)st;
     *grid = t->d_grid;
     *order = t->d_order;
     return GF_OK;
