@@ -899,7 +899,8 @@ int gf_level_step_host(gf_level* L, double* q, double t, double dt, double* maxc
                                                    &L->d_status->err, sk));
         else
             GF_CK(c, gf::launch_patch_update(L->mx, L->d_work + p0, np, c->d_phys, dt, nullptr, nullptr, L->maux,
-                                             L->d_cfl + p0, &L->d_status->gmax, &L->d_status->err, sk));
+                                             L->d_cfl + p0, &L->d_status->gmax, &L->d_status->err, sk, 0, 0,
+                                             L->npatch));
         GF_CK(c, cudaEventRecord(upd[k], sk));
         /* chunks whose neighbours are all updated now */
         for (int j = 0; j < nc; ++j)

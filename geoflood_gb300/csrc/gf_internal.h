@@ -46,11 +46,12 @@ void host_parallel_for(long n, long bytes, const std::function<void(long, long)>
 /* gdt / gpar (nullable): per-group dt (<= 0 skips the group) and state
  * parity (1: the group's state is in the work items' qout buffers). */
 /* max_ctas > 0 caps the grid: each CTA then walks the work list with a
- * grid stride, leaving the other SMs to concurrent launches. */
+ * grid stride, leaving the other SMs to concurrent launches. whole: the patches
+ * of the level, for a launch over a part of it. */
 cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, const gf_phys* phys,
                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                 unsigned long long* gmax, int* err, cudaStream_t st,
-                                int max_ctas = 0, int goal = 0);
+                                int max_ctas = 0, int goal = 0, long whole = 0);
 /* resident CTAs per SM of the tile of capped launches, or of the one chosen by
  * hand or, without, by default for whole levels */
 int patch_update_occupancy(int m, bool capped = false);

@@ -281,8 +281,12 @@ static int capped_tile(int m)
 /* A choice by hand always stands, the tuned latency tile where it is asked for.
  * The tuned throughput tile serves launches of the size it was measured on:
  * below, the number of patches decides as without it (400 patches of 32^2 442 us
- * so, 504 by the tile that is the fastest for 4096; 760 612 and 671). */
-static int pick_tile(int m, long npatch, int max_ctas, int goal)
+ * so, 504 by the tile that is the fastest for 4096; 760 612 and 671). whole: the
+ * patches of the level that the launch is a part of; parts follow one another
+ * on two streams, without the last waves that decide for a launch by itself (host
+ * step of 4096 patches, half of them wet, 2.76 ms by the part's number, 2.47 by the
+ * level's). */
+static int pick_tile(int m, long npatch, int max_ctas, int goal, long whole = 0)
 {
     const int c = mcls(m);
     goal = goal != 0;
@@ -299,7 +303,7 @@ static int pick_tile(int m, long npatch, int max_ctas, int goal)
             (!s[i].one_wave || npatch <= tile_resident(m, s[i].v)))
             return s[i].v;
     if (const int by_hand = g_pin[0][c]; by_hand >= 0) return by_hand; /* goal 1 */
-    if (const int tuned = g_tuned[0][c]; tuned >= 0 && npatch * m * m >= kTuneCells) return tuned;
+    if (const int tuned = g_tuned[0][c]; tuned >= 0 && std::max(npatch, whole) * m * m >= kTuneCells) return tuned;
     if (c == 2 && (npatch <= tile_resident(m, kStream32) || npatch >= (long)kStream32Waves * sm_count()))
         return kStream32;
     return kDefault[c];
@@ -344,7 +348,7 @@ cudaError_t launch_patch_update_tile(int m, int v, const gf_patch_work* work, in
 cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, const gf_phys* phys,
                                 double dt, const double* gdt, const int* gpar, int maux, double* cfl,
                                 unsigned long long* gmax, int* err, cudaStream_t st, int max_ctas,
-                                int goal)
+                                int goal, long whole)
 {
     if (!(m == 8 || m == 16 || m == 32)) return cudaErrorInvalidValue;
     if (nwork <= 0) { /* set every tile's attributes, ahead of a capture */
@@ -357,8 +361,8 @@ cudaError_t launch_patch_update(int m, const gf_patch_work* work, int nwork, con
         }
         return cudaSuccess;
     }
-    return launch_patch_update_tile(m, pick_tile(m, nwork, max_ctas, goal), work, nwork, phys, dt, gdt, gpar,
-                                    maux, cfl, gmax, err, st, max_ctas);
+    return launch_patch_update_tile(m, pick_tile(m, nwork, max_ctas, goal, whole), work, nwork, phys, dt, gdt,
+                                    gpar, maux, cfl, gmax, err, st, max_ctas);
 }
 
 int sm_count()
