@@ -131,17 +131,29 @@ class Context:
         if rc != 0:
             raise GeoFloodError(rc, f"gf_ctx_create(device={device}) failed")
         self.h = h
-        # levels and forests live on this context: they are closed before it
+        # levels and forests live on this context: they are closed before it,
+        # also where the collector takes them together and has cleared the weak
+        # references (their handles and how to destroy them are kept for that)
         self._children = weakref.WeakSet()
+        self._open = {}
         self.set_phys(0, phys or Phys())
 
-    def _adopt(self, child):
+    def _adopt(self, child, destroy):
         self._children.add(child)
+        self._open[id(child)] = (destroy, child.h)
+
+    def _destroy(self, child):
+        destroy, h = self._open.pop(id(child), (None, None))
+        if destroy:
+            destroy(h)
 
     def close(self):
         if getattr(self, "h", None):
             for ch in list(self._children):
                 ch.close()
+            while self._open:
+                destroy, h = self._open.popitem()[1]
+                destroy(h)
             self._lib.gf_ctx_destroy(self.h)
             self.h = None
 
@@ -306,7 +318,7 @@ class Level:
         _check(ctx.h, self._lib.gf_level_create(ctx.h, self.npatch, self.m, self.m, self.maux,
                                                 C.byref(h)))
         self.h = h
-        ctx._adopt(self)
+        ctx._adopt(self, self._lib.gf_level_destroy)
 
     @property
     def shape_q(self):
@@ -318,7 +330,7 @@ class Level:
 
     def close(self):
         if getattr(self, "h", None):
-            self._lib.gf_level_destroy(self.h)
+            self.ctx._destroy(self)
             self.h = None
 
     def __del__(self):

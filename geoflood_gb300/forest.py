@@ -85,11 +85,11 @@ class Forest:
         h = C.c_void_p()
         _check(ctx.h, self._lib.gf_forest_create(ctx.h, C.byref(o), dptr(planes), C.byref(h)))
         self.h = h
-        ctx._adopt(self)
+        ctx._adopt(self, self._lib.gf_forest_destroy)
 
     def close(self):
         if getattr(self, "h", None):
-            self._lib.gf_forest_destroy(self.h)
+            self.ctx._destroy(self)
             self.h = None
 
     def __del__(self):
